@@ -2072,6 +2072,11 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_pcg_part_mixed(KArgs a) {
     pcg_part_mixed<IC, LOCAL>(a, sh, part_smem);
 }
 
+}  // namespace pf2
+
+#include "part_halo.cuh"
+
+namespace pf2 {
 
 __global__ void __launch_bounds__(kSolverThreads, kSolverBlocksPerSm) k_pcg_one(KArgs a) {
     __shared__ double sh[kShDoubles];
@@ -2840,6 +2845,13 @@ struct pf2_solver {
     DevBuf<unsigned char> q_bnd;
     DevBuf<double> q_val, q_f, q_x, q_gp, q_gt, q_gz;
     DevBuf<float> q_val32, q_f32, q_gp32, q_gt32, q_gz32;  // mixed precision
+    // the parts with halo rows (k_pcg_halo; shares q_s, q_a, q_x, the entry maps and values)
+    bool halo = false;
+    int halo_RL = 0;
+    long long halo_entries = 0;
+    DevBuf<int> h_hs, h_hoff, h_hq, h_foff, h_fg, h_zoff, h_zg, h_r1off, h_ebase, h_rp;
+    DevBuf<unsigned short> h_fl, h_zl, h_r1, h_lcol;
+    DevBuf<unsigned char> h_dg, h_pub;
     bool factored = false;
     const pf2_csr* last = nullptr;  // matrix of the last setup / solve
 };
@@ -3025,6 +3037,201 @@ static void graph_parts(int n, const std::vector<int>& rp, const std::vector<int
 // boundary flags.  Leaves S->part false where the plan does not apply: a group whose rows
 // depend on one another, or a part too large for the shared-memory vectors.
 constexpr int kPartMinRows = 512;
+
+// The halo form of the plan (part_halo.cuh) on the parts and the order Q of build_part_plan
+// (bq: Q position of B's row, qb its inverse, qa the row of A).  Leaves S->halo false where
+// it does not apply: a part's rows with its halo exceed the shared memory or the 16-bit local
+// columns, or the halo is larger than the part (many groups: a 3D graph), where every part
+// would compute most of its neighbours' sweeps.  Where it applies it measured faster at every
+// size (us per IC(0) iteration, waits in the sweeps against halo rows: 340 rows 23.1 / 19.4,
+// 16,705 rows 25.2 / 19.0, 125,364 rows 29.7 / 21.8, 499,288 rows 43.1 / 39.5).
+static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, const std::vector<int>& bcol,
+                                  const std::vector<int>& bmap, const std::vector<int>& bdiag,
+                                  const std::vector<int>& perm, const std::vector<int>& part,
+                                  const std::vector<int>& grp, const std::vector<int>& qs, const std::vector<int>& bq,
+                                  const std::vector<int>& qb, const std::vector<int>& qa, int P, int ng, int R,
+                                  int optin, bool tri, bool mixed) {
+    S->halo = false;
+    const int n = S->n;
+    if (const char* e = getenv("PF2_CG_PART"))
+        if (atoi(e) == 3) return PF2_OK;  // tests: the kernel with waits inside the sweeps
+    if (const char* e = getenv("PF2_CG_PART_LOCAL"))
+        if (mixed && tri && atoi(e) != 0) return PF2_OK;
+    // rows of B by part (Q order: consecutive), pid the part of a row of B
+    std::vector<int> pid(n), local(n, -1), stamp(n, -1);
+    std::vector<unsigned char> cls(n, 0), pub(n, 0);
+    for (int r = 0; r < n; ++r) pid[r] = part[perm[r]];
+    std::vector<int> hs((size_t)P * ng * 4), hoff(P + 1, 0), hq, foff(P + 1, 0), fg, zoff(P + 1, 0), zg, r1off(P + 1, 0),
+        ebase(P + 1, 0), rp, amap, fmap;
+    std::vector<unsigned short> fl, zl, r1, lcol;
+    std::vector<unsigned char> dg;
+    rp.reserve(n + n / 8 + P);
+    dg.reserve(n + n / 8);
+    lcol.reserve(S->nnz + S->nnz / 8);
+    amap.reserve(S->nnz + S->nnz / 8);
+    fmap.reserve(S->nnz + S->nnz / 8);
+    std::vector<std::vector<int>> bucket(ng);
+    std::vector<int> ring, halo;
+    int RL = 0;
+    enum { F = 1, Z = 2 };
+    for (int k = 0; k < P; ++k) {
+        const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0;
+        // ring 1, the F rows among it (read by an own row's lower entries) and the closures
+        ring.clear();
+        halo.clear();
+        for (auto& b : bucket) b.clear();
+        auto add = [&](int j, int bits) {
+            if (stamp[j] != k) {
+                stamp[j] = k;
+                cls[j] = 0;
+                halo.push_back(j);
+                bucket[grp[j]].push_back(j);
+            }
+            cls[j] |= bits;
+        };
+        for (int q = p0; q < p0 + np; ++q) {
+            const int i = qb[q];
+            for (int e = brp[i]; e < brp[i + 1]; ++e) {
+                const int j = bcol[e];
+                if (pid[j] == k) continue;
+                if (stamp[j] != k) ring.push_back(j);
+                add(j, !tri ? F : (e < bdiag[i] ? F | Z : Z));
+            }
+        }
+        if (tri) {
+            for (int g = ng - 1; g >= 0; --g)  // rows added have lower groups
+                for (size_t h = 0; h < bucket[g].size(); ++h) {
+                    const int i = bucket[g][h];
+                    if (!(cls[i] & F)) continue;
+                    for (int e = brp[i]; e < bdiag[i]; ++e)
+                        if (pid[bcol[e]] != k) add(bcol[e], F);
+                }
+            for (int g = 0; g < ng; ++g)  // rows added have higher groups
+                for (size_t h = 0; h < bucket[g].size(); ++h) {
+                    const int i = bucket[g][h];
+                    if (!(cls[i] & Z)) continue;
+                    for (int e = bdiag[i] + 1; e < brp[i + 1]; ++e)
+                        if (pid[bcol[e]] != k) add(bcol[e], Z);
+                }
+        }
+        const int nh = (int)halo.size();
+        if (nh > std::max(np, 64) || np + nh > 65535) {
+            S->part_why = "the halo rows outnumber a part's rows";
+            return PF2_OK;
+        }
+        RL = std::max(RL, np + nh);
+        // local numbering: own rows, then the halo by group as F only, F and Z, Z only
+        for (int q = p0; q < p0 + np; ++q) local[qb[q]] = q - p0;
+        int at = 0;
+        halo.clear();
+        for (int g = 0; g < ng; ++g) {
+            auto& b = bucket[g];
+            std::sort(b.begin(), b.end());
+            int* o = &hs[((size_t)k * ng + g) * 4];
+            auto put = [&](int want) {
+                for (int i : b)
+                    if (cls[i] == want) {
+                        halo.push_back(i);
+                        local[i] = np + at++;
+                    }
+            };
+            o[0] = at;
+            put(F);
+            o[1] = at;
+            put(F | Z);
+            o[2] = at;
+            put(Z);
+            o[3] = at;
+        }
+        for (int i : halo) {
+            hq.push_back(bq[i]);
+            if (cls[i] & F) {
+                fl.push_back((unsigned short)local[i]);
+                fg.push_back(bq[i]);
+                pub[bq[i]] |= 1;
+            } else {
+                zl.push_back((unsigned short)local[i]);
+                zg.push_back(bq[i]);
+                pub[bq[i]] |= 2;
+            }
+        }
+        for (int i : ring) r1.push_back((unsigned short)local[i]);
+        // entries: the own rows whole; a halo row's lower part (F), diagonal and upper part (Z)
+        const int e0 = (int)lcol.size();
+        ebase[k] = e0;
+        auto row = [&](int i, int b0, int b1, bool own) {
+            rp.push_back((int)lcol.size() - e0);
+            dg.push_back((unsigned char)(bdiag[i] - b0));
+            for (int e = b0; e < b1; ++e) {
+                lcol.push_back((unsigned short)local[bcol[e]]);
+                amap.push_back(own || (!tri && e == bdiag[i]) ? bmap[e] : -1);
+                fmap.push_back(e);
+            }
+        };
+        for (int q = p0; q < p0 + np; ++q) row(qb[q], brp[qb[q]], brp[qb[q] + 1], true);
+        for (int i : halo)
+            row(i, tri && (cls[i] & F) ? brp[i] : bdiag[i], tri && (cls[i] & Z) ? brp[i + 1] : bdiag[i] + 1, false);
+        rp.push_back((int)lcol.size() - e0);
+        hoff[k + 1] = (int)hq.size();
+        foff[k + 1] = (int)fl.size();
+        zoff[k + 1] = (int)zl.size();
+        r1off[k + 1] = (int)r1.size();
+    }
+    const long long ne = (long long)lcol.size();
+    const size_t smem = halo_smem_bytes(R, RL, tri, mixed ? sizeof(float) : sizeof(double), mixed);
+    if (smem + 2048 > (size_t)optin || ne > INT32_MAX) {
+        S->part_why = "a part's vectors exceed the shared memory of a block";
+        return PF2_OK;
+    }
+    ebase[P] = (int)ne;
+    auto up = [&](auto& d, const auto& h) -> pf2_status {
+        PF2_TRY(d.alloc(std::max<size_t>(h.size(), 1)));
+        if (!h.empty()) PF2_CUDA(cudaMemcpy(d.p, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice));
+        return PF2_OK;
+    };
+    PF2_TRY(up(S->q_s, qs));
+    PF2_TRY(up(S->q_a, qa));
+    PF2_TRY(up(S->q_amap, amap));
+    if (tri) PF2_TRY(up(S->q_fmap, fmap));
+    PF2_TRY(up(S->h_hs, hs));
+    PF2_TRY(up(S->h_hoff, hoff));
+    PF2_TRY(up(S->h_hq, hq));
+    PF2_TRY(up(S->h_foff, foff));
+    PF2_TRY(up(S->h_fl, fl));
+    PF2_TRY(up(S->h_fg, fg));
+    PF2_TRY(up(S->h_zoff, zoff));
+    PF2_TRY(up(S->h_zl, zl));
+    PF2_TRY(up(S->h_zg, zg));
+    PF2_TRY(up(S->h_r1off, r1off));
+    PF2_TRY(up(S->h_r1, r1));
+    PF2_TRY(up(S->h_ebase, ebase));
+    PF2_TRY(up(S->h_rp, rp));
+    PF2_TRY(up(S->h_dg, dg));
+    PF2_TRY(up(S->h_pub, pub));
+    PF2_TRY(up(S->h_lcol, lcol));
+    PF2_TRY(S->q_val.alloc(ne));
+    PF2_TRY(S->q_x.alloc(n));
+    if (tri) PF2_TRY(S->q_f.alloc(ne));
+    if (mixed) {
+        PF2_TRY(S->q_val32.alloc(ne));
+        PF2_TRY(S->q_f32.alloc(ne));
+        PF2_TRY(S->q_gp32.alloc(n));
+        PF2_TRY(S->q_gt32.alloc(2 * (size_t)n));
+    } else {
+        PF2_TRY(S->q_gp.alloc(n));
+        if (tri) PF2_TRY(S->q_gt.alloc(2 * (size_t)n));
+    }
+    S->halo = S->part = true;
+    S->halo_RL = RL;
+    S->halo_entries = ne;
+    S->part_local = false;
+    S->part_P = P;
+    S->part_R = R;
+    S->part_ng = ng;
+    S->part_smem = smem;
+    return PF2_OK;
+}
+
 static pf2_status build_part_plan(pf2_solver* S, const std::vector<int>& rp, const std::vector<int>& col,
                                   const std::vector<int>& brp, const std::vector<int>& bcol,
                                   const std::vector<int>& bmap, const std::vector<int>& bdiag,
@@ -3072,6 +3279,8 @@ static pf2_status build_part_plan(pf2_solver* S, const std::vector<int>& rp, con
     int optin = 0;
     PF2_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
     const bool mixed = S->opt.precision == PF2_PRECISION_MIXED;
+    PF2_TRY(build_halo_plan(S, brp, bcol, bmap, bdiag, perm, part, grp, qs, bq, qb, qa, P, ng, R, optin, tri, mixed));
+    if (S->halo) return PF2_OK;
     const size_t smem = (part_smem_bytes(R, tri, mixed ? sizeof(float) : sizeof(double), mixed) + 15) / 16 * 16;
     if (smem + 2048 > (size_t)optin) {
         S->part_why = "a part's vectors exceed the shared memory of a block";
@@ -3161,6 +3370,13 @@ static bool part_eligible(const pf2_solver* S) {
 
 // The partitioned CG kernel of the solver's preconditioner.
 static void* part_kernel(const pf2_solver* S) {
+    if (S->halo) {
+        if (S->opt.precision == PF2_PRECISION_MIXED)
+            return S->opt.precond == PF2_PRECOND_IC ? (void*)k_pcg_halo_mixed<true> : (void*)k_pcg_halo_mixed<false>;
+        if (S->opt.precond == PF2_PRECOND_IC) return (void*)k_pcg_halo<1>;
+        if (S->opt.precond == PF2_PRECOND_ILU) return (void*)k_pcg_halo<2>;
+        return (void*)k_pcg_halo<0>;
+    }
     if (S->opt.precision == PF2_PRECISION_MIXED) {
         if (S->part_local)
             return S->opt.precond == PF2_PRECOND_IC ? (void*)k_pcg_part_mixed<true, true>
@@ -3528,12 +3744,13 @@ static pf2_status factorize(pf2_solver* S, const pf2_csr* A, cudaStream_t st) {
                                                                                     S->fsym.p);
         PF2_LAUNCH_CHECK();
         if (S->part) {
-            k_gather_values<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(
-                S->nnz, S->fsym.p, S->q_fmap.p, S->q_f.p);
+            const long long ne = S->halo ? S->halo_entries : S->nnz;
+            k_gather_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(
+                ne, S->fsym.p, S->q_fmap.p, S->q_f.p);
             PF2_LAUNCH_CHECK();
             if (S->q_f32.p) {
-                k_to_float<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(S->nnz, S->q_f.p,
-                                                                                                S->q_f32.p);
+                k_to_float<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, S->q_f.p,
+                                                                                            S->q_f32.p);
                 PF2_LAUNCH_CHECK();
             }
         }
@@ -3635,19 +3852,18 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     const int applies = max_applies(S);
     if (S->part && !precond_only) {
         // A's values in Q order for this solve's matrix; t and z start as pending markers
-        k_gather_values<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(
-            S->nnz, a.A.val, S->q_amap.p, S->q_val.p);
+        const long long ne = S->halo ? S->halo_entries : S->nnz;
+        k_gather_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, a.A.val, S->q_amap.p,
+                                                                                         S->q_val.p);
         PF2_LAUNCH_CHECK();
-        if (uses_tri(S)) {
-            PF2_CUDA(cudaMemsetAsync(S->q_gt.p, 0xff, S->q_gt.bytes(), st));
-            PF2_CUDA(cudaMemsetAsync(S->q_gz.p, 0xff, S->q_gz.bytes(), st));
-        }
+        if (S->q_gt.p) PF2_CUDA(cudaMemsetAsync(S->q_gt.p, 0xff, S->q_gt.bytes(), st));
+        if (S->q_gz.p) PF2_CUDA(cudaMemsetAsync(S->q_gz.p, 0xff, S->q_gz.bytes(), st));
         if (S->q_val32.p) {
-            k_to_float<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(S->nnz, S->q_val.p,
-                                                                                            S->q_val32.p);
+            k_to_float<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, S->q_val.p,
+                                                                                        S->q_val32.p);
             PF2_LAUNCH_CHECK();
             PF2_CUDA(cudaMemsetAsync(S->q_gt32.p, 0xff, S->q_gt32.bytes(), st));
-            PF2_CUDA(cudaMemsetAsync(S->q_gz32.p, 0xff, S->q_gz32.bytes(), st));
+            if (S->q_gz32.p) PF2_CUDA(cudaMemsetAsync(S->q_gz32.p, 0xff, S->q_gz32.bytes(), st));
         }
         a.part = PartCg{ S->part_P, S->part_R, S->part_ng, S->q_s.p, S->q_rp.p, S->q_col.p, S->q_diag.p, S->q_a.p,
                          S->q_bnd.p, S->q_val.p, S->q_f.p, S->q_x.p, S->q_gp.p, S->q_gt.p, S->q_gz.p,
@@ -3655,7 +3871,14 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
         PF2_CUDA(cudaMemsetAsync(S->bar.p, 0, 2 * sizeof(unsigned), st));
         PF2_CUDA(cudaMemsetAsync(S->err.p, 0, sizeof(int), st));
         PF2_CUDA(cudaMemsetAsync(S->rec.p, 0, 5 * sizeof(int), st));
-        void* args[] = { &a };
+        PartHalo h{};
+        if (S->halo)
+            h = PartHalo{ S->part_P, S->part_ng, S->part_R, S->halo_RL, S->q_s.p, S->h_hs.p, S->h_hoff.p, S->h_hq.p,
+                          S->h_foff.p, S->h_fl.p, S->h_fg.p, S->h_zoff.p, S->h_zl.p, S->h_zg.p, S->h_r1off.p,
+                          S->h_r1.p, S->h_ebase.p, S->h_rp.p, S->h_dg.p, S->h_pub.p, S->h_lcol.p, S->q_a.p,
+                          S->q_val.p, S->q_f.p, S->q_x.p, S->q_gp.p, S->q_gt.p, S->q_val32.p, S->q_f32.p,
+                          S->q_gp32.p, S->q_gt32.p };
+        void* args[] = { &a, &h };
         PF2_COOP_LAUNCH(part_kernel(S), dim3(S->part_P), dim3(kPartThreads), args, S->part_smem, st);
         return PF2_OK;
     }
