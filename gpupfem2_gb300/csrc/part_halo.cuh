@@ -6,11 +6,10 @@
 // inputs, so the same bits as their owner), and an iteration has no wait inside a sweep:
 //   F rows: other parts' rows that the part's forward sweep reads, closed under the sweep's
 //           dependencies (lower groups).  Their r lives here too: r -= alpha q with the owner's
-//           q, which owners publish before the p.q reduction and which is read behind its
-//           barrier.
+//           q, which owners publish before the p.q reduction and which is read beside it.
 //   Z rows: the neighbour rows of the part's rows (ring 1, whose p the SpMV reads), closed under
 //           the backward sweep's dependencies (higher groups).  Their forward result t is either
-//           computed here (F rows) or read once from the owner, polled on the pending marker.
+//           computed here (F rows) or read once from the owner.
 // p on ring 1 follows from its z, so the direction needs no exchange.  Per iteration: SpMV;
 // reduction of p.q; forward sweep; (IC(0): arrival at the t.t reduction;) t of the Z rows that
 // are not F rows; backward sweep; reduction (IC(0): the wait alone).
@@ -19,20 +18,44 @@
 // group's rows as F only, F and Z, Z only.  Columns are local (16 bits), so no lookup or branch
 // tells own entries from others'.
 //
-// What bounds it: FP64 issue of the rows (SpMV, sweeps) plus two reductions' latency.  Measured,
-// us per iteration, k_pcg_part -> this kernel (same bits), cylinder pressure matrix:
-//   125,364 rows: IC(0) 29.7 -> 21.8, ILU(0) 34.4 -> 22.5, mixed IC(0) 28.3 -> 19.0, Jacobi 16.1 -> 14.9
-//   499,288 rows: IC(0) 43.1 -> 39.5, ILU(0) 45.2 -> 40.4, mixed IC(0) 34.1 -> 27.2, Jacobi 28.3 -> 24.9
+// Rows are taken in slices of 32 by warps (slice i of the SpMV, and of each group of a sweep, by
+// warp i mod kHaloWarps).  A slice's entries, entry k of its rows side by side, lie in items of
+// at most KC entry rows, and a warp's items lie in the order in which it uses them (forward
+// sweep, backward sweep, SpMV).  A sweep slice's first entry row holds the inverse pivots and, as
+// columns, the rows themselves.  Two forms (RES): a part whose values and columns fit in shared
+// memory beside its vectors (up to ~900 rows of a triangular mesh) loads them once, by bulk
+// copies; a larger part reads them from L2 in every iteration, coalesced, a slice's loads issued
+// together and (sweeps) before the barrier that its row sums wait for.
+//
+// What bounds it: FP64 issue and the latency between grid-wide steps.  GB300 takes 64 clocks per
+// FP64 warp instruction on an SM sub-partition, with no latency beyond that, so a few warps per
+// sub-partition keep the pipe busy and more only make barriers and block sums dearer
+// (__syncthreads 75 clocks at 1,024 threads, 43 at 512).  Reductions use few dependent FP64
+// instructions (a butterfly step is 128 clocks, a division 666, a square root 600: the tests
+// compare squares).  Measured, us per iteration, the kernel with waits in the sweeps -> this one,
+// cylinder pressure matrix:
+//   125,364 rows: IC(0) 29.8 -> 14.1, mixed IC(0) 27.5 -> 12.1, Jacobi 15.9 -> 9.9
+//   499,288 rows: IC(0) 43.5 -> 36.5, mixed IC(0) 34.1 -> 23.9, Jacobi 28.4 -> 20.6
+// (FP64 issue alone: ~18 us per IC(0) iteration at 499,288 rows, ~5 at 125,364.)
 #pragma once
 
 namespace pf2 {
+
+constexpr int kHaloWarps = 16;
+constexpr int kHaloThreads = 32 * kHaloWarps;
+constexpr unsigned short kHaloNone = 0xffff;   // padding row of a slice
+constexpr unsigned short kHaloPubT = 0x8000;   // the row's t is published
+constexpr int kHaloMaxLocal = 0x7fff;          // local rows of a part
+constexpr int kHaloItem = 8;                   // entry rows per item
+constexpr unsigned char kHaloLast = 0x80;      // item byte: entry rows, and whether it ends its slice
 
 struct PartHalo {
     int P, ng;
     int R;                      // largest number of own rows
     int RL;                     // largest number of local rows (own + halo)
+    int TL;                     // largest number of items of a part
+    int E;                      // largest number of entry rows of a part (resident)
     const int* qs;              // own group starts (PartCg::qs)
-    const int* hs;              // [(part * ng + group) * 4]: halo rows' F start, Z start, F end, Z end
     const int* hoff;            // P + 1: the parts' halo rows in hq
     const int* hq;              // halo row -> row in Q order
     const int* foff;            // P + 1: the parts' F rows in fl, fg (local index, row in Q order)
@@ -43,78 +66,184 @@ struct PartHalo {
     const int* zg;
     const int* r1off;           // P + 1: the parts' ring-1 rows in r1
     const unsigned short* r1;   // local indices of ring-1 rows
-    const int* ebase;           // P + 1: the parts' first entry
-    const int* rp;              // part k: np + nh + 1 entry offsets at qs[k ng] + hoff[k] + k
-    const unsigned char* dg;    // offset of the diagonal in the row's entries, at qs[k ng] + hoff[k]
-    const unsigned char* pub;   // own rows: bit 0 q (and r) is read by another part, bit 1 t is
-    const unsigned short* lcol; // local columns
-    const int* qa;              // Q row -> row of A
+    const unsigned char* pub;   // own rows: 1 where q (and r) is read by another part
+    const int* ioff;            // P + 1: the parts' items in item
+    const unsigned char* item;  // entry rows of an item | kHaloLast
+    const int* wit;             // at (part * kHaloWarps + warp) * 2: the warp's first item (from the part's)
+                                // and its first SpMV item
+    const int* went;            // P * kHaloWarps + 1: the warps' first entry row in the streams
+    const int* gsl;             // part k, at k (2 ng): numbers of slices of the forward and backward groups
+    const unsigned short* col;  // streams: 32 entries per entry row
     const double* val;
-    const double* f;
+    const int* qa;              // Q row -> row of A
+    const double* diag;         // Jacobi / none: diagonal entries of the local rows, at qs[k ng] + hoff[k]
     double* x;
-    double* gq;                 // published q (r at the start and at refinements), Q order
-    double* gt;                 // 2 n: published t, the sweeps alternate halves (pending markers)
     const float* val32;
-    const float* f32;
-    float* gq32;
-    float* gt32;
+    unsigned long long* gq;     // packets (zeroed before the launch): published q (r at the start and
+    unsigned long long* gt;     // at refinements) and t; 2 n each, alternate exchanges take alternate halves
 };
 
 template <class V> struct HaloVecs;
 template <> struct HaloVecs<double> {
     __device__ static const double* val(const PartHalo& C) { return C.val; }
-    __device__ static const double* f(const PartHalo& C) { return C.f; }
-    __device__ static double* gq(const PartHalo& C) { return C.gq; }
-    __device__ static double* gt(const PartHalo& C) { return C.gt; }
 };
 template <> struct HaloVecs<float> {
     __device__ static const float* val(const PartHalo& C) { return C.val32; }
-    __device__ static const float* f(const PartHalo& C) { return C.f32; }
-    __device__ static float* gq(const PartHalo& C) { return C.gq32; }
-    __device__ static float* gt(const PartHalo& C) { return C.gt32; }
+};
+
+// ------------------------------------------------------------ exchanges
+// A value with the number of its exchange in one 16-byte (FP64) or 8-byte (FP32) word, stored and
+// loaded whole: the reader sees that the value is the one it waits for, so neither a fence nor a
+// counter orders an exchange (an arrival with a gpu-scope release costs ~700 clocks, the poll of
+// a counter and the read behind it ~700 each).  Alternate exchanges use alternate halves, so a
+// half is written again two exchanges later, when its readers have long contributed to a
+// reduction that the writer has waited for, with values that depend on what they read.
+template <class V> struct HaloPacket;
+template <> struct HaloPacket<double> {
+    static constexpr int kWords = 2;
+    __device__ static __forceinline__ void put(unsigned long long* p, double v, unsigned seq) {
+        asm volatile(
+            "{\n\t.reg .b128 x;\n\tmov.b128 x, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], x;\n\t}"
+            :
+            : "l"(p), "l"(__double_as_longlong(v)), "l"((long long)seq)
+            : "memory");
+    }
+    __device__ static __forceinline__ bool get(const unsigned long long* p, double& v, unsigned seq) {
+        long long a, b;
+        asm volatile(
+            "{\n\t.reg .b128 x;\n\tld.relaxed.gpu.global.b128 x, [%2];\n\tmov.b128 {%0, %1}, x;\n\t}"
+            : "=l"(a), "=l"(b)
+            : "l"(p)
+            : "memory");
+        v = __longlong_as_double(a);
+        return (unsigned)b == seq;
+    }
+};
+template <> struct HaloPacket<float> {
+    static constexpr int kWords = 1;
+    __device__ static __forceinline__ void put(unsigned long long* p, float v, unsigned seq) {
+        const unsigned long long x = (unsigned long long)seq << 32 | __float_as_uint(v);
+        asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+    }
+    __device__ static __forceinline__ bool get(const unsigned long long* p, float& v, unsigned seq) {
+        unsigned long long x;
+        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(x) : "l"(p) : "memory");
+        v = __uint_as_float((unsigned)x);
+        return (unsigned)(x >> 32) == seq;
+    }
+};
+
+// The packet's value once it has arrived (bounded; a wait that runs out records DEV_TIMEOUT and
+// yields 0: the kernel returns at its next grid-wide step).
+template <class V>
+__device__ __forceinline__ V halo_settle(const unsigned long long* p, bool here, V v, unsigned seq, const GridBarrier& b,
+                                         int kind, int what) {
+    long long polls = 0;
+    while (!here) {
+        if (++polls > (b.max_polls > 0 ? b.max_polls : kFlagPolls)) {
+            atomicExch(b.err, (int)DEV_TIMEOUT);
+            record_timeout(b.rec, kind, kind == 1 ? (int)blockIdx.x : what, kind == 1 ? (int)seq : what, (int)seq, 0);
+            return V(0);
+        }
+        if ((polls & 255) == 0 && *(volatile int*)b.err != 0) return V(0);
+        here = HaloPacket<V>::get(p, v, seq);
+    }
+    return v;
+}
+
+// ------------------------------------------------------------ resident entries
+__device__ __forceinline__ unsigned halo_smem_u32(const void* p) {
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+
+constexpr long long kHaloCopyPolls = 1ll << 22;
+
+// Bounded wait for phase `parity` of an mbarrier.
+__device__ __forceinline__ bool halo_mbar_wait(unsigned mbar, unsigned parity) {
+    for (long long i = 0; i < kHaloCopyPolls; ++i) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(mbar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void halo_bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned mbar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :
+                 : "r"(dst), "l"(src), "r"(bytes), "r"(mbar)
+                 : "memory");
+}
+
+// A warp's items in order, from this lane's values and columns of the first entry row on.
+template <class V, bool RES>
+struct HaloItems {
+    const unsigned char *i0, *item;
+    const V *v0, *v;
+    const unsigned short *c0, *c;
+    __device__ __forceinline__ void begin() {
+        item = i0;
+        v = v0;
+        c = c0;
+    }
+    __device__ __forceinline__ V value(int k) const { return RES ? v[32 * k] : __ldg(&v[32 * k]); }
+    __device__ __forceinline__ int column(int k) const { return RES ? c[32 * k] : __ldg(&c[32 * k]); }
+    __device__ __forceinline__ void next() {
+        const int n = (*item++ & 0x7f) * 32;
+        v += n;
+        c += n;
+    }
 };
 
 // A part in shared memory: r, p, q, t (z shares t's array; Jacobi / none: t = 1 / a_ii and z
 // apart) over the local rows, the mixed solver's update d over the own rows, the reduction
-// scratch, the rows' entry offsets and diagonals, the own rows' publication flags.  val, f and
-// lcol point at the part's first entry.
-template <class V>
+// scratch, the groups' slice counts, the own rows' publication flags, the item bytes and (RES)
+// the entry rows.
+template <class V, bool RES>
 struct HaloSm {
     V *r, *p, *q, *t, *z, *d;
     double* red;
-    const int* rp;
-    const unsigned char *dg, *pub;
-    const V *val, *f;
-    const unsigned short* lcol;
+    const int* gsl;
+    const unsigned char* pub;
     const int* hq;   // the part's halo rows
-    const int* hs;   // the part's group table
-    const int* qs;   // the part's group starts
-    int p0, np, nh, n, par;
+    int p0, np, nh, n, nsl;
+    unsigned target; // arrivals that complete the next grid barrier
+    unsigned qs, ts, rs;  // numbers of the last exchanges of q and t and of the last reduction
     // the exchanged rows of this thread's first pass (fetches without a look-up load before them)
     int nf, f_l, f_g, nz, z_l, z_g;
+    HaloItems<V, RES> items;
 };
 
+constexpr int kHaloRedDoubles = 2 * kHaloThreads;
 __host__ __device__ constexpr size_t halo_vec_bytes(int R, int RL, bool tri, size_t vsz, bool mixed) {
-    return ((size_t)(4 + (tri ? 0 : 1)) * RL * vsz + (mixed ? (size_t)R * vsz : 0) + 15) / 16 * 16;
+    return ((size_t)(4 + (tri ? 0 : 1)) * RL * vsz + (mixed ? (size_t)R * vsz : 0) + 127) / 128 * 128;
 }
-__host__ __device__ constexpr size_t halo_smem_bytes(int R, int RL, bool tri, size_t vsz, bool mixed) {
-    return (halo_vec_bytes(R, RL, tri, vsz, mixed) + sizeof(double) * 2 * kPartThreads +
-            sizeof(int) * ((size_t)RL + 1) + (size_t)RL + (size_t)R + 15) / 16 * 16;
+// (E: the part's entry rows when they are resident, else 0)
+__host__ __device__ constexpr size_t halo_smem_bytes(int R, int RL, int TL, int ng, bool tri, size_t vsz, bool mixed,
+                                                     int E) {
+    return (halo_vec_bytes(R, RL, tri, vsz, mixed) + (size_t)E * 32 * (vsz + 2) + sizeof(double) * kHaloRedDoubles +
+            sizeof(int) * 2 * (size_t)ng + (size_t)R + (size_t)TL + 15) / 16 * 16;
 }
 
-template <class V>
-__device__ __forceinline__ HaloSm<V> halo_sm(const PartHalo& C, int n, unsigned char* base, bool tri, bool mixed) {
-    HaloSm<V> S;
-    const int k = blockIdx.x;
+template <class V, bool RES>
+__device__ __forceinline__ HaloSm<V, RES> halo_sm(const PartHalo& C, int n, unsigned char* base, bool tri, bool mixed,
+                                                  int* err) {
+    __shared__ unsigned long long mbar;
+    HaloSm<V, RES> S;
+    const int k = blockIdx.x, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     S.n = n;
-    S.qs = C.qs + k * C.ng;
-    S.p0 = S.qs[0];
-    S.np = S.qs[C.ng] - S.p0;
+    S.p0 = C.qs[k * C.ng];
+    S.np = C.qs[(k + 1) * C.ng] - S.p0;
+    S.nsl = (S.np + 31) / 32;
     const int h0 = C.hoff[k];
     S.nh = C.hoff[k + 1] - h0;
     S.hq = C.hq + h0;
-    S.hs = C.hs + 4 * k * C.ng;
-    S.par = 0;
+    S.target = S.qs = S.ts = S.rs = 0;
     V* v = reinterpret_cast<V*>(base);
     S.r = v;
     S.p = v + C.RL;
@@ -122,336 +251,592 @@ __device__ __forceinline__ HaloSm<V> halo_sm(const PartHalo& C, int n, unsigned 
     S.t = v + 3 * C.RL;
     S.z = tri ? S.t : v + 4 * C.RL;
     S.d = mixed ? v + (tri ? 4 : 5) * C.RL : nullptr;
-    S.red = reinterpret_cast<double*>(base + halo_vec_bytes(C.R, C.RL, tri, sizeof(V), mixed));
-    int* rp = reinterpret_cast<int*>(S.red + 2 * kPartThreads);
-    unsigned char* dg = reinterpret_cast<unsigned char*>(rp + C.RL + 1);
-    unsigned char* pub = dg + C.RL;
-    const int e0 = C.ebase[k];
-    S.val = HaloVecs<V>::val(C) + e0;
-    S.f = HaloVecs<V>::f(C) ? HaloVecs<V>::f(C) + e0 : nullptr;
-    S.lcol = C.lcol + e0;
-    const int nl = S.np + S.nh;
-    const int* grp = C.rp + S.p0 + h0 + k;
-    const unsigned char* gdg = C.dg + S.p0 + h0;
-    for (int l = threadIdx.x; l <= nl; l += kPartThreads) rp[l] = __ldg(&grp[l]);
-    for (int l = threadIdx.x; l < nl; l += kPartThreads) dg[l] = __ldg(&gdg[l]);
-    for (int l = threadIdx.x; l < S.np; l += kPartThreads) pub[l] = __ldg(&C.pub[S.p0 + l]);
-    S.rp = rp;
-    S.dg = dg;
+    unsigned char* entries = base + halo_vec_bytes(C.R, C.RL, tri, sizeof(V), mixed);
+    S.red = reinterpret_cast<double*>(entries + (RES ? (size_t)C.E * 32 * (sizeof(V) + 2) : 0));
+    int* gsl = reinterpret_cast<int*>(S.red + kHaloRedDoubles);
+    unsigned char* pub = reinterpret_cast<unsigned char*>(gsl + 2 * C.ng);
+    unsigned char* item = pub + C.R;
+    const int i0 = C.ioff[k], ni = C.ioff[k + 1] - i0;
+    for (int i = tid; i < ni; i += kHaloThreads) item[i] = C.item[i0 + i];
+    for (int i = tid; i < 2 * C.ng; i += kHaloThreads) gsl[i] = C.gsl[k * 2 * C.ng + i];
+    for (int l = tid; l < S.np; l += kHaloThreads) pub[l] = C.pub[S.p0 + l];
+    S.gsl = gsl;
     S.pub = pub;
+    S.items.i0 = item + C.wit[2 * (k * kHaloWarps + w)];
+    const int ew = C.went[k * kHaloWarps + w];  // the warp's first entry row
+    if constexpr (RES) {
+        // all entry rows of the part, values then columns, in bulk copies of 16 KB
+        const unsigned m = halo_smem_u32(&mbar);
+        if (tid == 0) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(m));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncthreads();
+        const int e0 = C.went[k * kHaloWarps], e1 = C.went[(k + 1) * kHaloWarps];
+        unsigned char* cols = entries + (size_t)C.E * 32 * sizeof(V);
+        if (tid == 0) {
+            const unsigned vb = (unsigned)(e1 - e0) * 32 * sizeof(V), cb = (unsigned)(e1 - e0) * 64;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(m), "r"(vb + cb) : "memory");
+            const unsigned char* gv = reinterpret_cast<const unsigned char*>(HaloVecs<V>::val(C) + (size_t)e0 * 32);
+            const unsigned char* gc = reinterpret_cast<const unsigned char*>(C.col + (size_t)e0 * 32);
+            for (unsigned o = 0; o < vb; o += 16384) halo_bulk_copy(halo_smem_u32(entries) + o, gv + o, min(16384u, vb - o), m);
+            for (unsigned o = 0; o < cb; o += 16384) halo_bulk_copy(halo_smem_u32(cols) + o, gc + o, min(16384u, cb - o), m);
+        }
+        if (!halo_mbar_wait(m, 0)) atomicExch(err, (int)DEV_TIMEOUT);
+        S.items.v0 = reinterpret_cast<const V*>(entries) + (size_t)(ew - e0) * 32 + lane;
+        S.items.c0 = reinterpret_cast<const unsigned short*>(cols) + (size_t)(ew - e0) * 32 + lane;
+    } else {
+        S.items.v0 = HaloVecs<V>::val(C) + (size_t)ew * 32 + lane;
+        S.items.c0 = C.col + (size_t)ew * 32 + lane;
+    }
+    S.items.begin();
     const int f0 = C.foff[k], z0 = C.zoff[k];
     S.nf = C.foff[k + 1] - f0;
     S.nz = C.zoff[k + 1] - z0;
     S.f_l = S.f_g = S.z_l = S.z_g = 0;
-    if ((int)threadIdx.x < S.nf) {
-        S.f_l = C.fl[f0 + threadIdx.x];
-        S.f_g = C.fg[f0 + threadIdx.x];
+    const int fi = tid - 64;  // warps 0 and 1 sum the partials while the others fetch
+    if (fi >= 0 && fi < S.nf) {
+        S.f_l = C.fl[f0 + fi];
+        S.f_g = C.fg[f0 + fi];
     }
-    if ((int)threadIdx.x < S.nz) {
-        S.z_l = C.zl[z0 + threadIdx.x];
-        S.z_g = C.zg[z0 + threadIdx.x];
+    if (tid < S.nz) {
+        S.z_l = C.zl[z0 + tid];
+        S.z_g = C.zg[z0 + tid];
     }
+    __syncthreads();  // the tables are in place
     return S;
 }
 
 // Row in Q order of local row l.
-template <class V>
-__device__ __forceinline__ int halo_global(const HaloSm<V>& S, int l) {
+template <class V, bool RES>
+__device__ __forceinline__ int halo_global(const HaloSm<V, RES>& S, int l) {
     return l < S.np ? S.p0 + l : __ldg(&S.hq[l - S.np]);
 }
 
-// q = A p over the part's rows (part_spmv's arithmetic); the rows that are F rows elsewhere
-// are published.  Returns the thread's p.q terms in FP64.
+// ------------------------------------------------------------ grid-wide steps
+// GridBarrier's counter with the arrivals counted here (`target` grows by the arrivals of each
+// step), so no read of the counter precedes an arrival, and the error word is loaded beside the
+// first poll instead of after the last.  Thread 0 waits; false on a timeout or an error.
+template <bool ACQUIRE>
+__device__ __forceinline__ bool halo_poll(const GridBarrier& b, unsigned target) {
+    const long long limit = b.max_polls > 0 ? b.max_polls : kBarrierPolls;
+    int e = *(volatile int*)b.err;
+    long long polls = 0;
+    unsigned c;
+    while ((int)((c = ACQUIRE ? ld_acquire_gpu(b.count) : ld_relaxed_gpu(b.count)) - target) < 0) {
+        if (++polls > limit) {
+            atomicExch(b.err, (int)DEV_TIMEOUT);
+            record_timeout(b.rec, 1, (int)blockIdx.x, (int)(target / gridDim.x) - 1, (int)c, 0);
+            return false;
+        }
+        if ((polls & 255) == 0 && (e = *(volatile int*)b.err) != 0) return false;
+    }
+    return e == 0;
+}
+
+template <class V, bool RES>
+__device__ __forceinline__ bool halo_sync(const GridBarrier& b, HaloSm<V, RES>& S) {
+    S.target += gridDim.x;
+    __syncthreads();
+    int ok = 1;
+    if (threadIdx.x == 0) {
+        arrive_release_gpu(b.count);
+        ok = halo_poll<true>(b, S.target);
+    }
+    return __syncthreads_and(ok);
+}
+
+// Arrival at a reduction of two values: 64 threads per value add eight threads' values each,
+// then one warp per value adds two and a butterfly; its lane 0 puts the block's sum.
+template <class V, bool RES>
+__device__ __forceinline__ unsigned long long* halo_slot(const GridBarrier& b, const HaloSm<V, RES>& S, int value, int block) {
+    return reinterpret_cast<unsigned long long*>(b.part) + 2 * (((S.rs & 1u) * 2 + value) * (size_t)gridDim.x + block);
+}
+template <class V, bool RES>
+__device__ __forceinline__ void halo_arrive(const GridBarrier& b, HaloSm<V, RES>& S, double v0, double v1) {
+    constexpr int T = kHaloThreads, Q = 64, M = T / Q;
+    static_assert(T % Q == 0 && M >= 2, "block size of the tree");
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    S.red[tid] = v0;
+    S.red[T + tid] = v1;
+    __syncthreads();
+    if (tid < 2 * Q) {
+        double* c = S.red + (tid / Q) * T + tid % Q;
+        double s = c[0];
+#pragma unroll
+        for (int i = 1; i < M; ++i) s += c[i * Q];
+        c[0] = s;
+    }
+    __syncthreads();
+    ++S.rs;
+    if (w < 2) {
+        const double* c = S.red + w * T + lane;
+        const double s = warp_sum(c[0] + c[32]);
+        if (lane == 0) {
+            HaloPacket<double>::put(halo_slot(b, S, w, blockIdx.x), s, S.rs);
+            asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" : : "l"(b.count) : "memory");
+        }
+    }
+    S.target += 2 * gridDim.x;
+}
+
+// Blocks from which on a wait watches the arrival counter (one word, no ordering asked of it)
+// before it reads the packets: every block polling every block's packets slows the stores it
+// waits for (us per iteration without and with the counter: 152 blocks, 125,364 rows, Jacobi
+// 11.0 / 10.0, IC(0) 16.4 / 14.1; 32 blocks, 16,705 rows, Jacobi 9.0 / 9.7, IC(0) 12.9 / 13.4).
+constexpr unsigned kHaloCountBlocks = 64;
+
+// The wait: warp j takes value j's sums of all blocks, adds them in block order (lane l: l, l +
+// 32, ...; butterfly) and its lane 0 runs post(j, total, out) (out: the block's scalars), while
+// side() runs on the warps from 2 on.  sh: totals at [16 + j], out at [24].  watch: the others'
+// sums may be a while off.  False on a timeout or an error anywhere.
+template <class V, bool RES, class Post, class Side>
+__device__ __forceinline__ bool halo_wait(const GridBarrier& b, HaloSm<V, RES>& S, double* sh, bool watch, Post post,
+                                          Side side) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    int ok = 1;
+    if (w < 2) {
+        if (watch && gridDim.x >= kHaloCountBlocks) {
+            if (lane == 0) ok = halo_poll<false>(b, S.target);
+            __syncwarp();
+        }
+        if (tid == 0) ok = ok && *(volatile int*)b.err == 0;
+        constexpr int N = 5;
+        double t = 0.0;
+        for (int q0 = lane; q0 < (int)gridDim.x; q0 += 32 * N) {
+            double v[N];
+            bool here[N];
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int q = q0 + 32 * i;
+                here[i] = true;
+                v[i] = 0.0;
+                if (q < (int)gridDim.x) here[i] = HaloPacket<double>::get(halo_slot(b, S, w, q), v[i], S.rs);
+            }
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (q0 + 32 * i < (int)gridDim.x)
+                    t += halo_settle(halo_slot(b, S, w, q0 + 32 * i), here[i], v[i], S.rs, b, 1, 0);
+        }
+        __syncwarp();
+        t = warp_sum(t);
+        if (lane == 0) {
+            sh[16 + w] = t;
+            post(w, t, sh + 24);
+        }
+        if (tid == 0) ok = ok && *(volatile int*)b.err == 0;
+    } else {
+        side();
+    }
+    return __syncthreads_and(ok);
+}
+
+template <class V, bool RES, class Post, class Side>
+__device__ __forceinline__ bool halo_reduce(const GridBarrier& b, HaloSm<V, RES>& S, double v0, double v1, double* sh,
+                                            Post post, Side side) {
+    halo_arrive(b, S, v0, v1);
+    return halo_wait(b, S, sh, true, post, side);
+}
+
+// ------------------------------------------------------------ rows
+// The entry rows [lead, n) of an item in registers, and s +- sum_k f_k x[col_k] over them in
+// order as a chain of fused multiply-adds.  n is uniform over the warp: the switches keep the
+// loads of a slice together and the chain free of tests.
 template <class V>
-__device__ __forceinline__ double halo_spmv(const PartHalo& C, const HaloSm<V>& S) {
-    V* gq = HaloVecs<V>::gq(C);
+struct HaloEntries {
+    V f[kHaloItem];
+    int c[kHaloItem];
+};
+template <int N, class V, bool RES>
+__device__ __forceinline__ void halo_load_n(const HaloItems<V, RES>& I, int lead, HaloEntries<V>& E) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) E.f[k] = I.value(lead + k);
+#pragma unroll
+    for (int k = 0; k < N; ++k) E.c[k] = I.column(lead + k);
+}
+template <int N, bool NEG, class V>
+__device__ __forceinline__ V halo_chain_n(const HaloEntries<V>& E, const V* x, V s) {
+    V y[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) y[k] = x[E.c[k]];
+#pragma unroll
+    for (int k = 0; k < N; ++k) s = fma_rn(NEG ? -E.f[k] : E.f[k], y[k], s);
+    return s;
+}
+#define PF2_HALO_CASES(X) \
+    case 1: X(1); break;  \
+    case 2: X(2); break;  \
+    case 3: X(3); break;  \
+    case 4: X(4); break;  \
+    case 5: X(5); break;  \
+    case 6: X(6); break;  \
+    case 7: X(7); break;  \
+    case 8: X(8); break;
+template <class V, bool RES>
+__device__ __forceinline__ void halo_load(const HaloItems<V, RES>& I, int lead, int n, HaloEntries<V>& E) {
+    switch (n - lead) {
+#define PF2_X(N) halo_load_n<N>(I, lead, E)
+        PF2_HALO_CASES(PF2_X)
+#undef PF2_X
+    }
+}
+template <bool NEG, class V>
+__device__ __forceinline__ V halo_chain(int n, const HaloEntries<V>& E, const V* x, V s) {
+    switch (n) {
+#define PF2_X(N) s = halo_chain_n<N, NEG>(E, x, s)
+        PF2_HALO_CASES(PF2_X)
+#undef PF2_X
+    }
+    return s;
+}
+// ... straight from the resident entry rows
+template <int N, bool NEG, class V>
+__device__ __forceinline__ V halo_chain_at_n(const V* v, const unsigned short* c, const V* x, V s) {
+    V f[N], y[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) f[k] = v[32 * k];
+#pragma unroll
+    for (int k = 0; k < N; ++k) y[k] = x[c[32 * k]];
+#pragma unroll
+    for (int k = 0; k < N; ++k) s = fma_rn(NEG ? -f[k] : f[k], y[k], s);
+    return s;
+}
+template <bool NEG, class V>
+__device__ __forceinline__ V halo_chain_at(int n, const V* v, const unsigned short* c, const V* x, V s) {
+    switch (n) {
+#define PF2_X(N) s = halo_chain_at_n<N, NEG>(v, c, x, s)
+        PF2_HALO_CASES(PF2_X)
+#undef PF2_X
+    }
+    return s;
+}
+#undef PF2_HALO_CASES
+
+// The packet of row j in the half of exchange seq.
+template <class V, bool RES>
+__device__ __forceinline__ unsigned long long* halo_row(unsigned long long* g, const HaloSm<V, RES>& S, unsigned seq, int j) {
+    return g + ((size_t)(seq & 1u) * S.n + j) * HaloPacket<V>::kWords;
+}
+
+// q = A p over the part's rows (each row's entries in A's order); the rows that are F rows
+// elsewhere are published.  Returns the thread's p.q terms in FP64.
+template <class V, bool RES>
+__device__ __forceinline__ double halo_spmv(const PartHalo& C, HaloSm<V, RES>& S) {
+    unsigned long long* gq = halo_row(C.gq, S, ++S.qs, S.p0);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double pq = 0.0;
-    for (int l = threadIdx.x; l < S.np; l += kPartThreads) {
-        const int s = S.rp[l], e = S.rp[l + 1];
+#pragma unroll 1
+    for (int s = w; s < S.nsl; s += kHaloWarps) {
+        const int l = s * 32 + lane;
         V acc = V(0);
-        for (int k = s; k < e; ++k) acc += __ldg(&S.val[k]) * S.p[__ldg(&S.lcol[k])];
-        S.q[l] = acc;
-        if (S.pub[l] & 1) __stcg(&gq[S.p0 + l], acc);
-        pq += (double)S.p[l] * (double)acc;
+        unsigned char it;
+        do {
+            it = *S.items.item;
+            if constexpr (RES) {
+                acc = halo_chain_at<false>(it & 0x7f, S.items.v, S.items.c, S.p, acc);
+            } else {
+                HaloEntries<V> E;
+                halo_load(S.items, 0, it & 0x7f, E);
+                acc = halo_chain<false>(it & 0x7f, E, S.p, acc);
+            }
+            S.items.next();
+        } while (!(it & kHaloLast));
+        if (l < S.np) {
+            S.q[l] = acc;
+            if (S.pub[l]) HaloPacket<V>::put(gq + (size_t)l * HaloPacket<V>::kWords, acc, S.qs);
+            pq += (double)S.p[l] * (double)acc;
+        }
     }
     return pq;
 }
 
-// dst of the part's F rows from the published values (behind a grid barrier).
-template <class V>
-__device__ __forceinline__ void halo_fetch(const PartHalo& C, const HaloSm<V>& S, V* dst) {
-    const V* gq = HaloVecs<V>::gq(C);
-    if ((int)threadIdx.x < S.nf) dst[S.f_l] = __ldcg(&gq[S.f_g]);
-    for (int i = threadIdx.x + kPartThreads, f0 = __ldg(&C.foff[blockIdx.x]); i < S.nf; i += kPartThreads)
-        dst[__ldg(&C.fl[f0 + i])] = __ldcg(&gq[__ldg(&C.fg[f0 + i])]);
+// dst of the part's F rows from the last published values, by the threads from 64 on.
+template <class V, bool RES>
+__device__ __forceinline__ void halo_fetch(const PartHalo& C, const HaloSm<V, RES>& S, const GridBarrier& b, V* dst) {
+    const unsigned long long* gq = halo_row(C.gq, S, S.qs, 0);
+    const int fi = (int)threadIdx.x - 64;
+    if (fi < 0) return;
+    auto take = [&](int l, int j) {
+        const unsigned long long* p = gq + (size_t)j * HaloPacket<V>::kWords;
+        V v;
+        const bool here = HaloPacket<V>::get(p, v, S.qs);
+        dst[l] = halo_settle(p, here, v, S.qs, b, 2, j);
+    };
+    if (fi < S.nf) take(S.f_l, S.f_g);
+    for (int i = fi + kHaloThreads - 64, f0 = __ldg(&C.foff[blockIdx.x]); i < S.nf; i += kHaloThreads - 64)
+        take(__ldg(&C.fl[f0 + i]), __ldg(&C.fg[f0 + i]));
 }
 
-// r of the own rows published for the parts that hold them as F rows.
-template <class V>
-__device__ __forceinline__ void halo_publish_r(const PartHalo& C, const HaloSm<V>& S) {
-    V* gq = HaloVecs<V>::gq(C);
-    for (int l = threadIdx.x; l < S.np; l += kPartThreads)
-        if (S.pub[l] & 1) __stcg(&gq[S.p0 + l], S.r[l]);
+// A slice of a sweep: head(row) gives the chain's start for the lane's row (kHaloNone: padding;
+// it may wait for a barrier), tail(row, sum, pivot) takes s - sum_k f_k x[col_k] over the row's
+// entries in entry order.
+template <class V, bool RES, class Head, class Tail>
+__device__ __forceinline__ void halo_slice(HaloItems<V, RES>& I, const V* x, Head head, Tail tail) {
+    unsigned char it = *I.item;
+    const V piv = I.value(0);
+    const int row = I.column(0);
+    V s;
+    if constexpr (RES) {
+        s = head(row);
+        s = halo_chain_at<true>((it & 0x7f) - 1, I.v + 32, I.c + 32, x, s);
+        while (!(it & kHaloLast)) {
+            I.next();
+            it = *I.item;
+            s = halo_chain_at<true>(it & 0x7f, I.v, I.c, x, s);
+        }
+        tail(row, s, piv);
+        I.next();
+        return;
+    }
+    HaloEntries<V> E;
+    halo_load(I, 1, it & 0x7f, E);
+    I.next();
+    s = head(row);
+    s = halo_chain<true>((it & 0x7f) - 1, E, x, s);
+    while (!(it & kHaloLast)) {
+        it = *I.item;
+        halo_load(I, 0, it & 0x7f, E);
+        I.next();
+        s = halo_chain<true>(it & 0x7f, E, x, s);
+    }
+    tail(row, s, piv);
 }
 
-// s - sum_k f_k v[col_k] over the entries [k0, k1) (sweep_rest's chain of fused multiply-adds).
-template <class V>
-__device__ __forceinline__ V halo_rest(const HaloSm<V>& S, int k0, int k1, const V* v, V s) {
-    for (int k = k0; k < k1; ++k) s = fma_rn(-__ldg(&S.f[k]), v[__ldg(&S.lcol[k])], s);
-    return s;
-}
-
-// Forward sweep (part_fwd's arithmetic) over the own rows and the F rows, group by group, with
-// r -= alpha q unless first.  Own t that is read elsewhere goes to this sweep's half of gt, and
-// the other half, which every part has read before the last grid barrier, back to the marker.
-// Returns the own rows' r.r (want_rr) and t.t terms.
-template <bool IC, class V>
-__device__ double2 halo_fwd(const PartHalo& C, HaloSm<V>& S, bool first, V alpha, bool want_rr) {
-    V* gt = HaloVecs<V>::gt(C) + (size_t)S.par * S.n + S.p0;
-    V* gt_next = HaloVecs<V>::gt(C) + (size_t)(S.par ^ 1) * S.n + S.p0;
+// Forward sweep over the own rows and the F rows, group by group: r -= alpha q, t = L^{-1} r
+// (alpha = 0 with q = 0 leaves r as it is).  Own t that is read elsewhere is published.
+// Returns the own rows' r.r (want_rr) and (IC) t.t terms.
+template <bool IC, class V, bool RES>
+__device__ __forceinline__ double2 halo_fwd(const PartHalo& C, HaloSm<V, RES>& S, V alpha, bool want_rr) {
+    unsigned long long* gt = halo_row(C.gt, S, ++S.ts, S.p0);
+    const int w = threadIdx.x >> 5;
     double rr = 0.0, tt = 0.0;
+    S.items.begin();
+#pragma unroll 1
     for (int g = 0; g < C.ng; ++g) {
-        const int g0 = S.qs[g] - S.p0, no = S.qs[g + 1] - S.p0 - g0;
-        const int f0 = S.np + __ldg(&S.hs[4 * g]), nf = S.np + __ldg(&S.hs[4 * g + 2]) - f0;
-        if ((int)threadIdx.x < no + nf) {
-            const int l = (int)threadIdx.x < no ? g0 + threadIdx.x : f0 + threadIdx.x - no;
-            const int k0 = S.rp[l], d = k0 + S.dg[l];
-            prefetch_l1(&S.lcol[k0]);
-            prefetch_l1(&S.f[k0]);
-            prefetch_l1(&S.f[d]);
-        }
-        __syncthreads();  // the part's earlier groups are done
-        for (int i = threadIdx.x; i < no + nf; i += kPartThreads) {
-            const bool own = i < no;
-            const int l = own ? g0 + i : f0 + i - no;
-            const int k0 = S.rp[l], d = k0 + S.dg[l];
-            V ra = S.r[l];
-            if (!first) {
-                ra -= alpha * S.q[l];
-                S.r[l] = ra;
-            }
-            const V rest = halo_rest(S, k0, d, S.t, ra);
-            const V v = IC ? rest * __ldg(&S.f[d]) : rest;
-            S.t[l] = v;
-            if (own) {
-                if (S.pub[l] & 2) {
-                    __stcg(&gt[l], v);
-                    __stcg(&gt_next[l], Pending<V>::marker());
+        const int ns = S.gsl[g];
+        bool wait = g > 0;  // for the part's earlier groups, once
+#pragma unroll 1
+        for (int s = w; s < ns; s += kHaloWarps) {
+            V ra = V(0);
+            halo_slice(S.items, S.t, [&](int row) {
+                if (row != kHaloNone) {  // the update of r needs no earlier group: before the barrier
+                    const int l = row & kHaloMaxLocal;
+                    ra = fma_rn(-alpha, S.q[l], S.r[l]);
+                    S.r[l] = ra;
                 }
-                if (want_rr) rr += (double)ra * (double)ra;
-                if (IC) tt += (double)v * (double)v;
-            }
+                __syncwarp();
+                if (wait) __syncthreads();
+                wait = false;
+                return ra;
+            }, [&](int row, V rest, V piv) {
+                if (row == kHaloNone) return;
+                const int l = row & kHaloMaxLocal;
+                const V v = IC ? rest * piv : rest;
+                S.t[l] = v;
+                if (row & kHaloPubT) HaloPacket<V>::put(gt + (size_t)l * HaloPacket<V>::kWords, v, S.ts);
+                if (l < S.np) {
+                    if (want_rr) rr += (double)ra * (double)ra;
+                    if (IC) tt += (double)v * (double)v;
+                }
+            });
         }
+        if (wait) __syncthreads();
     }
     return make_double2(rr, tt);
 }
 
-// t of the Z rows that are not F rows, from their owners (bounded polls; a wait that runs out
-// records DEV_TIMEOUT and yields 0: the kernel returns at its next grid barrier).  The next
-// forward sweep uses the other half of gt.
-template <class V>
-__device__ __forceinline__ void halo_fetch_t(const PartHalo& C, HaloSm<V>& S, int* err, int* rec) {
-    const V* gt = HaloVecs<V>::gt(C) + (size_t)S.par * S.n;
-    auto fetch = [&](int l, int j) {
-        V v = *(volatile const V*)&gt[j];
-        if (Pending<V>::bits(v) == Pending<V>::kBits && !wait_value(gt, j, v, err, rec, j)) v = V(0);
-        S.t[l] = v;
-    };
-    if ((int)threadIdx.x < S.nz) fetch(S.z_l, S.z_g);
-    for (int i = threadIdx.x + kPartThreads, z0 = __ldg(&C.zoff[blockIdx.x]); i < S.nz; i += kPartThreads)
-        fetch(__ldg(&C.zl[z0 + i]), __ldg(&C.zg[z0 + i]));
-    S.par ^= 1;
+// t of the Z rows that are not F rows, from their owners.  work() runs between the first load
+// and its use.
+template <class V, bool RES, class Work>
+__device__ __forceinline__ void halo_fetch_t(const PartHalo& C, HaloSm<V, RES>& S, const GridBarrier& b, Work work) {
+    const unsigned long long* gt = halo_row(C.gt, S, S.ts, 0);
+    const bool mine = (int)threadIdx.x < S.nz;
+    const unsigned long long* p0 = gt + (size_t)S.z_g * HaloPacket<V>::kWords;
+    V v0 = V(0);
+    bool here = false;
+    if (mine) here = HaloPacket<V>::get(p0, v0, S.ts);
+    work();
+    if (mine) S.t[S.z_l] = halo_settle(p0, here, v0, S.ts, b, 2, S.z_g);
+    for (int i = threadIdx.x + kHaloThreads, z0 = __ldg(&C.zoff[blockIdx.x]); i < S.nz; i += kHaloThreads) {
+        const int j = __ldg(&C.zg[z0 + i]);
+        const unsigned long long* p = gt + (size_t)j * HaloPacket<V>::kWords;
+        V v;
+        const bool h = HaloPacket<V>::get(p, v, S.ts);
+        S.t[__ldg(&C.zl[z0 + i])] = halo_settle(p, h, v, S.ts, b, 2, j);
+    }
 }
 
-// Backward sweep (part_bwd's arithmetic) over the own rows and the Z rows: z = U^{-1} t in t's
-// array.  Returns the own rows' r.z terms (want_rz).
-template <class V>
-__device__ double halo_bwd(const PartHalo& C, const HaloSm<V>& S, bool want_rz) {
+// Backward sweep over the own rows and the Z rows: z = U^{-1} t in t's array.  Returns the own
+// rows' r.z terms (want_rz).
+template <class V, bool RES>
+__device__ __forceinline__ double halo_bwd(const PartHalo& C, HaloSm<V, RES>& S, bool want_rz) {
+    const int w = threadIdx.x >> 5;
     double rz = 0.0;
+#pragma unroll 1
     for (int g = C.ng - 1; g >= 0; --g) {
-        const int g0 = S.qs[g] - S.p0, no = S.qs[g + 1] - S.p0 - g0;
-        const int z0 = S.np + __ldg(&S.hs[4 * g + 1]), nz = S.np + __ldg(&S.hs[4 * g + 3]) - z0;
-        if ((int)threadIdx.x < no + nz) {
-            const int l = (int)threadIdx.x < no ? g0 + threadIdx.x : z0 + threadIdx.x - no;
-            const int d = S.rp[l] + S.dg[l];
-            prefetch_l1(&S.lcol[d]);
-            prefetch_l1(&S.f[d]);
-            prefetch_l1(&S.f[S.rp[l + 1] - 1]);
+        const int ns = S.gsl[C.ng + g];
+        bool wait = true;  // for the part's later groups and the fetched t, once
+#pragma unroll 1
+        for (int s = w; s < ns; s += kHaloWarps) {
+            halo_slice(S.items, S.z, [&](int row) {
+                __syncwarp();
+                if (wait) __syncthreads();
+                wait = false;
+                return row != kHaloNone ? S.t[row] : V(0);
+            }, [&](int row, V rest, V piv) {
+                if (row == kHaloNone) return;
+                const V v = rest * piv;
+                S.z[row] = v;
+                if (want_rz && row < S.np) rz += (double)S.r[row] * (double)v;
+            });
         }
-        __syncthreads();  // the part's later groups are done
-        for (int i = threadIdx.x; i < no + nz; i += kPartThreads) {
-            const bool own = i < no;
-            const int l = own ? g0 + i : z0 + i - no;
-            const int d = S.rp[l] + S.dg[l];
-            const V v = halo_rest(S, d + 1, S.rp[l + 1], S.z, S.t[l]) * __ldg(&S.f[d]);
-            S.z[l] = v;
-            if (want_rz && own) rz += (double)S.r[l] * (double)v;
-        }
+        if (wait) __syncthreads();
     }
     return rz;
 }
 
-// p = z + beta p (first: p = z) on the own rows and ring 1.  No barrier inside; the SpMV that
-// follows needs one.
-template <class V>
-__device__ __forceinline__ void halo_p_update(const PartHalo& C, const HaloSm<V>& S, V beta, bool first) {
+// p = z + beta p on the own rows and ring 1.  No barrier inside; the SpMV that follows needs one.
+template <class V, bool RES>
+__device__ __forceinline__ void halo_p_update(const PartHalo& C, const HaloSm<V, RES>& S, V beta) {
     const int k = blockIdx.x;
     const int a0 = __ldg(&C.r1off[k]), nr = __ldg(&C.r1off[k + 1]) - a0;
-    for (int i = threadIdx.x; i < S.np + nr; i += kPartThreads) {
+    for (int i = threadIdx.x; i < S.np + nr; i += kHaloThreads) {
         const int l = i < S.np ? i : (int)__ldg(&C.r1[a0 + i - S.np]);
-        S.p[l] = first ? S.z[l] : fma_rn(beta, S.p[l], S.z[l]);
+        S.p[l] = fma_rn(beta, S.p[l], S.z[l]);
     }
 }
 
-// b - A x in FP64 for the part's row l (x from the global iterate in Q order).
-template <class V>
-__device__ __forceinline__ double halo_residual(const KArgs& a, const PartHalo& C, const HaloSm<V>& S, int l, double& bi) {
-    bi = a.b[__ldg(&C.qa[S.p0 + l])];
-    const double* val = C.val + C.ebase[blockIdx.x];
-    double v = 0.0;
-    for (int k = S.rp[l]; k < S.rp[l + 1]; ++k)
-        v += __ldg(&val[k]) * __ldcg(&C.x[halo_global(S, (int)__ldg(&S.lcol[k]))]);
-    return bi - v;
+// r = b - A x in FP64 over the part's rows (x from the global iterate in Q order), published for
+// the parts that hold it as halo: store(l, r).  Returns the b.b and r.r terms.
+template <class V, bool RES, class Store>
+__device__ __forceinline__ double2 halo_residual(const KArgs& a, const PartHalo& C, const HaloSm<V, RES>& S, Store store) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wk = blockIdx.x * kHaloWarps + w;
+    const int i0 = C.wit[2 * wk], i1 = C.wit[2 * wk + 1];
+    int row = C.went[wk], i = i1 - i0;
+    const unsigned char* item = S.items.i0;
+    for (int j = 0; j < i; ++j) row += item[j] & 0x7f;
+    double bb = 0.0, rr = 0.0;
+    for (int s = w; s < S.nsl; s += kHaloWarps) {
+        const int l = s * 32 + lane;
+        double v = 0.0;
+        unsigned char it;
+        do {
+            it = item[i++];
+            for (int k = 0; k < (it & 0x7f); ++k, ++row) {
+                const size_t e = (size_t)row * 32 + lane;
+                if (l < S.np) v = __fma_rn(__ldg(&C.val[e]), __ldcg(&C.x[halo_global(S, (int)__ldg(&C.col[e]))]), v);
+            }
+        } while (!(it & kHaloLast));
+        if (l < S.np) {
+            const double bi = a.b[__ldg(&C.qa[S.p0 + l])];
+            const double ri = bi - v;
+            store(l, ri);
+            bb += bi * bi;
+            rr += ri * ri;
+        }
+    }
+    return make_double2(bb, rr);
 }
 
-// FP64 CG: MODE 0 Jacobi or no preconditioner, 1 IC(0), 2 ILU(0) (pcg_part's iterations).
-template <int MODE>
-__device__ void pcg_halo(const KArgs& a, const PartHalo& C, double* sh, unsigned char* smem) {
-    HaloSm<double> S = halo_sm<double>(C, a.A.n, smem, MODE != 0, false);
+struct HaloNoSide {
+    __device__ void operator()() const {}
+};
+struct HaloNoPost {
+    __device__ void operator()(int, double, double*) const {}
+};
+
+// FP64 CG: MODE 0 Jacobi or no preconditioner, 1 IC(0), 2 ILU(0) (pcg_part's iterations).  The
+// loop starts at the preconditioner with alpha = beta = 0 and p = q = 0, which leaves r and x
+// as they are and makes p = z.
+template <int MODE, bool RES>
+__device__ __forceinline__ void pcg_halo(const KArgs& a, const PartHalo& C, HaloSm<double, RES>& S, double* sh) {
     const int tid = threadIdx.x, np = S.np;
-    int* err = a.bar.err;
-    int* rec = a.bar.rec;
+    constexpr int T = kHaloThreads;
     const bool rel = a.criterion == PF2_CRITERION_REL;
     const bool jac = a.precond == PF2_PRECOND_JACOBI;
-    for (int l = tid; l < np; l += kPartThreads) __stcg(&C.x[S.p0 + l], a.x[__ldg(&C.qa[S.p0 + l])]);
-    if (!grid_sync(a.bar, gridDim.x)) return;
-    double red[3] = { 0.0, 0.0, 0.0 };  // r.z, b.b, r.r
-    for (int l = tid; l < np; l += kPartThreads) {
-        double bi;
-        S.r[l] = halo_residual(a, C, S, l, bi);
-        red[1] += bi * bi;
+    for (int l = tid; l < np; l += T) __stcg(&C.x[S.p0 + l], a.x[__ldg(&C.qa[S.p0 + l])]);
+    for (int l = tid; l < np + S.nh; l += T) {
+        S.p[l] = 0.0;
+        S.q[l] = 0.0;
+        // (tri: finite values where a padding entry of the first sweep looks)
+        S.t[l] = MODE == 0 ? 1.0 / __ldg(&C.diag[S.p0 + C.hoff[blockIdx.x] + l]) : 0.0;
     }
-    if (MODE == 0)
-        for (int l = tid; l < np + S.nh; l += kPartThreads) S.t[l] = 1.0 / __ldg(&S.val[S.rp[l] + S.dg[l]]);
-    __syncthreads();
-    halo_publish_r(C, S);
-    if (!grid_sync(a.bar, gridDim.x)) return;
-    halo_fetch(C, S, S.r);
-    __syncthreads();
-    if (MODE == 0) {
-        for (int l = tid; l < np + S.nh; l += kPartThreads) {
-            const double ri = S.r[l];
-            const double zi = jac ? ri * S.t[l] : ri;
-            S.z[l] = zi;
-            S.p[l] = zi;
-            if (l < np) {
-                red[0] += ri * zi;
-                red[2] += ri * ri;
-            }
-        }
-    } else {
-        red[2] = halo_fwd<MODE == 1, double>(C, S, true, 0.0, true).x;
-        halo_fetch_t(C, S, err, rec);
-        red[0] = halo_bwd(C, S, true);
-        __syncthreads();
-        halo_p_update(C, S, 0.0, true);
-    }
-    double r2[2] = { red[0], red[1] }, r1[1] = { red[2] };
-    if (!part_reduce<2>(a.bar, r2, sh, S.red)) return;
-    // bnorm and the first test (thread 0; see part_reduce)
-    if (!part_reduce<1>(a.bar, r1, sh, S.red, [&](const double* tot, double* out) {
-            out[0] = sqrt(r2[1]);
-            out[1] = rel ? (sqrt(tot[0]) <= a.tol * out[0]) : (r2[0] < a.tol * a.tol);
-        }))
-        return;
-    double gamma = r2[0];
-    const double bnorm = sh[24];
-    double rr = r1[0];
+    if (!halo_sync(a.bar, S)) return;
+    unsigned long long* gr = halo_row(C.gq, S, ++S.qs, S.p0);
+    const double2 br = halo_residual(a, C, S, [&](int l, double ri) {
+        S.r[l] = ri;
+        if (S.pub[l]) HaloPacket<double>::put(gr + 2 * (size_t)l, ri, S.qs);
+    });
+    // b.b and r.r beside the fetch of the F rows' r
+    if (!halo_reduce(a.bar, S, br.x, br.y, sh, HaloNoPost(), [&]() { halo_fetch(C, S, a.bar, S.r); })) return;
+    const double bb_all = sh[16];
+    double rr = sh[17], gamma = 1.0, alpha = 0.0;
+    // the tests compare r.r or r.z with the square of the tolerance
+    const double bound = rel ? (a.tol * a.tol) * bb_all : a.tol * a.tol;
+    const double rr0 = rr;
     int it = 0;
-    bool conv = sh[25] != 0.0;
-    while (!conv && it < a.maxit) {
-        ++it;
-        double pq[1] = { halo_spmv(C, S) };
-        if (!part_reduce<1>(a.bar, pq, sh, S.red, [&](const double* tot, double* out) { out[0] = gamma / tot[0]; }))
-            return;
-        const double alpha = sh[24];
-        halo_fetch(C, S, S.q);
-        __syncthreads();
-        // with the absolute criterion (a test of r.z alone) r.r is reduced once after the loop
-        double g2[2] = { 0.0, 0.0 };  // r.z (IC: t.t), r.r
-        auto test = [&](const double* tot, double* out) {
-            out[0] = rel ? sqrt(tot[1]) <= a.tol * bnorm : tot[0] < a.tol * a.tol;
-            out[1] = tot[0] / gamma;
+    bool conv = false, first = true;
+    auto post = [&](int j, double tot, double* out) {
+        if (j == 0) out[1] = first ? 0.0 : tot / gamma;
+        if (rel ? j == 1 : j == 0) out[0] = rel ? tot <= bound : tot < bound;
+    };
+    while (true) {
+        // the update of x with the last alpha, beside the exchange or a reduction's wait
+        auto x_update = [&]() {
+            for (int l = tid; l < np; l += T)
+                __stcg(&C.x[S.p0 + l], __fma_rn(alpha, S.p[l], __ldcg(&C.x[S.p0 + l])));
         };
-        bool ok;
-        if (MODE == 1) {
-            // z = L^{-T} t does not depend on beta: the x update and the backward sweep run between
-            // the arrival at the t.t (and r.r) reduction and the wait for the others
-            const double2 f = halo_fwd<true, double>(C, S, false, alpha, rel);
-            auto window = [&]() {
-                for (int l = tid; l < np; l += kPartThreads)
-                    __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + alpha * S.p[l]);
-                halo_fetch_t(C, S, err, rec);
-                halo_bwd(C, S, false);
-            };
-            if (rel) {
-                double g[2] = { f.y, f.x };
-                const unsigned tk = grid_reduce_tree_arrive<kPartThreads, 2>(a.bar, g, sh, S.red);
-                window();
-                ok = grid_reduce_tree_wait<kPartThreads, 2>(a.bar, tk, g, sh, test);
-                g2[0] = g[0];
-                g2[1] = g[1];
-            } else {
-                double g[1] = { f.y };
-                const unsigned tk = grid_reduce_tree_arrive<kPartThreads, 1>(a.bar, g, sh, S.red);
-                window();
-                ok = grid_reduce_tree_wait<kPartThreads, 1>(a.bar, tk, g, sh, test);
-                g2[0] = g[0];
-            }
-        } else {
-            if (MODE == 0) {
-                for (int l = tid; l < np + S.nh; l += kPartThreads) {
-                    const double ri = S.r[l] - alpha * S.q[l];
-                    const double zi = jac ? ri * S.t[l] : ri;
-                    S.r[l] = ri;
-                    S.z[l] = zi;
-                    if (l < np) {
-                        __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + alpha * S.p[l]);
-                        g2[0] += ri * zi;
-                        if (rel) g2[1] += ri * ri;
-                    }
+        double rz = 0.0, r2 = 0.0;
+        if (MODE == 0) {
+            for (int l = tid; l < np + S.nh; l += T) {
+                const double ri = __fma_rn(-alpha, S.q[l], S.r[l]);
+                const double zi = jac ? ri * S.t[l] : ri;
+                S.r[l] = ri;
+                S.z[l] = zi;
+                if (l < np) {
+                    rz += ri * zi;
+                    if (rel) r2 += ri * ri;
                 }
-            } else {
-                g2[1] = halo_fwd<false, double>(C, S, false, alpha, rel).x;
-                for (int l = tid; l < np; l += kPartThreads)
-                    __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + alpha * S.p[l]);
-                halo_fetch_t(C, S, err, rec);
-                g2[0] = halo_bwd(C, S, true);
             }
-            // the test and beta = r.z / (previous r.z) (thread 0; see part_reduce)
-            if (rel) {
-                ok = part_reduce<2>(a.bar, g2, sh, S.red, test);
-            } else {
-                double g1[1] = { g2[0] };
-                ok = part_reduce<1>(a.bar, g1, sh, S.red, test);
-                g2[0] = g1[0];
-            }
+            halo_arrive(a.bar, S, rz, r2);
+            x_update();
+        } else {
+            const double2 f = halo_fwd<MODE == 1>(C, S, alpha, rel);
+            // IC(0): z = L^{-T} t does not depend on beta, so the x update and the backward sweep run
+            // between the arrival at the t.t (and r.r) reduction and the wait for the others
+            if (MODE == 1) halo_arrive(a.bar, S, f.y, f.x);
+            halo_fetch_t(C, S, a.bar, x_update);
+            rz = halo_bwd(C, S, MODE == 2);
+            if (MODE == 2) halo_arrive(a.bar, S, rz, f.x);
         }
-        if (!ok) return;
-        if (rel) rr = g2[1];
-        gamma = g2[0];
+        if (!halo_wait(a.bar, S, sh, MODE != 1, post, HaloNoSide())) return;
+        gamma = sh[16];
+        if (rel) rr = sh[17];
+        first = false;
         if (sh[24] != 0.0) { conv = true; break; }
-        halo_p_update(C, S, sh[25], false);
+        if (it >= a.maxit) break;
+        ++it;
+        halo_p_update(C, S, sh[25]);
         __syncthreads();
+        if (MODE == 0) S.items.begin();
+        const double pq = halo_spmv(C, S);
+        // alpha beside the fetch of the F rows' q
+        if (!halo_reduce(a.bar, S, pq, 0.0, sh,
+                         [&](int j, double tot, double* out) { if (j == 0) out[0] = gamma / tot; },
+                         [&]() { halo_fetch(C, S, a.bar, S.q); }))
+            return;
+        alpha = sh[24];
     }
-    if (!rel && it > 0) {
-        double f[1] = { 0.0 };
-        for (int l = tid; l < np; l += kPartThreads) f[0] += S.r[l] * S.r[l];
-        if (!part_reduce<1>(a.bar, f, sh, S.red)) return;
-        rr = f[0];
+    if (!rel && it > 0) {  // with the absolute criterion (a test of r.z alone) r.r is reduced once, here
+        double f = 0.0;
+        for (int l = tid; l < np; l += T) f += S.r[l] * S.r[l];
+        if (!halo_reduce(a.bar, S, f, 0.0, sh, HaloNoPost(), HaloNoSide())) return;
+        rr = sh[16];
     }
-    for (int l = tid; l < np; l += kPartThreads) a.x[__ldg(&C.qa[S.p0 + l])] = __ldcg(&C.x[S.p0 + l]);
+    if (it == 0) rr = rr0;
+    for (int l = tid; l < np; l += T) a.x[__ldg(&C.qa[S.p0 + l])] = __ldcg(&C.x[S.p0 + l]);
     if (blockIdx.x == 0 && tid == 0) {
+        const double bnorm = sqrt(bb_all);
         a.out->iterations = it;
         a.out->converged = conv ? 1 : 0;
         a.out->residual = rel ? sqrt(rr) / (bnorm > 0 ? bnorm : 1.0) : sqrt(gamma);
@@ -461,131 +846,95 @@ __device__ void pcg_halo(const KArgs& a, const PartHalo& C, double* sh, unsigned
 }
 
 // Mixed-precision CG (pcg_part_mixed's algorithm: FP32 iteration, FP64 sums, reliable updates).
-template <bool IC>
-__device__ void pcg_halo_mixed(const KArgs& a, const PartHalo& C, double* sh, unsigned char* smem) {
-    HaloSm<float> S = halo_sm<float>(C, a.A.n, smem, true, true);
+// Passes of the loop: the first (preconditioner of r, gamma = r.z), ordinary ones, and after a
+// refinement one more preconditioner with the true residual, which gives the next beta.
+template <bool IC, bool RES>
+__device__ __forceinline__ void pcg_halo_mixed(const KArgs& a, const PartHalo& C, HaloSm<float, RES>& S, double* sh) {
     const int tid = threadIdx.x, np = S.np;
-    int* err = a.bar.err;
-    int* rec = a.bar.rec;
-    for (int l = tid; l < np; l += kPartThreads) {
+    constexpr int T = kHaloThreads;
+    for (int l = tid; l < np; l += T) {
         __stcg(&C.x[S.p0 + l], a.x[__ldg(&C.qa[S.p0 + l])]);
         S.d[l] = 0.0f;
     }
-    if (!grid_sync(a.bar, gridDim.x)) return;
-    // r = b - A x in FP64, published for the parts that hold it as halo
-    auto residual = [&](double& rr_, double* bb_) {
-        for (int l = tid; l < np; l += kPartThreads) {
-            double bi;
-            const double ri = halo_residual(a, C, S, l, bi);
-            S.r[l] = (float)ri;
-            if (S.pub[l] & 1) __stcg(&C.gq32[S.p0 + l], (float)ri);
-            rr_ += ri * ri;
-            if (bb_) *bb_ += bi * bi;
-        }
-    };
-    double red[2] = { 0.0, 0.0 };  // b.b, r.r
-    residual(red[1], &red[0]);
-    // square roots by thread 0 (see part_reduce)
-    if (!part_reduce<2>(a.bar, red, sh, S.red, [&](const double* tot, double* out) {
-            out[0] = sqrt(tot[0]);
-            out[1] = sqrt(tot[1]);
-        }))
-        return;
-    const double bnorm = sh[24];
-    const double target = a.tol * bnorm;
-    double rnorm = sh[25];
-    double rlast = rnorm;
-    int it = 0, refinements = 1;
-    bool conv = rnorm <= target;
-    if (!conv) {
-        // z = M^{-1} r, p = z, gamma = r.z
-        halo_fetch(C, S, S.r);
-        __syncthreads();
-        halo_fwd<IC, float>(C, S, true, 0.0f, false);
-        halo_fetch_t(C, S, err, rec);
-        double g[1] = { halo_bwd(C, S, true) };
-        __syncthreads();
-        halo_p_update(C, S, 0.0f, true);
-        if (!part_reduce<1>(a.bar, g, sh, S.red)) return;
-        double gamma = g[0];
-        while (it < a.maxit) {
-            double pq[1] = { halo_spmv(C, S) };
-            ++it;
-            if (!part_reduce<1>(a.bar, pq, sh, S.red, [&](const double* tot, double* out) {
-                    out[0] = (double)(float)(gamma / tot[0]);
-                }))
-                return;
-            const float alpha = (float)sh[24];
-            halo_fetch(C, S, S.q);
-            __syncthreads();
-            double g2[2];  // r.z (IC: t.t), r.r
-            // refinement test and beta (thread 0; see part_reduce)
-            auto post = [&](const double* tot, double* out) {
-                const double rit = sqrt(tot[1]);
-                out[0] = rit <= a.inner_eta * rlast || rit <= target;
-                out[1] = (double)(float)(tot[0] / gamma);
-            };
-            const double2 f = halo_fwd<IC, float>(C, S, false, alpha, true);
-            auto d_update = [&]() {
-                for (int l = tid; l < np; l += kPartThreads) S.d[l] = S.d[l] + alpha * S.p[l];
-            };
-            g2[1] = f.x;
-            if (IC) {
-                // the backward sweep (z alone) overlaps the reduction, as in pcg_halo
-                g2[0] = f.y;
-                const unsigned tk = grid_reduce_tree_arrive<kPartThreads, 2>(a.bar, g2, sh, S.red);
-                d_update();
-                halo_fetch_t(C, S, err, rec);
-                halo_bwd(C, S, false);
-                if (!grid_reduce_tree_wait<kPartThreads, 2>(a.bar, tk, g2, sh, post)) return;
-            } else {
-                d_update();
-                halo_fetch_t(C, S, err, rec);
-                g2[0] = halo_bwd(C, S, true);
-                if (!part_reduce<2>(a.bar, g2, sh, S.red, post)) return;
-            }
-            double gnew = g2[0];
-            float beta = (float)sh[25];
-            if (sh[24] != 0.0) {
-                // refinement: x += d, r = b - A x and the test in FP64
-                for (int l = tid; l < np; l += kPartThreads) {
-                    __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + (double)S.d[l]);
-                    S.d[l] = 0.0f;
-                }
-                if (!grid_sync(a.bar, gridDim.x)) return;
-                double rr[1] = { 0.0 };
-                residual(rr[0], nullptr);
-                if (!part_reduce<1>(a.bar, rr, sh, S.red, [&](const double* tot, double* out) {
-                        out[0] = sqrt(tot[0]);
-                    }))
-                    return;
-                ++refinements;
-                rnorm = sh[24];
-                if (rnorm <= target) { conv = true; break; }
-                rlast = rnorm;
-                // continue from the true residual, keeping the search direction
-                halo_fetch(C, S, S.r);
-                __syncthreads();
-                const double2 f3 = halo_fwd<IC, float>(C, S, true, 0.0f, false);
-                halo_fetch_t(C, S, err, rec);
-                const double rz = halo_bwd(C, S, !IC);
-                double g3[1] = { IC ? f3.y : rz };
-                if (!part_reduce<1>(a.bar, g3, sh, S.red, [&](const double* tot, double* out) {
-                        out[0] = (double)(float)(tot[0] / gamma);
-                    }))
-                    return;
-                gnew = g3[0];
-                beta = (float)sh[24];
-            }
-            gamma = gnew;
-            halo_p_update(C, S, beta, false);
-            __syncthreads();
-        }
-        if (!conv)  // iteration limit: keep the accumulated update
-            for (int l = tid; l < np; l += kPartThreads)
-                __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + (double)S.d[l]);
+    for (int l = tid; l < np + S.nh; l += T) {
+        S.p[l] = 0.0f;
+        S.q[l] = 0.0f;
+        S.t[l] = 0.0f;  // finite where a padding entry of the first sweep looks
     }
-    for (int l = tid; l < np; l += kPartThreads) a.x[__ldg(&C.qa[S.p0 + l])] = __ldcg(&C.x[S.p0 + l]);
+    if (!halo_sync(a.bar, S)) return;
+    enum { FIRST, ORDINARY, REFINED };
+    int pass = FIRST, it = 0, refinements = 0;
+    double bnorm = 0.0, target = 0.0, rnorm = 0.0, rlast = 0.0, gamma = 0.0;
+    float alpha = 0.0f;
+    bool conv = false;
+    while (true) {
+        if (pass != ORDINARY) {
+            // r = b - A x and the test in FP64
+            unsigned long long* gr = halo_row(C.gq, S, ++S.qs, S.p0);
+            const double2 br = halo_residual(a, C, S, [&](int l, double ri) {
+                S.r[l] = (float)ri;
+                if (S.pub[l]) HaloPacket<float>::put(gr + l, (float)ri, S.qs);
+            });
+            if (!halo_reduce(a.bar, S, br.x, br.y, sh, [&](int j, double tot, double* out) { out[j] = sqrt(tot); },
+                             [&]() { halo_fetch(C, S, a.bar, S.r); }))
+                return;
+            ++refinements;
+            bnorm = sh[24];
+            rnorm = sh[25];
+            target = a.tol * bnorm;
+            rlast = rnorm;
+            if (rnorm <= target) { conv = true; break; }
+            alpha = 0.0f;  // the sweep takes r as it is
+            if (pass == FIRST && it >= a.maxit) break;
+        }
+        // refinement test (squares: rit <= max(eta rlast, target)) and beta (0 in the first pass)
+        const double lim = fmax(a.inner_eta * rlast, target), lim2 = lim * lim;
+        auto post = [&](int j, double tot, double* out) {
+            if (j == 0) out[1] = pass == FIRST ? 0.0 : (double)(float)(tot / gamma);
+            else out[0] = tot <= lim2;
+        };
+        auto d_update = [&]() {
+            if (pass == ORDINARY)
+                for (int l = tid; l < np; l += T) S.d[l] = S.d[l] + alpha * S.p[l];
+        };
+        const double2 f = halo_fwd<IC>(C, S, alpha, pass == ORDINARY);
+        // IC(0): the backward sweep (z alone) overlaps the reduction, as in pcg_halo; the first pass
+        // takes gamma = r.z from the backward sweep
+        const bool tt = IC && pass != FIRST;
+        if (tt) halo_arrive(a.bar, S, f.y, f.x);
+        halo_fetch_t(C, S, a.bar, d_update);
+        const double rz = halo_bwd(C, S, !tt);
+        if (!tt) halo_arrive(a.bar, S, rz, f.x);
+        if (!halo_wait(a.bar, S, sh, !tt, post, HaloNoSide())) return;
+        if (pass == ORDINARY && sh[24] != 0.0) {
+            // refinement: x += d; the next pass recomputes r and runs the sweeps on it (the search
+            // direction is kept)
+            for (int l = tid; l < np; l += T) {
+                __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + (double)S.d[l]);
+                S.d[l] = 0.0f;
+            }
+            if (!halo_sync(a.bar, S)) return;
+            pass = REFINED;
+            continue;
+        }
+        gamma = sh[16];
+        const float beta = (float)sh[25];
+        if (pass != FIRST && it >= a.maxit) break;
+        pass = ORDINARY;
+        ++it;
+        halo_p_update(C, S, beta);
+        __syncthreads();
+        const double pq = halo_spmv(C, S);
+        if (!halo_reduce(a.bar, S, pq, 0.0, sh,
+                         [&](int j, double tot, double* out) { if (j == 0) out[0] = (double)(float)(gamma / tot); },
+                         [&]() { halo_fetch(C, S, a.bar, S.q); }))
+            return;
+        alpha = (float)sh[24];
+    }
+    if (!conv)  // iteration limit: keep the accumulated update
+        for (int l = tid; l < np; l += T)
+            __stcg(&C.x[S.p0 + l], __ldcg(&C.x[S.p0 + l]) + (double)S.d[l]);
+    for (int l = tid; l < np; l += T) a.x[__ldg(&C.qa[S.p0 + l])] = __ldcg(&C.x[S.p0 + l]);
     if (blockIdx.x == 0 && tid == 0) {
         a.out->iterations = it;
         a.out->converged = conv ? 1 : 0;
@@ -596,18 +945,20 @@ __device__ void pcg_halo_mixed(const KArgs& a, const PartHalo& C, double* sh, un
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kPartThreads, 1) k_pcg_halo(KArgs a, PartHalo C) {
+template <int MODE, bool RES>
+__global__ void __launch_bounds__(kHaloThreads, 1) k_pcg_halo(KArgs a, PartHalo C) {
     __shared__ double sh[kShDoubles];
-    extern __shared__ __align__(16) unsigned char part_smem[];
-    pcg_halo<MODE>(a, C, sh, part_smem);
+    extern __shared__ __align__(128) unsigned char halo_smem[];
+    HaloSm<double, RES> S = halo_sm<double, RES>(C, a.A.n, halo_smem, MODE != 0, false, a.bar.err);
+    pcg_halo<MODE>(a, C, S, sh);
 }
 
-template <bool IC>
-__global__ void __launch_bounds__(kPartThreads, 1) k_pcg_halo_mixed(KArgs a, PartHalo C) {
+template <bool IC, bool RES>
+__global__ void __launch_bounds__(kHaloThreads, 1) k_pcg_halo_mixed(KArgs a, PartHalo C) {
     __shared__ double sh[kShDoubles];
-    extern __shared__ __align__(16) unsigned char part_smem[];
-    pcg_halo_mixed<IC>(a, C, sh, part_smem);
+    extern __shared__ __align__(128) unsigned char halo_smem[];
+    HaloSm<float, RES> S = halo_sm<float, RES>(C, a.A.n, halo_smem, true, true, a.bar.err);
+    pcg_halo_mixed<IC>(a, C, S, sh);
 }
 
 }  // namespace pf2

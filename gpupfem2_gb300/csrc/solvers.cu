@@ -2847,11 +2847,14 @@ struct pf2_solver {
     DevBuf<float> q_val32, q_f32, q_gp32, q_gt32, q_gz32;  // mixed precision
     // the parts with halo rows (k_pcg_halo; shares q_s, q_a, q_x, the entry maps and values)
     bool halo = false;
-    int halo_RL = 0;
-    long long halo_entries = 0;
-    DevBuf<int> h_hs, h_hoff, h_hq, h_foff, h_fg, h_zoff, h_zg, h_r1off, h_ebase, h_rp;
-    DevBuf<unsigned short> h_fl, h_zl, h_r1, h_lcol;
-    DevBuf<unsigned char> h_dg, h_pub;
+    int halo_RL = 0, halo_TL = 0, halo_E = 0;
+    bool halo_res = false;
+    long long halo_ne = 0, halo_nd = 0;  // stream entries, diagonals
+    DevBuf<int> h_hoff, h_hq, h_foff, h_fg, h_zoff, h_zg, h_r1off, h_ioff, h_wit, h_went, h_gsl, h_dmap;
+    DevBuf<unsigned short> h_fl, h_zl, h_r1, h_col;
+    DevBuf<unsigned char> h_pub, h_item;
+    DevBuf<unsigned long long> h_gq, h_gt;  // packets of the exchanges
+    DevBuf<double> h_diag;
     bool factored = false;
     const pf2_csr* last = nullptr;  // matrix of the last setup / solve
 };
@@ -3036,15 +3039,19 @@ static void graph_parts(int n, const std::vector<int>& rp, const std::vector<int
 // (at least kPartMinRows rows each), the part order Q, the CSR arrays in Q order and the
 // boundary flags.  Leaves S->part false where the plan does not apply: a group whose rows
 // depend on one another, or a part too large for the shared-memory vectors.
-constexpr int kPartMinRows = 512;
+// Rows per part at least: fewer rows share less FP64 work per SM but more halo and more blocks
+// in a reduction.  Measured, us per IC(0) iteration at 512 / 256 / 170 / 128 rows: 4,355 rows
+// 12.7 / 10.9 / 10.7 / 10.5, 16,705 rows 13.1 / 11.5 / 11.2 / 11.4.
+constexpr int kPartMinRows = 170;
+constexpr int kHaloFactor = 1 << 30;  // flag of a factor value in the streams' value map
 
 // The halo form of the plan (part_halo.cuh) on the parts and the order Q of build_part_plan
 // (bq: Q position of B's row, qb its inverse, qa the row of A).  Leaves S->halo false where
 // it does not apply: a part's rows with its halo exceed the shared memory or the 16-bit local
-// columns, or the halo is larger than the part (many groups: a 3D graph), where every part
+// columns, or the halo is over four times the part (many groups: a 3D graph), where every part
 // would compute most of its neighbours' sweeps.  Where it applies it measured faster at every
-// size (us per IC(0) iteration, waits in the sweeps against halo rows: 340 rows 23.1 / 19.4,
-// 16,705 rows 25.2 / 19.0, 125,364 rows 29.7 / 21.8, 499,288 rows 43.1 / 39.5).
+// size (us per IC(0) iteration, waits in the sweeps against halo rows: 340 rows 23.6 / 12.8,
+// 16,705 rows 25.4 / 11.2, 125,364 rows 29.8 / 14.1, 499,288 rows 43.5 / 36.5).
 static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, const std::vector<int>& bcol,
                                   const std::vector<int>& bmap, const std::vector<int>& bdiag,
                                   const std::vector<int>& perm, const std::vector<int>& part,
@@ -3057,35 +3064,31 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
         if (atoi(e) == 3) return PF2_OK;  // tests: the kernel with waits inside the sweeps
     if (const char* e = getenv("PF2_CG_PART_LOCAL"))
         if (mixed && tri && atoi(e) != 0) return PF2_OK;
-    // rows of B by part (Q order: consecutive), pid the part of a row of B
+    // pid: the part of a row of B; cls: the row's membership in the halo of part stamp
     std::vector<int> pid(n), local(n, -1), stamp(n, -1);
-    std::vector<unsigned char> cls(n, 0), pub(n, 0);
+    std::vector<unsigned char> cls(n, 0), pub(n, 0), pub_t(n, 0);
     for (int r = 0; r < n; ++r) pid[r] = part[perm[r]];
-    std::vector<int> hs((size_t)P * ng * 4), hoff(P + 1, 0), hq, foff(P + 1, 0), fg, zoff(P + 1, 0), zg, r1off(P + 1, 0),
-        ebase(P + 1, 0), rp, amap, fmap;
-    std::vector<unsigned short> fl, zl, r1, lcol;
-    std::vector<unsigned char> dg;
-    rp.reserve(n + n / 8 + P);
-    dg.reserve(n + n / 8);
-    lcol.reserve(S->nnz + S->nnz / 8);
-    amap.reserve(S->nnz + S->nnz / 8);
-    fmap.reserve(S->nnz + S->nnz / 8);
-    std::vector<std::vector<int>> bucket(ng);
-    std::vector<int> ring, halo;
-    int RL = 0;
     enum { F = 1, Z = 2 };
+    struct Halo {
+        std::vector<int> rows, ring;          // rows of B: by group as F only, F and Z, Z only; ring 1
+        std::vector<int> f0, f1, z0, z1;      // per group: F rows, Z rows (positions in rows)
+        std::vector<unsigned char> cls;
+    };
+    std::vector<Halo> H(P);
+    std::vector<std::vector<int>> bucket(ng);
+    int RL = 0;
     for (int k = 0; k < P; ++k) {
+        Halo& h = H[k];
         const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0;
         // ring 1, the F rows among it (read by an own row's lower entries) and the closures
-        ring.clear();
-        halo.clear();
         for (auto& b : bucket) b.clear();
+        int nh = 0;
         auto add = [&](int j, int bits) {
             if (stamp[j] != k) {
                 stamp[j] = k;
                 cls[j] = 0;
-                halo.push_back(j);
                 bucket[grp[j]].push_back(j);
+                ++nh;
             }
             cls[j] |= bits;
         };
@@ -3094,106 +3097,177 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
             for (int e = brp[i]; e < brp[i + 1]; ++e) {
                 const int j = bcol[e];
                 if (pid[j] == k) continue;
-                if (stamp[j] != k) ring.push_back(j);
+                if (stamp[j] != k) h.ring.push_back(j);
                 add(j, !tri ? F : (e < bdiag[i] ? F | Z : Z));
             }
         }
         if (tri) {
             for (int g = ng - 1; g >= 0; --g)  // rows added have lower groups
-                for (size_t h = 0; h < bucket[g].size(); ++h) {
-                    const int i = bucket[g][h];
+                for (size_t c = 0; c < bucket[g].size(); ++c) {
+                    const int i = bucket[g][c];
                     if (!(cls[i] & F)) continue;
                     for (int e = brp[i]; e < bdiag[i]; ++e)
                         if (pid[bcol[e]] != k) add(bcol[e], F);
                 }
             for (int g = 0; g < ng; ++g)  // rows added have higher groups
-                for (size_t h = 0; h < bucket[g].size(); ++h) {
-                    const int i = bucket[g][h];
+                for (size_t c = 0; c < bucket[g].size(); ++c) {
+                    const int i = bucket[g][c];
                     if (!(cls[i] & Z)) continue;
                     for (int e = bdiag[i] + 1; e < brp[i + 1]; ++e)
                         if (pid[bcol[e]] != k) add(bcol[e], Z);
                 }
         }
-        const int nh = (int)halo.size();
-        if (nh > std::max(np, 64) || np + nh > 65535) {
+        if (nh > std::max(4 * np, 64) || np + nh >= kHaloMaxLocal) {
             S->part_why = "the halo rows outnumber a part's rows";
             return PF2_OK;
         }
         RL = std::max(RL, np + nh);
-        // local numbering: own rows, then the halo by group as F only, F and Z, Z only
-        for (int q = p0; q < p0 + np; ++q) local[qb[q]] = q - p0;
-        int at = 0;
-        halo.clear();
+        h.f0.resize(ng);
+        h.f1.resize(ng);
+        h.z0.resize(ng);
+        h.z1.resize(ng);
         for (int g = 0; g < ng; ++g) {
             auto& b = bucket[g];
             std::sort(b.begin(), b.end());
-            int* o = &hs[((size_t)k * ng + g) * 4];
             auto put = [&](int want) {
                 for (int i : b)
-                    if (cls[i] == want) {
-                        halo.push_back(i);
-                        local[i] = np + at++;
-                    }
+                    if (cls[i] == want) h.rows.push_back(i);
             };
-            o[0] = at;
+            h.f0[g] = (int)h.rows.size();
             put(F);
-            o[1] = at;
+            h.z0[g] = (int)h.rows.size();
             put(F | Z);
-            o[2] = at;
+            h.f1[g] = (int)h.rows.size();
             put(Z);
-            o[3] = at;
+            h.z1[g] = (int)h.rows.size();
         }
-        for (int i : halo) {
+        h.cls.resize(nh);
+        for (int c = 0; c < nh; ++c) {
+            h.cls[c] = cls[h.rows[c]];
+            (h.cls[c] & F ? pub : pub_t)[bq[h.rows[c]]] = 1;
+        }
+    }
+    std::vector<int> hoff(P + 1, 0), hq, foff(P + 1, 0), fg, zoff(P + 1, 0), zg, r1off(P + 1, 0), ioff(P + 1, 0), wit, went,
+        gsl, map, dmap;
+    std::vector<unsigned char> item;
+    std::vector<unsigned short> fl, zl, r1, col;
+    int TL = 0;
+    const size_t guess = (size_t)S->nnz * (tri ? 9 : 5) / 4;
+    col.reserve(guess);
+    map.reserve(guess);
+    const std::vector<int> none;
+    for (int k = 0; k < P; ++k) {
+        const Halo& h = H[k];
+        const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0, nh = (int)h.rows.size();
+        for (int q = p0; q < p0 + np; ++q) local[qb[q]] = q - p0;
+        for (int c = 0; c < nh; ++c) {
+            const int i = h.rows[c];
+            local[i] = np + c;
             hq.push_back(bq[i]);
-            if (cls[i] & F) {
+            if (h.cls[c] & F) {
                 fl.push_back((unsigned short)local[i]);
                 fg.push_back(bq[i]);
-                pub[bq[i]] |= 1;
             } else {
                 zl.push_back((unsigned short)local[i]);
                 zg.push_back(bq[i]);
-                pub[bq[i]] |= 2;
             }
         }
-        for (int i : ring) r1.push_back((unsigned short)local[i]);
-        // entries: the own rows whole; a halo row's lower part (F), diagonal and upper part (Z)
-        const int e0 = (int)lcol.size();
-        ebase[k] = e0;
-        auto row = [&](int i, int b0, int b1, bool own) {
-            rp.push_back((int)lcol.size() - e0);
-            dg.push_back((unsigned char)(bdiag[i] - b0));
-            for (int e = b0; e < b1; ++e) {
-                lcol.push_back((unsigned short)local[bcol[e]]);
-                amap.push_back(own || (!tri && e == bdiag[i]) ? bmap[e] : -1);
-                fmap.push_back(e);
+        for (int i : h.ring) r1.push_back((unsigned short)local[i]);
+        if (!tri) {
+            for (int q = p0; q < p0 + np; ++q) dmap.push_back(bmap[bdiag[qb[q]]]);
+            for (int i : h.rows) dmap.push_back(bmap[bdiag[i]]);
+        }
+        // the slice of rows row(s .. min(s + 32, m) - 1), entries [lo(i), hi(i)) of row i, cut into
+        // items; a padding entry has the value 0 and a column that is safe to read: the row's
+        // first entry, or the row itself.  set 0: SpMV (values of A), 1: forward, 2: backward
+        // (factor values, flagged in the map; the first entry row holds the pivots)
+        auto emit = [&](int m, int s, auto row, auto lo, auto hi, int set) {
+            const int wd = std::min(32, m - s);
+            int len = 0;
+            for (int j = 0; j < wd; ++j) len = std::max(len, hi(row(s + j)) - lo(row(s + j)));
+            const int lead = set ? 1 : 0, rows = len + lead;
+            const size_t at = col.size();
+            col.resize(at + 32 * (size_t)rows, 0);
+            map.resize(col.size(), -1);
+            for (int j = 0; j < wd; ++j) {
+                const int i = row(s + j), e0 = lo(i), n_i = hi(i) - e0;
+                if (lead) {
+                    const bool publish = set == 1 && local[i] < np && pub_t[bq[i]];
+                    col[at + j] = (unsigned short)(local[i] | (publish ? kHaloPubT : 0));
+                    map[at + j] = bdiag[i] | kHaloFactor;
+                }
+                for (int e = 0; e < len; ++e) {
+                    const size_t o = at + 32 * (size_t)(e + lead) + j;
+                    if (e < n_i) {
+                        col[o] = (unsigned short)local[bcol[e0 + e]];
+                        map[o] = set ? (e0 + e) | kHaloFactor : bmap[e0 + e];
+                    } else {
+                        col[o] = (unsigned short)local[n_i ? bcol[e0] : i];
+                    }
+                }
+            }
+            if (lead)
+                for (int j = wd; j < 32; ++j) col[at + j] = kHaloNone;
+            for (int e = 0; e < rows; e += kHaloItem) {
+                const int c = std::min(kHaloItem, rows - e);
+                item.push_back((unsigned char)(c | (e + c == rows ? kHaloLast : 0)));
             }
         };
-        for (int q = p0; q < p0 + np; ++q) row(qb[q], brp[qb[q]], brp[qb[q] + 1], true);
-        for (int i : halo)
-            row(i, tri && (cls[i] & F) ? brp[i] : bdiag[i], tri && (cls[i] & Z) ? brp[i + 1] : bdiag[i] + 1, false);
-        rp.push_back((int)lcol.size() - e0);
+        auto row_lo = [&](int i) { return brp[i]; };
+        auto row_hi = [&](int i) { return brp[i + 1]; };
+        auto low_hi = [&](int i) { return bdiag[i]; };
+        auto up_lo = [&](int i) { return bdiag[i] + 1; };
+        for (int dir = 0; dir < 2; ++dir)
+            for (int g = 0; g < ng; ++g) {
+                const int no = qs[(size_t)k * ng + g + 1] - qs[(size_t)k * ng + g];
+                const int nc = dir == 0 ? h.f1[g] - h.f0[g] : h.z1[g] - h.z0[g];
+                gsl.push_back(tri ? (no + nc + 31) / 32 : 0);
+            }
+        for (int w = 0; w < kHaloWarps; ++w) {
+            went.push_back((int)(col.size() / 32));
+            wit.push_back((int)item.size() - ioff[k]);
+            for (int dir = 0; dir < 2 && tri; ++dir)
+                for (int gi = 0; gi < ng; ++gi) {
+                    const int g = dir == 0 ? gi : ng - 1 - gi;
+                    const int o0 = qs[(size_t)k * ng + g], no = qs[(size_t)k * ng + g + 1] - o0;
+                    const int c0 = dir == 0 ? h.f0[g] : h.z0[g], nc = (dir == 0 ? h.f1[g] : h.z1[g]) - c0;
+                    auto row = [&](int c) { return c < no ? qb[o0 + c] : h.rows[c0 + c - no]; };
+                    for (int s = 32 * w; s < no + nc; s += 32 * kHaloWarps) {
+                        if (dir == 0) emit(no + nc, s, row, row_lo, low_hi, 1);
+                        else emit(no + nc, s, row, up_lo, row_hi, 2);
+                    }
+                }
+            wit.push_back((int)item.size() - ioff[k]);
+            for (int s = 32 * w; s < np; s += 32 * kHaloWarps)
+                emit(np, s, [&](int c) { return qb[p0 + c]; }, row_lo, row_hi, 0);
+        }
+        TL = std::max(TL, (int)item.size() - ioff[k]);
+        ioff[k + 1] = (int)item.size();
         hoff[k + 1] = (int)hq.size();
         foff[k + 1] = (int)fl.size();
         zoff[k + 1] = (int)zl.size();
         r1off[k + 1] = (int)r1.size();
     }
-    const long long ne = (long long)lcol.size();
-    const size_t smem = halo_smem_bytes(R, RL, tri, mixed ? sizeof(float) : sizeof(double), mixed);
-    if (smem + 2048 > (size_t)optin || ne > INT32_MAX) {
+    went.push_back((int)(col.size() / 32));
+    int E = 0;
+    for (int k = 0; k < P; ++k) E = std::max(E, went[(size_t)(k + 1) * kHaloWarps] - went[(size_t)k * kHaloWarps]);
+    const size_t vsz = mixed ? sizeof(float) : sizeof(double);
+    size_t smem = halo_smem_bytes(R, RL, TL, ng, tri, vsz, mixed, E);
+    bool res = smem + 2048 <= (size_t)optin;
+    if (const char* e = getenv("PF2_HALO_RESIDENT")) res = res && atoi(e) != 0;  // tests: the other form
+    if (!res) smem = halo_smem_bytes(R, RL, TL, ng, tri, vsz, mixed, 0);
+    if (smem + 2048 > (size_t)optin || col.size() > INT32_MAX || S->nnz >= kHaloFactor) {
         S->part_why = "a part's vectors exceed the shared memory of a block";
         return PF2_OK;
     }
-    ebase[P] = (int)ne;
-    auto up = [&](auto& d, const auto& h) -> pf2_status {
-        PF2_TRY(d.alloc(std::max<size_t>(h.size(), 1)));
-        if (!h.empty()) PF2_CUDA(cudaMemcpy(d.p, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice));
+    auto up = [&](auto& d, const auto& v) -> pf2_status {
+        PF2_TRY(d.alloc(std::max<size_t>(v.size(), 1)));
+        if (!v.empty()) PF2_CUDA(cudaMemcpy(d.p, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice));
         return PF2_OK;
     };
     PF2_TRY(up(S->q_s, qs));
     PF2_TRY(up(S->q_a, qa));
-    PF2_TRY(up(S->q_amap, amap));
-    if (tri) PF2_TRY(up(S->q_fmap, fmap));
-    PF2_TRY(up(S->h_hs, hs));
+    PF2_TRY(up(S->h_dmap, dmap));
     PF2_TRY(up(S->h_hoff, hoff));
     PF2_TRY(up(S->h_hq, hq));
     PF2_TRY(up(S->h_foff, foff));
@@ -3204,26 +3278,30 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
     PF2_TRY(up(S->h_zg, zg));
     PF2_TRY(up(S->h_r1off, r1off));
     PF2_TRY(up(S->h_r1, r1));
-    PF2_TRY(up(S->h_ebase, ebase));
-    PF2_TRY(up(S->h_rp, rp));
-    PF2_TRY(up(S->h_dg, dg));
+    PF2_TRY(up(S->h_ioff, ioff));
+    PF2_TRY(up(S->h_item, item));
+    PF2_TRY(up(S->h_wit, wit));
+    PF2_TRY(up(S->h_went, went));
+    PF2_TRY(up(S->h_gsl, gsl));
+    PF2_TRY(up(S->h_col, col));
+    PF2_TRY(up(S->q_amap, map));
     PF2_TRY(up(S->h_pub, pub));
-    PF2_TRY(up(S->h_lcol, lcol));
-    PF2_TRY(S->q_val.alloc(ne));
+    PF2_TRY(S->q_val.alloc(col.size()));
     PF2_TRY(S->q_x.alloc(n));
-    if (tri) PF2_TRY(S->q_f.alloc(ne));
+    PF2_TRY(S->h_diag.alloc(dmap.size()));
     if (mixed) {
-        PF2_TRY(S->q_val32.alloc(ne));
-        PF2_TRY(S->q_f32.alloc(ne));
-        PF2_TRY(S->q_gp32.alloc(n));
-        PF2_TRY(S->q_gt32.alloc(2 * (size_t)n));
-    } else {
-        PF2_TRY(S->q_gp.alloc(n));
-        if (tri) PF2_TRY(S->q_gt.alloc(2 * (size_t)n));
+        PF2_TRY(S->q_val32.alloc(col.size()));
     }
+    const size_t words = 2 * (size_t)n * (mixed ? HaloPacket<float>::kWords : HaloPacket<double>::kWords);
+    PF2_TRY(S->h_gq.alloc(words));
+    if (tri) PF2_TRY(S->h_gt.alloc(words));
+    S->halo_TL = TL;
+    S->halo_E = E;
+    S->halo_res = res;
+    S->halo_ne = (long long)col.size();
+    S->halo_nd = (long long)dmap.size();
     S->halo = S->part = true;
     S->halo_RL = RL;
-    S->halo_entries = ne;
     S->part_local = false;
     S->part_P = P;
     S->part_R = R;
@@ -3369,13 +3447,16 @@ static bool part_eligible(const pf2_solver* S) {
 }
 
 // The partitioned CG kernel of the solver's preconditioner.
+static int part_threads(const pf2_solver* S) { return S->halo ? kHaloThreads : kPartThreads; }
 static void* part_kernel(const pf2_solver* S) {
     if (S->halo) {
-        if (S->opt.precision == PF2_PRECISION_MIXED)
-            return S->opt.precond == PF2_PRECOND_IC ? (void*)k_pcg_halo_mixed<true> : (void*)k_pcg_halo_mixed<false>;
-        if (S->opt.precond == PF2_PRECOND_IC) return (void*)k_pcg_halo<1>;
-        if (S->opt.precond == PF2_PRECOND_ILU) return (void*)k_pcg_halo<2>;
-        return (void*)k_pcg_halo<0>;
+        const bool ic = S->opt.precond == PF2_PRECOND_IC, ilu = S->opt.precond == PF2_PRECOND_ILU;
+        if (S->opt.precision == PF2_PRECISION_MIXED) {
+            if (S->halo_res) return ic ? (void*)k_pcg_halo_mixed<true, true> : (void*)k_pcg_halo_mixed<false, true>;
+            return ic ? (void*)k_pcg_halo_mixed<true, false> : (void*)k_pcg_halo_mixed<false, false>;
+        }
+        if (S->halo_res) return ic ? (void*)k_pcg_halo<1, true> : ilu ? (void*)k_pcg_halo<2, true> : (void*)k_pcg_halo<0, true>;
+        return ic ? (void*)k_pcg_halo<1, false> : ilu ? (void*)k_pcg_halo<2, false> : (void*)k_pcg_halo<0, false>;
     }
     if (S->opt.precision == PF2_PRECISION_MIXED) {
         if (S->part_local)
@@ -3673,6 +3754,16 @@ __global__ void k_gather_values(long long nnz, const double* __restrict__ val, c
     }
 }
 
+// The streams of k_pcg_halo: out[k] = val[map[k]], or fsym[...] where the map is flagged (0
+// where map[k] < 0).
+__global__ void k_gather_stream(long long ne, const double* __restrict__ val, const double* __restrict__ fsym,
+                                const int* __restrict__ map, double* __restrict__ out) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < ne; k += (long long)gridDim.x * blockDim.x) {
+        const int m = map[k];
+        out[k] = m < 0 ? 0.0 : (m & kHaloFactor) ? fsym[m & ~kHaloFactor] : val[m];
+    }
+}
+
 __global__ void k_inv_diag(int n, const double* __restrict__ val, const int* __restrict__ diag, double* invd) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) invd[i] = 1.0 / val[diag[i]];
@@ -3743,14 +3834,13 @@ static pf2_status factorize(pf2_solver* S, const pf2_csr* A, cudaStream_t st) {
         k_fsym<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(S->nnz, S->tpos.p, S->fact.p,
                                                                                     S->fsym.p);
         PF2_LAUNCH_CHECK();
-        if (S->part) {
-            const long long ne = S->halo ? S->halo_entries : S->nnz;
-            k_gather_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(
-                ne, S->fsym.p, S->q_fmap.p, S->q_f.p);
+        if (S->part && !S->halo) {
+            k_gather_values<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(
+                S->nnz, S->fsym.p, S->q_fmap.p, S->q_f.p);
             PF2_LAUNCH_CHECK();
             if (S->q_f32.p) {
-                k_to_float<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, S->q_f.p,
-                                                                                            S->q_f32.p);
+                k_to_float<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(S->nnz, S->q_f.p,
+                                                                                                S->q_f32.p);
                 PF2_LAUNCH_CHECK();
             }
         }
@@ -3852,9 +3942,13 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     const int applies = max_applies(S);
     if (S->part && !precond_only) {
         // A's values in Q order for this solve's matrix; t and z start as pending markers
-        const long long ne = S->halo ? S->halo_entries : S->nnz;
-        k_gather_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, a.A.val, S->q_amap.p,
-                                                                                         S->q_val.p);
+        const long long ne = S->halo ? S->halo_ne : S->nnz;
+        if (S->halo)
+            k_gather_stream<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(
+                ne, a.A.val, S->fsym.p, S->q_amap.p, S->q_val.p);
+        else
+            k_gather_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, a.A.val, S->q_amap.p,
+                                                                                             S->q_val.p);
         PF2_LAUNCH_CHECK();
         if (S->q_gt.p) PF2_CUDA(cudaMemsetAsync(S->q_gt.p, 0xff, S->q_gt.bytes(), st));
         if (S->q_gz.p) PF2_CUDA(cudaMemsetAsync(S->q_gz.p, 0xff, S->q_gz.bytes(), st));
@@ -3862,7 +3956,7 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
             k_to_float<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(ne, S->q_val.p,
                                                                                         S->q_val32.p);
             PF2_LAUNCH_CHECK();
-            PF2_CUDA(cudaMemsetAsync(S->q_gt32.p, 0xff, S->q_gt32.bytes(), st));
+            if (S->q_gt32.p) PF2_CUDA(cudaMemsetAsync(S->q_gt32.p, 0xff, S->q_gt32.bytes(), st));
             if (S->q_gz32.p) PF2_CUDA(cudaMemsetAsync(S->q_gz32.p, 0xff, S->q_gz32.bytes(), st));
         }
         a.part = PartCg{ S->part_P, S->part_R, S->part_ng, S->q_s.p, S->q_rp.p, S->q_col.p, S->q_diag.p, S->q_a.p,
@@ -3871,15 +3965,26 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
         PF2_CUDA(cudaMemsetAsync(S->bar.p, 0, 2 * sizeof(unsigned), st));
         PF2_CUDA(cudaMemsetAsync(S->err.p, 0, sizeof(int), st));
         PF2_CUDA(cudaMemsetAsync(S->rec.p, 0, 5 * sizeof(int), st));
+        if (S->halo_nd) {
+            k_gather_values<<<std::min((int)blocks_for(S->halo_nd), num_sms() * 8), kThreads, 0, st>>>(
+                S->halo_nd, a.A.val, S->h_dmap.p, S->h_diag.p);
+            PF2_LAUNCH_CHECK();
+        }
+        if (S->halo) {  // exchange numbers start at 1
+            PF2_CUDA(cudaMemsetAsync(S->h_gq.p, 0, S->h_gq.bytes(), st));
+            if (S->h_gt.p) PF2_CUDA(cudaMemsetAsync(S->h_gt.p, 0, S->h_gt.bytes(), st));
+            PF2_CUDA(cudaMemsetAsync(S->partial.p, 0, 8 * sizeof(double) * S->part_P, st));
+        }
         PartHalo h{};
         if (S->halo)
-            h = PartHalo{ S->part_P, S->part_ng, S->part_R, S->halo_RL, S->q_s.p, S->h_hs.p, S->h_hoff.p, S->h_hq.p,
-                          S->h_foff.p, S->h_fl.p, S->h_fg.p, S->h_zoff.p, S->h_zl.p, S->h_zg.p, S->h_r1off.p,
-                          S->h_r1.p, S->h_ebase.p, S->h_rp.p, S->h_dg.p, S->h_pub.p, S->h_lcol.p, S->q_a.p,
-                          S->q_val.p, S->q_f.p, S->q_x.p, S->q_gp.p, S->q_gt.p, S->q_val32.p, S->q_f32.p,
-                          S->q_gp32.p, S->q_gt32.p };
+            h = PartHalo{ S->part_P, S->part_ng, S->part_R, S->halo_RL, S->halo_TL, S->halo_E, S->q_s.p,
+                          S->h_hoff.p, S->h_hq.p, S->h_foff.p, S->h_fl.p, S->h_fg.p, S->h_zoff.p, S->h_zl.p,
+                          S->h_zg.p, S->h_r1off.p, S->h_r1.p, S->h_pub.p, S->h_ioff.p, S->h_item.p, S->h_wit.p,
+                          S->h_went.p, S->h_gsl.p, S->h_col.p, S->q_val.p, S->q_a.p, S->h_diag.p, S->q_x.p,
+                          S->q_val32.p, S->h_gq.p, S->h_gt.p };
         void* args[] = { &a, &h };
-        PF2_COOP_LAUNCH(part_kernel(S), dim3(S->part_P), dim3(kPartThreads), args, S->part_smem, st);
+        PF2_COOP_LAUNCH(part_kernel(S), dim3(S->part_P), dim3(part_threads(S)), args, S->part_smem,
+                        st);
         return PF2_OK;
     }
     if (S->csr && !precond_only) {  // A's values in B's numbering, for this solve's matrix
@@ -4009,7 +4114,8 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
         int occ_p = 0;
         void* pf = part_kernel(S);
         if (cudaFuncSetAttribute(pf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->part_smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, pf, kPartThreads, S->part_smem) != cudaSuccess)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, pf, part_threads(S),
+                                                          S->part_smem) != cudaSuccess)
             return fail(cuda_fail(cudaGetLastError(), "partitioned CG attributes", __FILE__, __LINE__));
         if (occ_p < 1) {  // the other kernels then
             S->part = false;

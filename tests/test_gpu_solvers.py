@@ -568,17 +568,19 @@ def test_partitioned_mixed_cg_on_the_cylinder_mesh(cuda, monkeypatch):
 
 
 @pytest.mark.parametrize("pc,precision", [("none", 0), ("jacobi", 0), ("ic", 0), ("ilu", 0), ("ic", 1), ("ilu", 1)])
-@pytest.mark.parametrize("parts", ["1", "2", "7", "23"])
-def test_halo_cg_matches_the_waiting_sweeps(cuda, monkeypatch, pc, precision, parts):
+@pytest.mark.parametrize("parts,resident", [("1", "1"), ("2", "1"), ("7", "1"), ("23", "1"), ("70", "1"), ("7", "0")])
+def test_halo_cg_matches_the_waiting_sweeps(cuda, monkeypatch, pc, precision, parts, resident):
     """The partitioned CG with halo rows (no wait inside a sweep) against the partitioned
     kernel whose sweeps wait for other parts (PF2_CG_PART=3): the rows' arithmetic is the
     same, so both converge in the same number of iterations (within 2; mixed: 10 %) to
     solutions within 1e-10 (FP64, ||r|| <= 1e-12 ||b|| on a system of condition ~1e4) and
-    1e-6 (mixed, 1e-8).  One part (no halo), two, seven ragged ones, and 23 parts of ~95 rows
-    whose halo is as large as the part."""
+    1e-6 (mixed, 1e-8).  One part (no halo), two, seven ragged ones, 23 parts of ~95 rows whose halo
+    is as large as the part, 70 parts (a wait that watches the arrival counter); the entries
+    resident in shared memory, or read from L2."""
     m, A, rp, col, val, rhs = _system(128, 16)
     b = torch.tensor(rhs, device="cuda")
     monkeypatch.setenv("PF2_CG_PARTS", parts)
+    monkeypatch.setenv("PF2_HALO_RESIDENT", resident)
     out = {}
     for part in ("2", "3"):
         monkeypatch.setenv("PF2_CG_PART", part)
