@@ -86,22 +86,45 @@ struct Graph {
 };
 
 // ---------------------------------------------------------------- forward
-__global__ void k_mpnn_encoder(Graph G, const float* __restrict__ feat, const float* __restrict__ P, float* H0,
-                               unsigned long long* mask0) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= G.n) return;
-    float f[MIN];
+// Node-row kernels take 16 threads per node, four features each: a row is one 256-byte access
+// (a thread per node touches 32 rows with every load).
+constexpr int kRowThreads = 256;
+constexpr int kRowNodes = kRowThreads / 16;
+
+// Bound by the 128 MB it writes at 499,288 nodes: 172 us with a thread per node -> 40 us.
+__global__ void __launch_bounds__(kRowThreads) k_mpnn_encoder(Graph G, const float* __restrict__ feat,
+                                                              const float* __restrict__ P, float* H0,
+                                                              unsigned long long* mask0) {
+    const int o = (threadIdx.x & 15) * 4;
+    float w[4][MIN], c[4];
 #pragma unroll
-    for (int k = 0; k < MIN; ++k) f[k] = feat[(size_t)i * MIN + k];
-    unsigned long long mk = 0ull;
-    for (int o = 0; o < MH; ++o) {
-        float s = P[kParamC0 + o];
+    for (int j = 0; j < 4; ++j) {
+        c[j] = P[kParamC0 + o + j];
 #pragma unroll
-        for (int k = 0; k < MIN; ++k) s += P[kParamW0 + o * MIN + k] * f[k];
-        if (s > 0.0f) mk |= 1ull << o;
-        H0[(size_t)i * MH + o] = s > 0.0f ? s : 0.0f;
+        for (int k = 0; k < MIN; ++k) w[j][k] = P[kParamW0 + (o + j) * MIN + k];
     }
-    mask0[i] = mk;
+    for (int base = blockIdx.x * kRowNodes; base < G.n; base += gridDim.x * kRowNodes) {
+        const int i = base + (threadIdx.x >> 4);
+        const bool in = i < G.n;
+        float f[MIN];
+#pragma unroll
+        for (int k = 0; k < MIN; ++k) f[k] = in ? feat[(size_t)i * MIN + k] : 0.0f;
+        float h[4];
+        unsigned bits = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float s = c[j];
+#pragma unroll
+            for (int k = 0; k < MIN; ++k) s += w[j][k] * f[k];
+            if (s > 0.0f) bits |= 1u << ((o + j) & 31);
+            h[j] = s > 0.0f ? s : 0.0f;
+        }
+        if (in) *reinterpret_cast<float4*>(&H0[(size_t)i * MH + o]) = make_float4(h[0], h[1], h[2], h[3]);
+        // eight lanes hold a word of the node's mask
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, d);
+        if (in && (threadIdx.x & 7) == 0) reinterpret_cast<unsigned*>(mask0)[2 * (size_t)i + (o >> 5)] = bits;
+    }
 }
 
 // mean of the neighbours' h (fixed order: ascending column)
@@ -112,6 +135,31 @@ __device__ __forceinline__ void gather_mean(const Graph& G, const float* __restr
         if (j != i) s += H[(size_t)j * MH + o];
     }
     out = s * G.deg_inv[i];
+}
+
+// The sum of the neighbours' rows of X at features o .. o + 3 added to s, in ascending column
+// order (gather_mean's order), four columns' loads in flight together (eight cost registers that
+// four CTAs per SM do not have: a pass over 499,288 nodes 2.82 ms against 2.43).
+__device__ __forceinline__ float4 gather_rows(const Graph& G, const float* __restrict__ X, int i, int o, float4 s) {
+    const int k1 = __ldg(&G.rowptr[i + 1]);
+    for (int k = __ldg(&G.rowptr[i]); k < k1; k += 4) {
+        int j[4];
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) j[u] = k + u < k1 ? __ldg(&G.col[k + u]) : i;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (j[u] != i) v[u] = __ldg(reinterpret_cast<const float4*>(&X[(size_t)j[u] * MH + o]));
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (j[u] != i) {
+                s.x += v[u].x;
+                s.y += v[u].y;
+                s.z += v[u].z;
+                s.w += v[u].w;
+            }
+    }
+    return s;
 }
 
 // One layer: h_out = h_in + relu(W [h_in ; m] + c); stores m (for the backward pass)
@@ -175,13 +223,17 @@ __global__ void __launch_bounds__(kMpnnThreads) k_mpnn_layer(Graph G, const floa
 // offset) and those adjacent in rows 128 bytes apart (its stride byte offset).
 constexpr int kTcTile = 128;  // nodes per CTA: the MMA's M (accumulator lanes 0..127)
 constexpr long long kTcPolls = 1ll << 24;
-// Dynamic shared memory of k_mpnn_layer_tc: A (32 KB) in a 64 KB region, W (16 KB) in a
-// 24 KB region.  The MMAs read A within [start, start + 32 KB) and W within 16 KB; the
-// regions are larger so that the descriptors' reads stay inside the CTA's shared memory
-// whichever way the two offsets are read.
-constexpr int kTcRegionA = 64 * 1024;
-constexpr int kTcRegionB = 24 * 1024;
-constexpr int kTcSmem = kTcRegionA + kTcRegionB;
+// The layer kernels keep 48-53 KB of shared memory (operands, and the FP32 results staged in the
+// first operand's place for coalesced rows), so four CTAs of eight warps share an SM and one
+// CTA's gather or epilogue runs under another's.  CTAs are persistent: weights, tensor memory
+// and the mbarrier are set up once.
+constexpr int kTcThreads = 256;
+constexpr int kTcCtasPerSm = 4;
+constexpr int kZStride = MH + 4;                       // staged row of 64 floats (no bank conflicts by rows)
+constexpr int kTcRegionZ = 35 * 1024;                  // kTcTile rows of kZStride floats, or A (32 KB)
+static_assert(kTcRegionZ >= kTcTile * kZStride * 4 && kTcRegionZ >= kTcTile * MK * 2 && kTcRegionZ % 1024 == 0, "region");
+constexpr int kTcSmem = kTcRegionZ + MH * MK * 2;      // + W
+constexpr int kTcBwSmem = (MK + MH) * kTcTile * 2;     // [h ; m]^T and dz^T
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -250,95 +302,6 @@ __device__ __forceinline__ void tc_ld32(unsigned taddr, float (&v)[32]) {
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// One layer as k_mpnn_layer, 128 nodes per CTA on tcgen05: h_out = h_in + relu(W [h ; m]
-// + c), m (for the backward pass) and the relu mask stored.  CTA = 4 warps; warp 0 holds
-// the 64 accumulator columns of tensor memory; thread 0 issues the eight K = 16 MMAs
-// (M = 128, N = 64); warp w reads back the rows 32 w .. 32 w + 31, one row per thread.
-// A wait that runs out sets *err and skips the outputs.
-__global__ void __launch_bounds__(128) k_mpnn_layer_tc(Graph G, const float* __restrict__ Hin,
-                                                       const __nv_bfloat16* __restrict__ Wb,
-                                                       const float* __restrict__ c, float* Hout, float* M,
-                                                       unsigned long long* mask, int* err) {
-    extern __shared__ __align__(1024) unsigned char tc_smem[];
-    unsigned char* sA = tc_smem;               // [node][in], canonical layout
-    unsigned char* sB = tc_smem + kTcRegionA;  // W [out][in], canonical layout
-    __shared__ __align__(8) unsigned long long mbar;
-    __shared__ unsigned tmem_slot;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int base = blockIdx.x * kTcTile;
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(MH));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
-        asm volatile("fence.mbarrier_init.release.cluster;");
-    }
-    for (int q = threadIdx.x; q < MH * MK; q += blockDim.x) {
-        const int o = q / MK, k = q % MK;
-        *reinterpret_cast<__nv_bfloat16*>(sB + tc_offset(o, k, MH)) = Wb[q];
-    }
-    for (int q = threadIdx.x; q < kTcTile * MH; q += blockDim.x) {
-        const int r = q / MH, o = q % MH, i = base + r;
-        float h = 0.0f, m = 0.0f;
-        if (i < G.n) {
-            h = Hin[(size_t)i * MH + o];
-            gather_mean(G, Hin, i, o, m);
-            M[(size_t)i * MH + o] = m;
-        }
-        *reinterpret_cast<__nv_bfloat16*>(sA + tc_offset(r, o, kTcTile)) = __float2bfloat16_rn(h);
-        *reinterpret_cast<__nv_bfloat16*>(sA + tc_offset(r, MH + o, kTcTile)) = __float2bfloat16_rn(m);
-    }
-    // the operands written by threads become visible to the tensor cores' async proxy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem = tmem_slot;
-    if (threadIdx.x == 0) {
-        const unsigned a0 = smem_u32(sA), b0 = smem_u32(sB);
-        constexpr unsigned idesc = tc_idesc(kTcTile, MH);
-#pragma unroll
-        for (int ks = 0; ks < MK / 16; ++ks) {
-            const unsigned long long da = tc_desc(a0 + ks * 2 * (kTcTile * 16), kTcTile * 16, 128);
-            const unsigned long long db = tc_desc(b0 + ks * 2 * (MH * 16), MH * 16, 128);
-            tc_mma(tmem, da, db, idesc, ks > 0);
-        }
-        tc_commit(smem_u32(&mbar));
-    }
-    // every thread polls; the outcome is made block-uniform (the reads below are
-    // warp-collective)
-    const bool ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), 0));
-    if (!ok) {
-        if (threadIdx.x == 0) atomicExch(err, (int)DEV_TIMEOUT);
-        mbar_wait(smem_u32(&mbar), 0);  // bounded: the MMAs may still be writing
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-        const int r = warp * 32 + lane, i = base + r;
-        unsigned long long bits = 0ull;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float acc[32];
-            tc_ld32(tmem + ((unsigned)(warp * 32) << 16) + half * 32, acc);
-            if (i < G.n) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int o = half * 32 + j;
-                    const float z = acc[j] + c[o];
-                    if (z > 0.0f) bits |= 1ull << o;
-                    Hout[(size_t)i * MH + o] = Hin[(size_t)i * MH + o] + (z > 0.0f ? z : 0.0f);
-                }
-            }
-        }
-        if (i < G.n) mask[i] = bits;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(MH));
-}
-
 // The CTA's tensor-memory columns (warp 0 allocates; power of two >= 32).
 __device__ __forceinline__ void tc_alloc(unsigned* slot, int cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols));
@@ -356,131 +319,253 @@ __device__ __forceinline__ void tc_sync_in() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// Backward node part on tcgen05: [dself ; dm] = dz W for 128 nodes per CTA (M = 128,
-// N = 128 inputs, K = 64 outputs in four MMAs); dz = dh * mask; dm scaled by 1 / d_i.
-// Operand regions of 48 KB each (16 KB used), as k_mpnn_layer_tc.
-constexpr int kTcBnRegion = 48 * 1024;
-constexpr int kTcBnSmem = 2 * kTcBnRegion;
-__global__ void __launch_bounds__(128) k_mpnn_layer_back_nodes_tc(Graph G, const float* __restrict__ dH,
-                                                                  const unsigned long long* __restrict__ mask,
-                                                                  const __nv_bfloat16* __restrict__ Wb, float* dSelf,
-                                                                  float* dMs, int* err) {
+// One layer as k_mpnn_layer, tiles of 128 nodes on tcgen05: h_out = h_in + relu(W [h ; m] + c), m
+// (for the backward pass) and the relu mask stored.  Warp 0 holds the 64 accumulator columns of
+// tensor memory; thread 0 issues the eight K = 16 MMAs (M = 128, N = 64); warp w reads back rows
+// 32 (w mod 4) .. + 31, columns 32 (w / 4) .. + 31.  A wait that runs out sets *err and ends the
+// CTA.  Bound by L2 and DRAM traffic (three rows of 256 B written or read per node besides the
+// gathered ones).  Measured at 499,288 nodes: 1,522 us with 128 threads, one (node, feature) pair
+// per thread step and two CTAs per SM (latency of the gather) -> 157 us.
+__global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) k_mpnn_layer_tc(Graph G, const float* __restrict__ Hin,
+                                                                            const __nv_bfloat16* __restrict__ Wb,
+                                                                            const float* __restrict__ c, float* Hout,
+                                                                            float* M, unsigned* mask, int* err) {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    unsigned char* sA = tc_smem;                // dz [node][out]
-    unsigned char* sB = tc_smem + kTcBnRegion;  // W^T [in][out]
+    unsigned char* sA = tc_smem;                       // [node][in], canonical layout
+    float* sZ = reinterpret_cast<float*>(tc_smem);     // relu results, once the MMAs have read A
+    unsigned char* sB = tc_smem + kTcRegionZ;          // W [out][in], canonical layout
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ unsigned tmem_slot;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int base = blockIdx.x * kTcTile;
-    if (warp == 0) tc_alloc(&tmem_slot, MK);
-    if (threadIdx.x == 0) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) tc_alloc(&tmem_slot, MH);
+    if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    for (int q = threadIdx.x; q < MH * MK; q += blockDim.x) {
+    for (int q = tid; q < MH * MK / 8; q += kTcThreads) {
+        const int o = q / (MK / 8), k = q % (MK / 8) * 8;
+        *reinterpret_cast<uint4*>(sB + tc_offset(o, k, MH)) = __ldg(reinterpret_cast<const uint4*>(Wb + o * MK + k));
+    }
+    const int ntiles = (G.n + kTcTile - 1) / kTcTile;
+    unsigned phase = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int base = tile * kTcTile;
+        for (int q = tid; q < kTcTile * 16; q += kTcThreads) {
+            const int r = q >> 4, o = (q & 15) * 4, i = base + r;
+            float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f), m = h;
+            if (i < G.n) {
+                h = __ldg(reinterpret_cast<const float4*>(&Hin[(size_t)i * MH + o]));
+                m = gather_rows(G, Hin, i, o, m);
+                const float d = __ldg(&G.deg_inv[i]);
+                m = make_float4(m.x * d, m.y * d, m.z * d, m.w * d);
+                *reinterpret_cast<float4*>(&M[(size_t)i * MH + o]) = m;
+            }
+            *reinterpret_cast<uint2*>(sA + tc_offset(r, o, kTcTile)) = make_uint2(pack_bf16(h.x, h.y), pack_bf16(h.z, h.w));
+            *reinterpret_cast<uint2*>(sA + tc_offset(r, MH + o, kTcTile)) =
+                make_uint2(pack_bf16(m.x, m.y), pack_bf16(m.z, m.w));
+        }
+        tc_sync_in();  // the operands written by threads become visible to the tensor cores' async proxy
+        const unsigned tmem = tmem_slot;
+        if (tid == 0) {
+            const unsigned a0 = smem_u32(sA), b0 = smem_u32(sB);
+            constexpr unsigned idesc = tc_idesc(kTcTile, MH);
+#pragma unroll
+            for (int ks = 0; ks < MK / 16; ++ks)
+                tc_mma(tmem, tc_desc(a0 + ks * 2 * (kTcTile * 16), kTcTile * 16, 128),
+                       tc_desc(b0 + ks * 2 * (MH * 16), MH * 16, 128), idesc, ks > 0);
+            tc_commit(smem_u32(&mbar));
+        }
+        // every thread polls; the outcome is made block-uniform (the reads below are
+        // warp-collective)
+        const bool ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), phase));
+        phase ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!ok) {
+            if (tid == 0) atomicExch(err, (int)DEV_TIMEOUT);
+            mbar_wait(smem_u32(&mbar), phase ^ 1u);  // bounded: the MMAs may still be writing
+            break;
+        }
+        {
+            const int r = (warp & 3) * 32 + lane, half = warp >> 2, i = base + r;
+            float acc[32];
+            tc_ld32(tmem + ((unsigned)((warp & 3) * 32) << 16) + half * 32, acc);
+            unsigned bits = 0u;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const float z = acc[j] + __ldg(&c[half * 32 + j]);
+                if (z > 0.0f) bits |= 1u << j;
+                acc[j] = z > 0.0f ? z : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4*>(&sZ[r * kZStride + half * 32 + j]) =
+                    make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            if (i < G.n) mask[2 * (size_t)i + half] = bits;
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int q = tid; q < kTcTile * 16; q += kTcThreads) {
+            const int r = q >> 4, o = (q & 15) * 4, i = base + r;
+            if (i >= G.n) continue;
+            const float4 h = __ldg(reinterpret_cast<const float4*>(&Hin[(size_t)i * MH + o]));
+            const float4 z = *reinterpret_cast<const float4*>(&sZ[r * kZStride + o]);
+            *reinterpret_cast<float4*>(&Hout[(size_t)i * MH + o]) =
+                make_float4(h.x + z.x, h.y + z.y, h.z + z.z, h.w + z.w);
+        }
+        __syncthreads();  // sZ is free for the next tile's operands
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tc_dealloc(tmem_slot, MH);
+}
+
+// Backward node part on tcgen05: [dself ; dm] = dz W for tiles of 128 nodes (M = 128, N = 128
+// inputs, K = 64 outputs in four MMAs); dz = dh * mask; writes dh + dself and dm / d_i.  Bound by
+// traffic (rows of dh read twice, two rows written).  Measured at 499,288 nodes: 682 us with a
+// row per thread in the epilogue (32 rows per store) -> 105 us.
+constexpr int kTcBnSmem = kTcRegionZ + MK * MH * 2;
+__global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) k_mpnn_layer_back_nodes_tc(
+    Graph G, const float* __restrict__ dH, const unsigned* __restrict__ mask, const __nv_bfloat16* __restrict__ Wb,
+    float* dSelf, float* dMs, int* err) {
+    extern __shared__ __align__(1024) unsigned char tc_smem[];
+    unsigned char* sA = tc_smem;                     // dz [node][out]
+    float* sZ = reinterpret_cast<float*>(tc_smem);   // results, 64 columns at a time
+    unsigned char* sB = tc_smem + kTcRegionZ;        // W^T [in][out]
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ unsigned tmem_slot;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) tc_alloc(&tmem_slot, MK);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+    }
+    for (int q = tid; q < MH * MK; q += kTcThreads) {
         const int o = q / MK, k = q % MK;
         *reinterpret_cast<__nv_bfloat16*>(sB + tc_offset(k, o, MK)) = Wb[q];
     }
-    for (int q = threadIdx.x; q < kTcTile * MH; q += blockDim.x) {
-        const int r = q / MH, o = q % MH, i = base + r;
-        float v = 0.0f;
-        if (i < G.n && ((mask[i] >> o) & 1ull)) v = dH[(size_t)i * MH + o];
-        *reinterpret_cast<__nv_bfloat16*>(sA + tc_offset(r, o, kTcTile)) = __float2bfloat16_rn(v);
-    }
-    tc_sync_in();
-    const unsigned tmem = tmem_slot;
-    if (threadIdx.x == 0) {
-        const unsigned a0 = smem_u32(sA), b0 = smem_u32(sB);
-        constexpr unsigned idesc = tc_idesc(kTcTile, MK);
-#pragma unroll
-        for (int ks = 0; ks < MH / 16; ++ks)
-            tc_mma(tmem, tc_desc(a0 + ks * 2 * (kTcTile * 16), kTcTile * 16, 128),
-                   tc_desc(b0 + ks * 2 * (MK * 16), MK * 16, 128), idesc, ks > 0);
-        tc_commit(smem_u32(&mbar));
-    }
-    const bool ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), 0));
-    if (!ok) {
-        if (threadIdx.x == 0) atomicExch(err, (int)DEV_TIMEOUT);
-        mbar_wait(smem_u32(&mbar), 0);
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-        const int r = warp * 32 + lane, i = base + r;
-        const float di = i < G.n ? G.deg_inv[i] : 0.0f;
-#pragma unroll
-        for (int q = 0; q < MK / 32; ++q) {
-            float acc[32];
-            tc_ld32(tmem + ((unsigned)(warp * 32) << 16) + q * 32, acc);
+    const int ntiles = (G.n + kTcTile - 1) / kTcTile;
+    unsigned phase = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int base = tile * kTcTile;
+        for (int q = tid; q < kTcTile * 16; q += kTcThreads) {
+            const int r = q >> 4, o = (q & 15) * 4, i = base + r;
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (i < G.n) {
+                const unsigned b = __ldg(&mask[2 * (size_t)i + (o >> 5)]) >> (o & 31);
+                v = __ldg(reinterpret_cast<const float4*>(&dH[(size_t)i * MH + o]));
+                v = make_float4(b & 1u ? v.x : 0.0f, b & 2u ? v.y : 0.0f, b & 4u ? v.z : 0.0f, b & 8u ? v.w : 0.0f);
+            }
+            *reinterpret_cast<uint2*>(sA + tc_offset(r, o, kTcTile)) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+        }
+        tc_sync_in();
+        const unsigned tmem = tmem_slot;
+        if (tid == 0) {
+            const unsigned a0 = smem_u32(sA), b0 = smem_u32(sB);
+            constexpr unsigned idesc = tc_idesc(kTcTile, MK);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int k = q * 32 + j;
-                    if (k < MH) dSelf[(size_t)i * MH + k] = acc[j];
-                    else dMs[(size_t)i * MH + (k - MH)] = acc[j] * di;
+            for (int ks = 0; ks < MH / 16; ++ks)
+                tc_mma(tmem, tc_desc(a0 + ks * 2 * (kTcTile * 16), kTcTile * 16, 128),
+                       tc_desc(b0 + ks * 2 * (MK * 16), MK * 16, 128), idesc, ks > 0);
+            tc_commit(smem_u32(&mbar));
+        }
+        const bool ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), phase));
+        phase ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!ok) {
+            if (tid == 0) atomicExch(err, (int)DEV_TIMEOUT);
+            mbar_wait(smem_u32(&mbar), phase ^ 1u);
+            break;
+        }
+#pragma unroll 1
+        for (int p = 0; p < 2; ++p) {  // columns 64 p .. 64 p + 63: dself, then dm
+            const int rr = (warp & 3) * 32 + lane, half = warp >> 2;
+            float acc[32];
+            tc_ld32(tmem + ((unsigned)((warp & 3) * 32) << 16) + p * MH + half * 32, acc);
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4*>(&sZ[rr * kZStride + half * 32 + j]) =
+                    make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncthreads();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int q = tid; q < kTcTile * 16; q += kTcThreads) {
+                const int r = q >> 4, o = (q & 15) * 4, i = base + r;
+                if (i >= G.n) continue;
+                const float4 z = *reinterpret_cast<const float4*>(&sZ[r * kZStride + o]);
+                if (p == 0) {
+                    const float4 h = __ldg(reinterpret_cast<const float4*>(&dH[(size_t)i * MH + o]));
+                    *reinterpret_cast<float4*>(&dSelf[(size_t)i * MH + o]) =
+                        make_float4(h.x + z.x, h.y + z.y, h.z + z.z, h.w + z.w);
+                } else {
+                    const float d = __ldg(&G.deg_inv[i]);
+                    *reinterpret_cast<float4*>(&dMs[(size_t)i * MH + o]) =
+                        make_float4(z.x * d, z.y * d, z.z * d, z.w * d);
                 }
             }
+            __syncthreads();
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, MK);
+    if (warp == 0) tc_dealloc(tmem_slot, MK);
 }
 
 // Backward weight part on tcgen05: per-CTA partial dW[out][in] = sum over the CTA's node
 // tiles of [h ; m]^T dz (M = 128 inputs, N = 64 outputs, K = 128 nodes per tile,
-// accumulated in tensor memory across the tiles) and dc on the CUDA cores.  A tile's
-// operands are overwritten only after its MMAs completed (mbarrier phase per tile).
-// Operand regions as k_mpnn_layer_tc.
-__global__ void __launch_bounds__(128) k_mpnn_layer_back_weights_tc(Graph G, const float* __restrict__ Hin,
-                                                                    const float* __restrict__ M,
-                                                                    const float* __restrict__ dH,
-                                                                    const unsigned long long* __restrict__ mask,
-                                                                    float* part, int* err) {
+// accumulated in tensor memory across the tiles) and dc on the CUDA cores.  A thread packs eight
+// nodes of one feature into the 16 bytes they take in the K-major operand (coalesced loads, no
+// bank conflicts); a tile's operands are overwritten only after its MMAs completed (mbarrier
+// phase per tile).  Bound by DRAM traffic (rows of h, m and dh).  Measured at 499,288 nodes: 626 us
+// with 2-byte stores and dc summed by 64 threads -> 137 us.
+__global__ void __launch_bounds__(kTcThreads, 2) k_mpnn_layer_back_weights_tc(
+    Graph G, const float* __restrict__ Hin, const float* __restrict__ M, const float* __restrict__ dH,
+    const unsigned* __restrict__ mask, float* part, int* err) {
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    unsigned char* sA = tc_smem;               // [h ; m]^T [in][node]
-    unsigned char* sB = tc_smem + kTcRegionA;  // dz^T [out][node]
+    unsigned char* sA = tc_smem;                      // [h ; m]^T [in][node]
+    unsigned char* sB = tc_smem + MK * kTcTile * 2;   // dz^T [out][node]
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ unsigned tmem_slot;
-    __shared__ float sC[MH];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) tc_alloc(&tmem_slot, MH);
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    for (int o = threadIdx.x; o < MH; o += blockDim.x) sC[o] = 0.0f;
     const int ntiles = (G.n + kTcTile - 1) / kTcTile;
+    const int o = tid & (MH - 1);
     unsigned phase = 0;
     bool ok = true, issued = false;
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    float dc = 0.0f;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int base = tile * kTcTile;
-        if (issued) {  // the previous tile's MMAs have read the operands
-            ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), phase));
-            phase ^= 1u;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!ok) break;
-        }
-        for (int q = threadIdx.x; q < kTcTile * MH; q += blockDim.x) {
-            const int r = q / MH, o = q % MH, i = base + r;
-            float h = 0.0f, m = 0.0f, z = 0.0f;
-            if (i < G.n) {
-                h = Hin[(size_t)i * MH + o];
-                m = M[(size_t)i * MH + o];
-                if ((mask[i] >> o) & 1ull) z = dH[(size_t)i * MH + o];
+        for (int rb = tid >> 6; rb < kTcTile / 8; rb += kTcThreads / MH) {
+            float h[8], m[8], z[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int i = base + rb * 8 + u;
+                const bool in = i < G.n;
+                const size_t e = (size_t)i * MH + o;
+                h[u] = in ? __ldg(&Hin[e]) : 0.0f;
+                m[u] = in ? __ldg(&M[e]) : 0.0f;
+                z[u] = in && ((__ldg(&mask[2 * (size_t)i + (o >> 5)]) >> (o & 31)) & 1u) ? __ldg(&dH[e]) : 0.0f;
             }
-            *reinterpret_cast<__nv_bfloat16*>(sA + tc_offset(o, r, MK)) = __float2bfloat16_rn(h);
-            *reinterpret_cast<__nv_bfloat16*>(sA + tc_offset(MH + o, r, MK)) = __float2bfloat16_rn(m);
-            *reinterpret_cast<__nv_bfloat16*>(sB + tc_offset(o, r, MH)) = __float2bfloat16_rn(z);
+            if (issued && rb == (tid >> 6)) {  // the previous tile's MMAs have read the operands
+                ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), phase));
+                phase ^= 1u;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!ok) break;
+            }
+            auto pack = [](const float* v) {
+                return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+            };
+            *reinterpret_cast<uint4*>(sA + tc_offset(o, rb * 8, MK)) = pack(h);
+            *reinterpret_cast<uint4*>(sA + tc_offset(MH + o, rb * 8, MK)) = pack(m);
+            *reinterpret_cast<uint4*>(sB + tc_offset(o, rb * 8, MH)) = pack(z);
         }
+        if (!ok) break;
         tc_sync_in();
-        // dc: the outputs' sums of the rounded dz over the tile's nodes
-        for (int o = threadIdx.x; o < MH; o += blockDim.x) {
-            float s = 0.0f;
-            for (int r = 0; r < kTcTile; ++r)
-                s += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(sB + tc_offset(o, r, MH)));
-            sC[o] += s;
-        }
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
             const unsigned a0 = smem_u32(sA), b0 = smem_u32(sB);
             constexpr unsigned idesc = tc_idesc(MK, MH);
 #pragma unroll
@@ -489,88 +574,129 @@ __global__ void __launch_bounds__(128) k_mpnn_layer_back_weights_tc(Graph G, con
                        tc_desc(b0 + ks * 2 * (MH * 16), MH * 16, 128), idesc, (issued || ks > 0) ? 1 : 0);
             tc_commit(smem_u32(&mbar));
         }
+        // dc: the outputs' sums of the rounded dz over the tile's nodes in order, beside the MMAs
+        if (tid >= kTcThreads - MH) {
+            float s = 0.0f;
+#pragma unroll 4
+            for (int rb = 0; rb < kTcTile / 8; ++rb) {
+                const uint4 v = *reinterpret_cast<const uint4*>(sB + tc_offset(o, rb * 8, MH));
+                const unsigned w[4] = { v.x, v.y, v.z, v.w };
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    s += __uint_as_float(w[u] << 16);
+                    s += __uint_as_float(w[u] & 0xffff0000u);
+                }
+            }
+            dc += s;
+        }
         issued = true;
-        __syncthreads();  // sC complete before the next tile overwrites sB
     }
     if (issued && ok) {
         ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), phase));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (!ok) {
-        if (threadIdx.x == 0) atomicExch(err, (int)DEV_TIMEOUT);
+        if (tid == 0) atomicExch(err, (int)DEV_TIMEOUT);
         if (issued) mbar_wait(smem_u32(&mbar), phase);
     }
     float* P = part + (size_t)blockIdx.x * (MH * MK + MH);
     const unsigned tmem = tmem_slot;
-    const int in = warp * 32 + lane;  // accumulator lane = input row of dW^T
+    const int in = (warp & 3) * 32 + lane, q = warp >> 2;  // accumulator lane = input row of dW^T
+    float acc[32];
 #pragma unroll
-    for (int q = 0; q < MH / 32; ++q) {
-        float acc[32];
-        if (issued && ok) tc_ld32(tmem + ((unsigned)(warp * 32) << 16) + q * 32, acc);
-        else
+    for (int j = 0; j < 32; ++j) acc[j] = 0.0f;
+    if (issued && ok) tc_ld32(tmem + ((unsigned)((warp & 3) * 32) << 16) + q * 32, acc);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[j] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) P[(q * 32 + j) * MK + in] = acc[j];
-    }
-    __syncthreads();
-    for (int o = threadIdx.x; o < MH; o += blockDim.x) P[MH * MK + o] = sC[o];
+    for (int j = 0; j < 32; ++j) P[(q * 32 + j) * MK + in] = acc[j];
+    if (tid >= kTcThreads - MH) P[MH * MK + o] = dc;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, MH);
+    if (warp == 0) tc_dealloc(tmem_slot, MH);
 }
 
-// y = w4 . h + c4; optionally loss partials and dy = 2 (y - t) / n
-__global__ void k_mpnn_decoder(int n, const float* __restrict__ H, const float* __restrict__ P, float* y,
-                               const float* __restrict__ target, float* dy, double* loss_part) {
+// y = w4 . h + c4 (terms in feature order) for tiles of 128 nodes whose rows are staged in shared
+// memory by coalesced loads.  With a target also the backward pass of the output layer: dy =
+// 2 (y - t) / n, dh = dy w4, and per-CTA partials of (dw4, dc4) and of the loss.  Bound by traffic (one
+// row read, one written).  Measured at 499,288 nodes, training: 116 us for y and 302 us for the
+// gradients as two kernels with a thread per node -> 46 us.
+constexpr int kDecThreads = 256;
+constexpr int kDecTile = 128;
+constexpr int kDecStride = MH + 1;
+__global__ void __launch_bounds__(kDecThreads) k_mpnn_decoder(int n, const float* __restrict__ H,
+                                                              const float* __restrict__ P, float* y,
+                                                              const float* __restrict__ target, float* dH,
+                                                              double* part /* [grid][MH + 1] */, double* loss_part) {
+    __shared__ float sH[kDecTile * kDecStride];
+    __shared__ float sW[MH + 1], sD[kDecTile], sP[kDecThreads / MH][MH + 1];
+    static_assert(kDecThreads / MH == 4 && kDecTile == 128, "32 nodes per partial sum, four per tile");
     __shared__ double sh[40];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (i < n) {
-        float s = P[kParamC4];
-        for (int o = 0; o < MH; ++o) s += P[kParamW4 + o] * H[(size_t)i * MH + o];
-        y[i] = s;
-        if (target) {
-            const float r = s - target[i];
-            dy[i] = 2.0f * r / (float)n;
-            l = (double)r * r;
+    const int tid = threadIdx.x;
+    if (tid <= MH) sW[tid] = P[kParamW4 + tid];  // w4, then c4
+    const int o = tid & (MH - 1), g = tid >> 6;
+    double grad = 0.0;  // threads 0 .. MH: (dw4, dc4) over this block's tiles
+    double loss = 0.0;
+    for (int base = blockIdx.x * kDecTile; base < n; base += gridDim.x * kDecTile) {
+        __syncthreads();  // the previous tile's readers are done
+        for (int q = tid; q < kDecTile * 16; q += kDecThreads) {
+            const int r = q >> 4, f = (q & 15) * 4, i = base + r;
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (i < n) v = __ldg(reinterpret_cast<const float4*>(&H[(size_t)i * MH + f]));
+            float* d = &sH[r * kDecStride + f];
+            d[0] = v.x;
+            d[1] = v.y;
+            d[2] = v.z;
+            d[3] = v.w;
         }
+        __syncthreads();
+        if (tid < kDecTile) {
+            const int i = base + tid;
+            float s = sW[MH];
+#pragma unroll 16
+            for (int k = 0; k < MH; ++k) s += sW[k] * sH[tid * kDecStride + k];
+            float d = 0.0f;
+            if (i < n) {
+                y[i] = s;
+                if (target) {
+                    const float r = s - target[i];
+                    d = 2.0f * r / (float)n;
+                    loss += (double)r * r;
+                }
+            }
+            sD[tid] = d;
+        }
+        if (!target) continue;
+        __syncthreads();
+        for (int q = tid; q < kDecTile * 16; q += kDecThreads) {
+            const int r = q >> 4, f = (q & 15) * 4, i = base + r;
+            if (i >= n) continue;
+            const float d = sD[r];
+            *reinterpret_cast<float4*>(&dH[(size_t)i * MH + f]) =
+                make_float4(d * sW[f], d * sW[f + 1], d * sW[f + 2], d * sW[f + 3]);
+        }
+        // the tile's (dw4, dc4): 32 nodes by a binary tree (node l with l + 16, ...), the four sums in
+        // order, the tiles in FP64
+        auto tree = [&](auto term) {
+            float v[16];
+#pragma unroll
+            for (int l = 0; l < 16; ++l) v[l] = __fadd_rn(term(l), term(l + 16));
+#pragma unroll
+            for (int d = 8; d > 0; d >>= 1)
+#pragma unroll
+                for (int l = 0; l < d; ++l) v[l] = __fadd_rn(v[l], v[l + d]);
+            return v[0];
+        };
+        sP[g][o] = tree([&](int l) { return __fmul_rn(sD[32 * g + l], sH[(32 * g + l) * kDecStride + o]); });
+        if (o == 0) sP[g][MH] = tree([&](int l) { return sD[32 * g + l]; });
+        __syncthreads();
+        if (tid <= MH) grad += (double)(((sP[0][tid] + sP[1][tid]) + sP[2][tid]) + sP[3][tid]);
     }
-    if (target) {
-        l = block_sum(l, sh);
-        if (threadIdx.x == 0) loss_part[blockIdx.x] = l;
-    }
+    if (!target) return;
+    loss = block_sum(loss, sh);
+    if (tid <= MH) part[(size_t)blockIdx.x * (MH + 1) + tid] = grad;
+    if (tid == 0) loss_part[blockIdx.x] = loss;
 }
 
 // ---------------------------------------------------------------- backward
-// dh = dy w4, and per-block partials of (dw4, dc4)
-__global__ void k_mpnn_decoder_back(int n, const float* __restrict__ H, const float* __restrict__ P,
-                                    const float* __restrict__ dy, float* dH, float* part /* [grid][MH+1] */) {
-    __shared__ float sp[MH + 1][kMpnnThreads / 32];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const float d = (i < n) ? dy[i] : 0.0f;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int o = 0; o <= MH; ++o) {
-        float v = 0.0f;
-        if (i < n) {
-            if (o < MH) {
-                v = d * H[(size_t)i * MH + o];
-                dH[(size_t)i * MH + o] = d * P[kParamW4 + o];
-            } else {
-                v = d;
-            }
-        }
-        v = warp_sumf(v);
-        if (lane == 0) sp[o][w] = v;
-    }
-    __syncthreads();
-    for (int o = threadIdx.x; o <= MH; o += blockDim.x) {
-        float s = 0.0f;
-        for (int k = 0; k < kMpnnThreads / 32; ++k) s += sp[o][k];
-        part[(size_t)blockIdx.x * (MH + 1) + o] = s;
-    }
-}
-
 // One layer backward, node part: dz = dh * mask; [dself ; dm] = dz W (tensor cores);
 // writes dself and dm / d_i.
 __global__ void __launch_bounds__(kMpnnThreads) k_mpnn_layer_back_nodes(Graph G, const float* __restrict__ dH,
@@ -614,18 +740,21 @@ __global__ void __launch_bounds__(kMpnnThreads) k_mpnn_layer_back_nodes(Graph G,
     }
 }
 
-// dh_prev_i = dh_i + dself_i + sum_{k in N(i)} dm_k / d_k (the graph is symmetric)
-__global__ void k_mpnn_agg_back(Graph G, const float* __restrict__ dH, const float* __restrict__ dSelf,
-                                const float* __restrict__ dMs, float* dHprev) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long long)G.n * MH) return;
-    const int i = (int)(q / MH), o = (int)(q % MH);
-    float s = dH[q] + dSelf[q];
-    for (int k = G.rowptr[i]; k < G.rowptr[i + 1]; ++k) {
-        const int j = G.col[k];
-        if (j != i) s += dMs[(size_t)j * MH + o];
+// dh_prev_i = (dh_i + dself_i) + sum_{k in N(i)} dm_k / d_k (the graph is symmetric); dH null:
+// dSelf holds dh + dself.  Measured at 499,288 nodes: 257 us with a thread per (node, feature) ->
+// 91 us.
+__global__ void __launch_bounds__(kRowThreads) k_mpnn_agg_back(Graph G, const float* __restrict__ dH,
+                                                               const float* __restrict__ dSelf,
+                                                               const float* __restrict__ dMs, float* dHprev) {
+    const int i = blockIdx.x * kRowNodes + (threadIdx.x >> 4), o = (threadIdx.x & 15) * 4;
+    if (i >= G.n) return;
+    const size_t q = (size_t)i * MH + o;
+    float4 s = __ldg(reinterpret_cast<const float4*>(&dSelf[q]));
+    if (dH) {
+        const float4 h = __ldg(reinterpret_cast<const float4*>(&dH[q]));
+        s = make_float4(h.x + s.x, h.y + s.y, h.z + s.z, h.w + s.w);
     }
-    dHprev[q] = s;
+    *reinterpret_cast<float4*>(&dHprev[q]) = gather_rows(G, dMs, i, o, s);
 }
 
 // One layer backward, weight part: per-CTA partial dW (= [h ; m]^T dz, tensor cores) and
@@ -692,41 +821,80 @@ __global__ void __launch_bounds__(kMpnnThreads) k_mpnn_layer_back_weights(Graph 
     for (int o = threadIdx.x; o < MH; o += blockDim.x) P[MH * MK + o] = sC[o];
 }
 
-// Encoder backward: per-block partials of (dW0, dc0)
-__global__ void k_mpnn_encoder_back(int n, const float* __restrict__ feat, const float* __restrict__ dH,
-                                    const unsigned long long* __restrict__ mask0, float* part /* [grid][MH*MIN+MH] */) {
-    __shared__ float sp[MH * (MIN + 1)];
-    for (int q = threadIdx.x; q < MH * (MIN + 1); q += blockDim.x) sp[q] = 0.0f;
-    __syncthreads();
+// Encoder backward: per-block partials of (dW0, dc0).  Thread (o, k) sums dz_o f_k (k < MIN) or
+// dz_o (k == MIN) over the block's nodes in order, from tiles of 64 nodes staged in shared memory
+// by coalesced loads, the next tile's loads in flight meanwhile.  Measured at 499,288 nodes:
+// 1,800 us with every thread loading its own terms -> 116 us.
+constexpr int kEncThreads = MH * (MIN + 1);
+constexpr int kEncTile = 64;
+__global__ void __launch_bounds__(kEncThreads) k_mpnn_encoder_back(int n, const float* __restrict__ feat,
+                                                                   const float* __restrict__ dH,
+                                                                   const unsigned* __restrict__ mask0,
+                                                                   float* part /* [grid][MH*MIN+MH] */) {
+    __shared__ __align__(16) float sD[kEncTile][MH];
+    __shared__ float sF[kEncTile][MIN];
+    __shared__ unsigned sM[kEncTile][2];
+    const int tid = threadIdx.x, o = tid / (MIN + 1), k = tid % (MIN + 1);
     const int nper = (n + gridDim.x - 1) / gridDim.x;
-    const int i0 = blockIdx.x * nper, i1 = min(n, i0 + nper);
-    // thread (o, k): sums dz_o * f_k (k < MIN) or dz_o (k == MIN) over this block's nodes
-    for (int q = threadIdx.x; q < MH * (MIN + 1); q += blockDim.x) {
-        const int o = q / (MIN + 1), k = q % (MIN + 1);
-        float s = 0.0f;
-        for (int i = i0; i < i1; ++i) {
-            if (!((mask0[i] >> o) & 1ull)) continue;
-            const float dz = dH[(size_t)i * MH + o];
-            s += (k < MIN) ? dz * feat[(size_t)i * MIN + k] : dz;
+    const int i0 = (int)std::min((long long)n, (long long)blockIdx.x * nper), i1 = min(n, i0 + nper);
+    constexpr int V = (kEncTile * 16 + kEncThreads - 1) / kEncThreads;  // float4 of dz per thread
+    float4 d[V];
+    float f = 0.0f;
+    unsigned m = 0u;
+    auto load = [&](int base) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int q = tid + v * kEncThreads, i = base + (q >> 4);
+            if (q < kEncTile * 16 && i < i1) d[v] = __ldg(reinterpret_cast<const float4*>(&dH[(size_t)i * MH + (q & 15) * 4]));
         }
-        sp[q] = s;
+        if (tid < kEncTile * MIN && base + tid / MIN < i1) f = __ldg(&feat[(size_t)base * MIN + tid]);
+        if (tid < 2 * kEncTile && base + tid / 2 < i1) m = __ldg(&mask0[2 * (size_t)base + tid]);
+    };
+    static_assert(kEncTile * MIN <= kEncThreads && 2 * kEncTile <= kEncThreads, "one feature and mask word per thread");
+    float s = 0.0f;
+    if (i0 < i1) load(i0);
+    for (int base = i0; base < i1; base += kEncTile) {
+        __syncthreads();  // the previous tile's readers are done
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int q = tid + v * kEncThreads;
+            if (q < kEncTile * 16) *reinterpret_cast<float4*>(&sD[q >> 4][(q & 15) * 4]) = d[v];
+        }
+        if (tid < kEncTile * MIN) (&sF[0][0])[tid] = f;
+        if (tid < 2 * kEncTile) (&sM[0][0])[tid] = m;
+        __syncthreads();
+        if (base + kEncTile < i1) load(base + kEncTile);
+        const int cnt = min(kEncTile, i1 - base);
+        for (int r = 0; r < cnt; ++r) {
+            if (!((sM[r][o >> 5] >> (o & 31)) & 1u)) continue;
+            const float dz = sD[r][o];
+            s += (k < MIN) ? dz * sF[r][k < MIN ? k : 0] : dz;
+        }
     }
-    __syncthreads();
     float* P = part + (size_t)blockIdx.x * (MH * MIN + MH);
-    for (int q = threadIdx.x; q < MH * (MIN + 1); q += blockDim.x) {
-        const int o = q / (MIN + 1), k = q % (MIN + 1);
-        if (k < MIN) P[o * MIN + k] = sp[q];
-        else P[MH * MIN + o] = sp[q];
-    }
+    if (k < MIN) P[o * MIN + k] = s;
+    else P[MH * MIN + o] = s;
 }
 
-// grad[off + j] = sum_b part[b * width + j], fixed order, FP64 accumulation
-__global__ void k_reduce_cols(const float* __restrict__ part, int nb, int width, float* grad, int off) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= width) return;
+// grad[off + j] = sum_b part[b * width + j], fixed order, FP64 accumulation: a block takes 32
+// columns, warp w the rows w, w + 8, ...; the eight sums are added in order.
+template <class T>
+__global__ void __launch_bounds__(256) k_reduce_cols(const T* __restrict__ part, int nb, int width, float* grad, int off) {
+    __shared__ double sh[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[(size_t)b * width + j];
-    grad[off + j] = (float)s;
+    if (j < width) {
+#pragma unroll 4
+        for (int b = w; b < nb; b += 8) s += (double)__ldg(&part[(size_t)b * width + j]);
+    }
+    sh[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && j < width) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s += sh[k][lane];
+        grad[off + j] = (float)s;
+    }
 }
 
 __global__ void k_adamw(int np, float* P, const float* __restrict__ g, float* m, float* v, float c1, float c2,
@@ -763,13 +931,15 @@ using namespace pf2;
 struct pf2_mpnn {
     int n = 0;
     const pf2_mesh* mesh = nullptr;
-    DevBuf<float> P, grad, am, av, dinv, feat, y, dy, H, M, dH, dH2, dSelf, dMs, part, target;
+    DevBuf<float> P, grad, am, av, dinv, feat, y, H, M, dH, dH2, dSelf, dMs, part, target;
     DevBuf<unsigned long long> mask;
     DevBuf<__nv_bfloat16> Wb;
-    DevBuf<double> loss_part;
+    DevBuf<double> loss_part, dpart;
     DevBuf<int> err;  // a tcgen05 wait that ran out (DEV_TIMEOUT)
     int step = 0;
-    int wgrid = 0;
+    int wgrid = 0;  // blocks of the gradient kernels (rows of part)
+    int tgrid = 0;  // persistent blocks of the layer kernels
+    int dgrid = 0;  // blocks of the decoder (rows of dpart and loss_part)
     bool tc = true;  // the layer GEMMs on tcgen05 (PF2_MPNN_MMA=sync: mma.sync)
     Graph graph() const { return Graph{ n, mesh->rowptr.p, mesh->col.p, dinv.p }; }
     float* Hl(int l) { return H.p + (size_t)l * n * MH; }
@@ -798,16 +968,19 @@ pf2_status mpnn_checkpoint(pf2_mpnn* N, CkptFile& io, cudaStream_t st) {
     return PF2_OK;
 }
 
+static unsigned* words(unsigned long long* m) { return reinterpret_cast<unsigned*>(m); }
+
 static pf2_status mpnn_forward(pf2_mpnn* N, cudaStream_t st) {
     const Graph G = N->graph();
-    k_mpnn_encoder<<<blocks_for(N->n), kThreads, 0, st>>>(G, N->feat.p, N->P.p, N->Hl(0), N->maskl(0));
+    k_mpnn_encoder<<<std::min(blocks_for(N->n, kRowNodes), (unsigned)num_sms() * 8), kRowThreads, 0, st>>>(
+        G, N->feat.p, N->P.p, N->Hl(0), N->maskl(0));
     PF2_LAUNCH_CHECK();
     const unsigned tiles = blocks_for(N->n, kTile);
     for (int l = 0; l < ML; ++l) {
         if (N->tc)
-            k_mpnn_layer_tc<<<blocks_for(N->n, kTcTile), 128, kTcSmem, st>>>(
+            k_mpnn_layer_tc<<<N->tgrid, kTcThreads, kTcSmem, st>>>(
                 G, N->Hl(l), N->Wb.p + (size_t)l * MH * MK, N->P.p + kParamLayer0 + l * kLayerSize + MH * MK,
-                N->Hl(l + 1), N->Ml(l), N->maskl(l + 1), N->err.p);
+                N->Hl(l + 1), N->Ml(l), words(N->maskl(l + 1)), N->err.p);
         else
             k_mpnn_layer<<<tiles, kMpnnThreads, 0, st>>>(G, N->Hl(l), N->Wb.p + (size_t)l * MH * MK,
                                                          N->P.p + kParamLayer0 + l * kLayerSize + MH * MK,
@@ -817,45 +990,53 @@ static pf2_status mpnn_forward(pf2_mpnn* N, cudaStream_t st) {
     return PF2_OK;
 }
 
+static pf2_status mpnn_decoder(pf2_mpnn* N, float* y, const float* target, cudaStream_t st) {
+    k_mpnn_decoder<<<N->dgrid, kDecThreads, 0, st>>>(N->n, N->Hl(ML), N->P.p, y, target, target ? N->dH.p : nullptr,
+                                                     target ? N->dpart.p : nullptr, target ? N->loss_part.p : nullptr);
+    PF2_LAUNCH_CHECK();
+    return PF2_OK;
+}
+
+template <class T>
+static pf2_status reduce_cols(pf2_mpnn* N, const T* part, int nb, int width, int off, cudaStream_t st) {
+    k_reduce_cols<T><<<blocks_for(width, 32), 256, 0, st>>>(part, nb, width, N->grad.p, off);
+    PF2_LAUNCH_CHECK();
+    return PF2_OK;
+}
+
+// After mpnn_decoder with a target: dH holds the gradient of the last layer's output, part the
+// output layer's partials.
 static pf2_status mpnn_backward(pf2_mpnn* N, cudaStream_t st) {
     const Graph G = N->graph();
-    const unsigned nb = blocks_for(N->n, kMpnnThreads);
-    k_mpnn_decoder_back<<<nb, kMpnnThreads, 0, st>>>(N->n, N->Hl(ML), N->P.p, N->dy.p, N->dH.p, N->part.p);
-    PF2_LAUNCH_CHECK();
-    k_reduce_cols<<<blocks_for(MH + 1), kThreads, 0, st>>>(N->part.p, (int)nb, MH + 1, N->grad.p, kParamW4);
-    PF2_LAUNCH_CHECK();
+    PF2_TRY(reduce_cols(N, N->dpart.p, N->dgrid, MH + 1, kParamW4, st));
     const unsigned tiles = blocks_for(N->n, kTile);
     float* dh = N->dH.p;
     float* dh2 = N->dH2.p;
     for (int l = ML - 1; l >= 0; --l) {
         const __nv_bfloat16* W = N->Wb.p + (size_t)l * MH * MK;
         if (N->tc)
-            k_mpnn_layer_back_weights_tc<<<N->wgrid, 128, kTcSmem, st>>>(G, N->Hl(l), N->Ml(l), dh, N->maskl(l + 1),
-                                                                         N->part.p, N->err.p);
+            k_mpnn_layer_back_weights_tc<<<N->wgrid, kTcThreads, kTcBwSmem, st>>>(
+                G, N->Hl(l), N->Ml(l), dh, words(N->maskl(l + 1)), N->part.p, N->err.p);
         else
             k_mpnn_layer_back_weights<<<N->wgrid, kMpnnThreads, 0, st>>>(G, N->Hl(l), N->Ml(l), dh,
                                                                          N->maskl(l + 1), N->part.p);
         PF2_LAUNCH_CHECK();
-        k_reduce_cols<<<blocks_for(kLayerSize), kThreads, 0, st>>>(N->part.p, N->wgrid, kLayerSize, N->grad.p,
-                                                                   kParamLayer0 + l * kLayerSize);
-        PF2_LAUNCH_CHECK();
+        PF2_TRY(reduce_cols(N, N->part.p, N->wgrid, kLayerSize, kParamLayer0 + l * kLayerSize, st));
         if (N->tc)
-            k_mpnn_layer_back_nodes_tc<<<blocks_for(N->n, kTcTile), 128, kTcBnSmem, st>>>(
-                G, dh, N->maskl(l + 1), W, N->dSelf.p, N->dMs.p, N->err.p);
+            k_mpnn_layer_back_nodes_tc<<<N->tgrid, kTcThreads, kTcBnSmem, st>>>(
+                G, dh, words(N->maskl(l + 1)), W, N->dSelf.p, N->dMs.p, N->err.p);
         else
             k_mpnn_layer_back_nodes<<<tiles, kMpnnThreads, 0, st>>>(G, dh, N->maskl(l + 1), W, N->dSelf.p,
                                                                     N->dMs.p);
         PF2_LAUNCH_CHECK();
-        k_mpnn_agg_back<<<blocks_for((long long)N->n * MH), kThreads, 0, st>>>(G, dh, N->dSelf.p, N->dMs.p, dh2);
+        k_mpnn_agg_back<<<blocks_for(N->n, kRowNodes), kRowThreads, 0, st>>>(G, N->tc ? nullptr : dh, N->dSelf.p,
+                                                                             N->dMs.p, dh2);
         PF2_LAUNCH_CHECK();
         std::swap(dh, dh2);
     }
-    k_mpnn_encoder_back<<<N->wgrid, kThreads, 0, st>>>(N->n, N->feat.p, dh, N->maskl(0), N->part.p);
+    k_mpnn_encoder_back<<<N->wgrid, kEncThreads, 0, st>>>(N->n, N->feat.p, dh, words(N->maskl(0)), N->part.p);
     PF2_LAUNCH_CHECK();
-    k_reduce_cols<<<blocks_for(MH * MIN + MH), kThreads, 0, st>>>(N->part.p, N->wgrid, MH * MIN + MH, N->grad.p,
-                                                                  kParamW0);
-    PF2_LAUNCH_CHECK();
-    return PF2_OK;
+    return reduce_cols(N, N->part.p, N->wgrid, MH * MIN + MH, kParamW0, st);
 }
 
 }  // namespace pf2
@@ -871,16 +1052,18 @@ pf2_status pf2_mpnn_create(const pf2_mesh* mesh, unsigned long long seed, pf2_mp
     const size_t n = N->n;
     auto fail = [&](pf2_status s) { delete N; return s; };
     N->wgrid = std::max(1, std::min((int)blocks_for(N->n, kTile), num_sms() * 2));
-    const size_t part = std::max<size_t>((size_t)N->wgrid * (MH * MK + MH),
-                                         (size_t)blocks_for(N->n, kMpnnThreads) * (MH + 1));
+    N->tgrid = std::max(1, std::min((int)blocks_for(N->n, kTcTile), num_sms() * kTcCtasPerSm));
+    N->dgrid = std::max(1, std::min((int)blocks_for(N->n, kDecTile), num_sms() * 4));
+    const size_t part = (size_t)N->wgrid * (MH * MK + MH);
     pf2_status s;
     if ((s = N->P.alloc(kParams)) || (s = N->grad.alloc(kParams)) || (s = N->am.alloc(kParams)) ||
         (s = N->av.alloc(kParams)) || (s = N->dinv.alloc(n)) || (s = N->feat.alloc(n * MIN)) ||
-        (s = N->y.alloc(n)) || (s = N->dy.alloc(n)) || (s = N->target.alloc(n)) ||
+        (s = N->y.alloc(n)) || (s = N->target.alloc(n)) ||
         (s = N->H.alloc((ML + 1) * n * MH)) || (s = N->M.alloc(ML * n * MH)) || (s = N->dH.alloc(n * MH)) ||
         (s = N->dH2.alloc(n * MH)) || (s = N->dSelf.alloc(n * MH)) || (s = N->dMs.alloc(n * MH)) ||
         (s = N->part.alloc(part)) || (s = N->mask.alloc((ML + 1) * n)) || (s = N->Wb.alloc(ML * MH * MK)) ||
-        (s = N->loss_part.alloc(blocks_for(N->n))) || (s = N->err.alloc(1)))
+        (s = N->loss_part.alloc(N->dgrid)) ||
+        (s = N->dpart.alloc((size_t)N->dgrid * (MH + 1))) || (s = N->err.alloc(1)))
         return fail(s);
     if (const char* e = getenv("PF2_MPNN_MMA")) N->tc = strcmp(e, "sync") != 0;
     if (cudaMemset(N->err.p, 0, sizeof(int)) != cudaSuccess ||
@@ -889,7 +1072,7 @@ pf2_status pf2_mpnn_create(const pf2_mesh* mesh, unsigned long long seed, pf2_mp
         cudaFuncSetAttribute((void*)k_mpnn_layer_back_nodes_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kTcBnSmem) != cudaSuccess ||
         cudaFuncSetAttribute((void*)k_mpnn_layer_back_weights_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kTcSmem) != cudaSuccess)
+                             kTcBwSmem) != cudaSuccess)
         return fail(cuda_fail(cudaGetLastError(), "mpnn set-up", __FILE__, __LINE__));
     // He-style initialisation from a splitmix64 stream (deterministic for a seed);
     // the output layer starts at zero so the untrained guess is the extrapolation alone
@@ -966,9 +1149,7 @@ pf2_status pf2_mpnn_forward(pf2_mpnn* N, const float* feat_dev, float* y_dev, vo
     cudaStream_t st = as_stream(stream);
     PF2_CUDA(cudaMemcpyAsync(N->feat.p, feat_dev, sizeof(float) * MIN * (size_t)N->n, cudaMemcpyDeviceToDevice, st));
     PF2_TRY(mpnn_forward(N, st));
-    k_mpnn_decoder<<<blocks_for(N->n), kThreads, 0, st>>>(N->n, N->Hl(ML), N->P.p, y_dev, nullptr, nullptr, nullptr);
-    PF2_LAUNCH_CHECK();
-    return PF2_OK;
+    return mpnn_decoder(N, y_dev, nullptr, st);
 }
 
 pf2_status pf2_mpnn_train_step(pf2_mpnn* N, const float* feat_dev, const float* target_dev, float lr, int apply,
@@ -978,9 +1159,7 @@ pf2_status pf2_mpnn_train_step(pf2_mpnn* N, const float* feat_dev, const float* 
     PF2_CUDA(cudaMemcpyAsync(N->feat.p, feat_dev, sizeof(float) * MIN * (size_t)N->n, cudaMemcpyDeviceToDevice, st));
     PF2_CUDA(cudaMemcpyAsync(N->target.p, target_dev, sizeof(float) * (size_t)N->n, cudaMemcpyDeviceToDevice, st));
     PF2_TRY(mpnn_forward(N, st));
-    k_mpnn_decoder<<<blocks_for(N->n), kThreads, 0, st>>>(N->n, N->Hl(ML), N->P.p, N->y.p, N->target.p, N->dy.p,
-                                                         N->loss_part.p);
-    PF2_LAUNCH_CHECK();
+    PF2_TRY(mpnn_decoder(N, N->y.p, N->target.p, st));
     PF2_TRY(mpnn_backward(N, st));
     if (apply) {
         ++N->step;
@@ -993,7 +1172,7 @@ pf2_status pf2_mpnn_train_step(pf2_mpnn* N, const float* feat_dev, const float* 
         PF2_LAUNCH_CHECK();
     }
     if (loss_host) {
-        std::vector<double> lp(blocks_for(N->n));
+        std::vector<double> lp(N->dgrid);
         PF2_CUDA(cudaMemcpyAsync(lp.data(), N->loss_part.p, sizeof(double) * lp.size(), cudaMemcpyDeviceToHost, st));
         PF2_CUDA(cudaStreamSynchronize(st));
         double s = 0.0;
