@@ -2075,6 +2075,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_pcg_part_mixed(KArgs a) {
 }  // namespace pf2
 
 #include "part_halo.cuh"
+#include "level_sweep.cuh"
 
 namespace pf2 {
 
@@ -2855,6 +2856,13 @@ struct pf2_solver {
     DevBuf<unsigned char> h_pub, h_item;
     DevBuf<unsigned long long> h_gq, h_gt;  // packets of the exchanges
     DevBuf<double> h_diag;
+    // CG with level sweeps in one block (k_pcg_level): streams, units and what their values are
+    bool level = false;
+    int level_blocks = 0, level_units[2] = { 0, 0 };
+    DevBuf<unsigned char> level_stream[2];
+    DevBuf<int4> level_unit[2], level_src[2];  // src: double of the stream, factor position, pivot position (-1 = none)
+    DevBuf<int> level_slot;
+    DevBuf<double> level_rf, level_tb;
     bool factored = false;
     const pf2_csr* last = nullptr;  // matrix of the last setup / solve
 };
@@ -3470,6 +3478,112 @@ static void* part_kernel(const pf2_solver* S) {
     return (void*)k_pcg_part<0>;
 }
 
+// The streams and units of k_pcg_level (level_sweep.cuh).  level[dir], order[dir]: level and level
+// order of B's rows; deps(dir, row, f): f(dependency, factor position).
+template <class Deps>
+static pf2_status build_level_plan(pf2_solver* S, const std::vector<int> (&level)[2], const std::vector<int> (&order)[2],
+                                   const std::vector<int>& bdiag, const std::vector<int>& perm, bool ic, Deps&& deps) {
+    const int n = S->n;
+    std::vector<std::vector<int>> units[2];  // rows
+    std::vector<int> unit_of[2], slot[2], first[2];
+    int slots[2];
+    for (int dir = 0; dir < 2; ++dir) {
+        unit_of[dir].assign(n, -1);
+        slot[dir].assign(n, -1);
+        int next = 0;
+        std::vector<std::vector<int>>& U = units[dir];
+        auto add = [&](const std::vector<int>& r) {
+            first[dir].push_back(next);
+            for (size_t q = 0; q < r.size(); ++q) {
+                unit_of[dir][r[q]] = (int)U.size();
+                slot[dir][r[q]] = next + (int)q;
+            }
+            next += ((int)r.size() + 31) / 32 * 32;
+            U.push_back(r);
+        };
+        const std::vector<int>& o = order[dir];
+        for (int i0 = 0; i0 < n;) {
+            int i1 = i0;
+            while (i1 < n && level[dir][o[i1]] == level[dir][o[i0]]) ++i1;
+            // rows with more late dependencies than registers come a unit later
+            std::vector<int> part[2];
+            const int last = (int)U.size() - 1;
+            for (int q = i0; q < i1; ++q) {
+                int late = 0;
+                deps(dir, o[q], [&](int j, int) { late += unit_of[dir][j] == last; });
+                part[late > kLevelCase].push_back(o[q]);
+            }
+            if (part[0].empty()) add(part[0]);
+            for (const std::vector<int>& r : part)
+                for (size_t q = 0; q < r.size(); q += 32 * kLevelSlices)
+                    add(std::vector<int>(r.begin() + q, r.begin() + std::min(r.size(), q + 32 * kLevelSlices)));
+            i0 = i1;
+        }
+        while (U.size() % kLevelGroups) add({});
+        slots[dir] = next;
+    }
+    for (int dir = 0; dir < 2; ++dir) {
+        std::vector<unsigned char> stream;
+        std::vector<int4> unit, src;
+        std::vector<std::pair<int, int>> list[2][32 * kLevelSlices];  // early, late: dependency, factor position
+        const bool pivot = dir == 1 || ic;
+        for (size_t u = 0; u < units[dir].size(); ++u) {
+            const std::vector<int>& r = units[dir][u];
+            const int at = first[dir][u], ns = ((int)r.size() + 31) / 32;
+            int K[2] = { 0, 0 };
+            for (size_t q = 0; q < r.size(); ++q) {
+                list[0][q].clear();
+                list[1][q].clear();
+                deps(dir, r[q], [&](int j, int k) { list[unit_of[dir][j] == (int)u - 1][q].emplace_back(j, k); });
+                for (int e = 0; e < 2; ++e) K[e] = std::max(K[e], (int)list[e][q].size());
+            }
+            const int sb = level_slice_bytes(K[0] + K[1]);
+            const size_t off = stream.size();
+            if (K[0] > 255 || (off + (size_t)ns * sb) / 8 > 0x7fffffffull) return PF2_OK;  // (no plan)
+            stream.resize(off + (size_t)ns * sb, 0);
+            int flags = 0;
+            for (int q = 0; q < 32 * ns; ++q) {
+                const size_t base = off + (size_t)(q / 32) * sb, v0 = base / 8 + q % 32;
+                int* word = reinterpret_cast<int*>(stream.data() + base) + q % 32;
+                const bool real = q < (int)r.size();
+                word[64] = (at + q) % kLevelRing * 8;
+                word[96] = !real ? -1 : dir == 0 ? slot[1][r[q]] : perm[r[q]];
+                if (!real) continue;
+                const int dpos = pivot ? bdiag[r[q]] : -1;
+                if (pivot) src.push_back(make_int4((int)v0, -1, dpos, 0));
+                for (int e = 0; e < 2; ++e)
+                    for (size_t k = 0; k < list[e][q].size(); ++k) {
+                        const int j = list[e][q][k].first, c = (e ? K[0] : 0) + (int)k;
+                        // the ring holds it until the row's unit is solved; else where the sweep writes it
+                        const bool near = slot[dir][j] >= at + 32 * ns - kLevelRing;
+                        word[192 + 96 * c] = near ? slot[dir][j] % kLevelRing * 8 : ~(dir == 0 ? slot[1][j] : perm[j]);
+                        if (!near) flags = kLevelFar;
+                        src.push_back(make_int4((int)(v0 + 64 + 48 * c), list[e][q][k].second, e ? dpos : -1, 0));
+                    }
+            }
+            unit.push_back(make_int4((int)(off / 16), K[0] | K[1] << 8 | ns << 16 | flags, at, 0));
+        }
+        if (src.empty()) src.push_back(make_int4(0, -1, -1, 0));  // (an inverse pivot that no row reads)
+        S->level_units[dir] = (int)unit.size();
+        PF2_TRY(S->level_stream[dir].alloc(stream.size()));
+        PF2_CUDA(cudaMemcpy(S->level_stream[dir].p, stream.data(), stream.size(), cudaMemcpyHostToDevice));
+        PF2_TRY(S->level_unit[dir].alloc(unit.size()));
+        PF2_CUDA(cudaMemcpy(S->level_unit[dir].p, unit.data(), sizeof(int4) * unit.size(), cudaMemcpyHostToDevice));
+        PF2_TRY(S->level_src[dir].alloc(src.size()));
+        PF2_CUDA(cudaMemcpy(S->level_src[dir].p, src.data(), sizeof(int4) * src.size(), cudaMemcpyHostToDevice));
+    }
+    std::vector<int> slot_a(n);  // by A's rows
+    for (int i = 0; i < n; ++i) slot_a[perm[i]] = slot[0][i];
+    PF2_TRY(S->level_slot.alloc(n));
+    PF2_CUDA(cudaMemcpy(S->level_slot.p, slot_a.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    PF2_TRY(S->level_rf.alloc(slots[0]));
+    PF2_TRY(S->level_tb.alloc(slots[1]));
+    PF2_CUDA(cudaMemset(S->level_rf.p, 0, S->level_rf.bytes()));
+    PF2_CUDA(cudaMemset(S->level_tb.p, 0, S->level_tb.bytes()));
+    S->level = true;
+    return PF2_OK;
+}
+
 static pf2_status build_tri_plan(pf2_solver* S) {
     const pf2_mesh* M = S->mesh;
     const int n = M->nv, nnz = M->nnz;
@@ -3514,6 +3628,8 @@ static pf2_status build_tri_plan(pf2_solver* S) {
         nl = std::max(nl, l + 1);
     }
     S->levels_fwd = nl;
+    std::vector<int> level[2], level_order[2];
+    level[0] = lev;
     std::vector<int> level_groups[2];
     level_groups[0].assign(nl + 1, 0);
     for (int i = 0; i < n; ++i) level_groups[0][lev[i] + 1]++;
@@ -3523,7 +3639,7 @@ static pf2_status build_tri_plan(pf2_solver* S) {
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return lev[a] < lev[b]; });
     PF2_TRY(S->fwd_order.alloc(n));
     PF2_CUDA(cudaMemcpy(S->fwd_order.p, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    const std::vector<int> fwd_h = order;
+    level_order[0] = order;
     // backward levels: 1 + max over the strictly upper entries (the pattern is symmetric)
     std::fill(lev.begin(), lev.end(), 0);
     nl = 0;
@@ -3534,6 +3650,7 @@ static pf2_status build_tri_plan(pf2_solver* S) {
         nl = std::max(nl, l + 1);
     }
     S->levels_bwd = nl;
+    level[1] = lev;
     level_groups[1].assign(nl + 1, 0);
     for (int i = 0; i < n; ++i) level_groups[1][lev[i] + 1]++;
     for (int l = 0; l < nl; ++l) level_groups[1][l + 1] += level_groups[1][l];
@@ -3541,7 +3658,7 @@ static pf2_status build_tri_plan(pf2_solver* S) {
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return lev[a] < lev[b]; });
     PF2_TRY(S->bwd_order.alloc(n));
     PF2_CUDA(cudaMemcpy(S->bwd_order.p, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    const std::vector<int> bwd_h = order;
+    level_order[1] = order;
     // rows of L^T: for each k, the entries l_ik with i > k as (row i, position in B)
     std::vector<int> off(n + 1, 0);
     for (int i = 0; i < n; ++i)
@@ -3610,6 +3727,27 @@ static pf2_status build_tri_plan(pf2_solver* S) {
     // CG with few levels: the whole iteration on B's CSR arrays (pcg_csr, pcg_csr_mixed)
     S->csr = std::max(S->levels_fwd, S->levels_bwd) < band_min && S->opt.kind == PF2_SOLVER_CG;
     if (const char* e = getenv("PF2_CG_SLOTS")) S->csr = S->csr && atoi(e) == 0;  // tuning: keep the slot sweeps
+    // FP64 CG in the natural order, or on any order with long chains: one block's level sweeps.
+    // us per IC(0) iteration, the banded, slot or ticket solve -> level sweeps:
+    //   triangles   4,355 rows 375 -> 68; 16,705 rows 1,040 -> 152; 36,042 rows 2,181 -> 294;
+    //               125,364 rows 8,927 -> 1,008; 499,288 rows 53,594 -> 4,241
+    //   tetrahedra  1,617 rows 2,109 -> 54; 9,471 rows 3,730 -> 131; 77,531 rows 2,997 -> 684;
+    //               251,991 rows 15,972 -> 2,095
+    // The other CG variants keep their kernels.  PF2_CG_LEVEL=0, or an override of the banded or slot
+    // solve, keeps those (tests and tuning); PF2_CG_LEVEL=2 (tests) requires the level sweeps.
+    const char* le = getenv("PF2_CG_LEVEL");
+    const bool want = le ? atoi(le) != 0 : !getenv("PF2_BAND_ROWS") && !getenv("PF2_BAND_MIN_LEVELS") && !getenv("PF2_CG_SLOTS");
+    if (want && S->opt.kind == PF2_SOLVER_CG && S->opt.precision == PF2_PRECISION_FP64 &&
+        (S->csr ? S->opt.ordering == PF2_ORDERING_NATURAL && S->opt.cg_variant == PF2_CG_STANDARD : banded || K > kBandMaxDeps))
+        PF2_TRY(build_level_plan(S, level, level_order, bdiag, perm, ic, deps));
+    if (le && atoi(le) == 2 && !S->level) {
+        set_error("the level sweeps do not apply");
+        return PF2_BAD_INPUT;
+    }
+    if (S->level) {
+        S->csr = false;
+        S->part_why = "ILU(0) / IC(0) in the natural order";
+    }
     if (S->csr) {
         std::vector<int> tpos(std::max(nnz, 1));
         for (int r = 0; r < n; ++r)
@@ -3653,7 +3791,7 @@ static pf2_status build_tri_plan(pf2_solver* S) {
             srow.reserve(n);
             std::vector<int> loc(n, 0);
             if (!banded) {
-                srow = dir == 0 ? fwd_h : bwd_h;
+                srow = level_order[dir];
                 PF2_TRY(up(H.gstart, level_groups[dir]));
                 H.ngroups = (int)level_groups[dir].size() - 1;
             }
@@ -3787,6 +3925,16 @@ __global__ void k_band_values(long long nk, int n, const int* __restrict__ pos, 
     }
 }
 
+// The streams of k_pcg_level: factor values (late ones scaled by the row's inverse pivot) and
+// inverse pivots.
+__global__ void k_level_values(long long ne, const int4* __restrict__ src, const double* __restrict__ fact,
+                               double* __restrict__ stream) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < ne; k += (long long)gridDim.x * blockDim.x) {
+        const int4 s = src[k];
+        stream[s.x] = (s.y >= 0 ? fact[s.y] : 1.0) * (s.z >= 0 ? 1.0 / fact[s.z] : 1.0);
+    }
+}
+
 // The factors on B's pattern for the CSR sweeps (pf2_solver::tpos).
 __global__ void k_fsym(long long nnz, const int* __restrict__ tpos, const double* __restrict__ fact, double* fsym) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nnz; k += (long long)gridDim.x * blockDim.x) {
@@ -3829,6 +3977,12 @@ static pf2_status factorize(pf2_solver* S, const pf2_csr* A, cudaStream_t st) {
                 nk, S->n, H.pos.p, H.dpos.p, S->fact.p, H.val.p, H.dinv.p, H.val32.p, H.dinv32.p);
             PF2_LAUNCH_CHECK();
         }
+    }
+    for (int d = 0; d < 2 && S->level; ++d) {
+        const long long ne = (long long)S->level_src[d].n;
+        k_level_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(
+            ne, S->level_src[d].p, S->fact.p, reinterpret_cast<double*>(S->level_stream[d].p));
+        PF2_LAUNCH_CHECK();
     }
     if (S->csr) {
         k_fsym<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(S->nnz, S->tpos.p, S->fact.p,
@@ -3987,6 +4141,20 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
                         st);
         return PF2_OK;
     }
+    if (S->level && !precond_only) {
+        LevelCg c{};
+        for (int d = 0; d < 2; ++d)
+            (d ? c.b : c.f) = LevelSweep{ S->level_stream[d].p, S->level_unit[d].p, S->level_units[d] };
+        c.slot_f = S->level_slot.p;
+        c.rf = S->level_rf.p;
+        c.tb = S->level_tb.p;
+        PF2_CUDA(cudaMemsetAsync(S->bar.p, 0, 2 * sizeof(unsigned), st));
+        PF2_CUDA(cudaMemsetAsync(S->err.p, 0, sizeof(int), st));
+        PF2_CUDA(cudaMemsetAsync(S->rec.p, 0, 5 * sizeof(int), st));
+        void* args[] = { &a, &c };
+        PF2_COOP_LAUNCH((void*)k_pcg_level, dim3(S->level_blocks), dim3(kLevelThreads), args, kLevelSmem, st);
+        return PF2_OK;
+    }
     if (S->csr && !precond_only) {  // A's values in B's numbering, for this solve's matrix
         k_gather_values<<<std::min((int)blocks_for(S->nnz), num_sms() * 8), kThreads, 0, st>>>(
             S->nnz, a.A.val, S->bmap.p, S->bval.p);
@@ -4129,6 +4297,11 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
                       "solver kind, variant, precision or preconditioner");
             return fail(PF2_BAD_INPUT);
         }
+    if (S->level) {
+        if (cudaFuncSetAttribute((void*)k_pcg_level, cudaFuncAttributeMaxDynamicSharedMemorySize, kLevelSmem) != cudaSuccess)
+            return fail(cuda_fail(cudaGetLastError(), "level sweep attributes", __FILE__, __LINE__));
+        S->level_blocks = std::max(1, std::min(num_sms(), (S->n + kLevelThreads - 1) / kLevelThreads));
+    }
     // the banded triangular solve keeps a range of the solution in shared memory
     S->smem = S->band_P ? sizeof(double) * (size_t)S->band_R : 0;
     void* fn = solve_kernel(*opt, S->csr);
@@ -4169,7 +4342,7 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
         (opt->kind == PF2_SOLVER_CG && opt->cg_variant == PF2_CG_PIPELINED && (s = S->pipe.alloc(6 * S->n))) ||
         (opt->kind == PF2_SOLVER_BICGSTAB && ((s = S->s.alloc(S->n)) || (s = S->rhat.alloc(S->n)) ||
                                                (s = S->yv.alloc(S->n)) || (s = S->tv.alloc(S->n)))) ||
-        (s = S->invd.alloc(S->n)) || (s = S->partial.alloc(8 * (size_t)std::max(S->blocks, S->part_P))) || (s = S->bar.alloc(2)) ||
+        (s = S->invd.alloc(S->n)) || (s = S->partial.alloc(8 * (size_t)std::max({ S->blocks, S->part_P, S->level_blocks }))) || (s = S->bar.alloc(2)) ||
         (s = S->err.alloc(1)) || (s = S->rec.alloc(5)) || (s = S->out.alloc(1)) || (s = S->h_out.alloc(1)))
         return fail(s);
     if (mixed && ((s = S->val32.alloc(S->nnz)) || (s = S->d32.alloc(S->n)) || (s = S->r32.alloc(S->n)) ||

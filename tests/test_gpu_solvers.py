@@ -592,3 +592,66 @@ def test_halo_cg_matches_the_waiting_sweeps(cuda, monkeypatch, pc, precision, pa
     assert i2.converged == 1 and i3.converged == 1 and i2.status == 0
     assert abs(i2.iterations - i3.iterations) <= (0.1 * i3.iterations + 2 if precision else 2)
     assert rel_err(x2.cpu().numpy(), x3.cpu().numpy()) < (1e-6 if precision else 1e-10)
+
+
+def _odd_mesh(kind):
+    """channel: ordinary levels; box: up to 13 dependencies a row; wide: few levels, of several units; ring: an
+    annulus numbered around, whose last rows depend on ones that have left the sweeps' window of
+    solved values; hub / star: a last row of 30 / 20 neighbours, solved one after the other / in the
+    two levels before."""
+    if kind == "channel":
+        return mg.channel(64, 16, 4.0, 1.0)
+    if kind == "box":
+        return mg.box_tets(9, 7, 5)
+    if kind == "wide":
+        xy, tri = mg.channel(64, 16, 4.0, 1.0)
+        order = np.random.default_rng(3).permutation(len(xy))
+        return np.asarray(xy)[order], np.argsort(order)[np.asarray(tri)].astype(np.int32)
+    if kind == "ring":
+        n = 1500
+        k = np.arange(n)
+        t = 2 * np.pi * k / n
+        xy = np.stack([np.stack([r * np.cos(t), r * np.sin(t)], 1) for r in (1.0, 1.01)], 1).reshape(-1, 2)
+        a, b = 2 * k, 2 * ((k + 1) % n)
+        return xy, np.concatenate([np.stack([a, a + 1, b], 1), np.stack([b, a + 1, b + 1], 1)]).astype(np.int32)
+    n = 30 if kind == "hub" else 20
+    t = 2 * np.pi * np.arange(n) / n
+    xy = np.concatenate([np.stack([np.cos(t), np.sin(t)], 1), np.zeros((1, 2))])
+    # star: every second rim node first, so two levels before the hub's
+    name = np.arange(n) if kind == "hub" else np.arange(n) // 2 + np.arange(n) % 2 * (n // 2)
+    pts = np.empty_like(xy)
+    pts[name], pts[n] = xy[:n], xy[n]
+    nxt = np.roll(name, -1)
+    return pts, np.stack([name, nxt, np.full(n, n)], 1).astype(np.int32)
+
+
+@pytest.mark.parametrize("pc", ["ic", "ilu"])
+@pytest.mark.parametrize("kind", ["channel", "box", "wide", "ring", "hub", "star"])
+def test_level_sweeps_match_the_other_solves(cuda, monkeypatch, kind, pc):
+    """CG in the natural order with one block's level sweeps (PF2_CG_LEVEL=2) against the banded, slot
+    or ticket solve (0).  After 6 iterations only rounding differs: off-diagonal sums within 1/1.05
+    of the diagonal bound the condition of every factor and of the matrix by 41, so the iterates
+    differ by at most some 6 x 20 operations x 41 x 1.1e-16 = 5.4e-13 relative; 1e-11 allowed.  To
+    convergence, the iteration counts agree within one."""
+    xy, cells = _odd_mesh(kind)
+    m = (g.Mesh3D if kind == "box" else g.Mesh2D).from_arrays(xy, cells)
+    A = g.SparseMatrixCSR(m)
+    rp, col, _ = A.download()
+    n = rp.size - 1
+    row = np.repeat(np.arange(n), np.diff(rp))
+    val = np.where(row == col, 0.0, -1.0 - 0.3 * np.cos(row + col.astype(np.float64)))
+    sums = np.zeros(n)
+    np.add.at(sums, row, -val)
+    val[row == col] = 1.05 * sums
+    A.upload_values(val)
+    b = torch.tensor(np.sin(1.0 + np.arange(n)), device="cuda")
+    out = {}
+    for level in ("2", "0"):
+        monkeypatch.setenv("PF2_CG_LEVEL", level)
+        x6, x = torch.zeros_like(b), torch.zeros_like(b)
+        g.LinearSolver(A, "cg", pc, tol=0.0, maxit=6, criterion=g.CRITERION_REL).solve(A, x6, b, check=False)
+        info = g.LinearSolver(A, "cg", pc, tol=1e-9, maxit=500, criterion=g.CRITERION_REL).solve(A, x, b)
+        assert info.converged == 1 and info.status == 0
+        out[level] = (info.iterations, x6.cpu().numpy())
+    assert abs(out["2"][0] - out["0"][0]) <= 1
+    assert rel_err(out["2"][1], out["0"][1]) < 1e-11
