@@ -601,7 +601,6 @@ struct KArgs {
     double* V;      // (m+1) x n
     double* H;      // m x m, column-major
     int m;          // Krylov dimension
-    int gs;         // PF2_GS_MODIFIED or PF2_GS_CLASSICAL_TWICE
     double* vpart;  // (m + 1) x gridDim partial dots (classical Gram-Schmidt)
     double* vtot;   // m + 1 totals
     // mixed precision
@@ -2274,8 +2273,8 @@ __device__ bool grid_reduce_vec(const KArgs& a, double* vals, int K, double* sh)
     return true;
 }
 
-// SolverGMRES::solve (linear_solver.cu:560-660): left-preconditioned GMRES, the
-// projections taken one after another on the updated vector, Givens rotations
+// SolverGMRES::solve (linear_solver.cu:560-660): left-preconditioned GMRES (classical
+// Gram-Schmidt taken twice; modified Gram-Schmidt is k_gmres_mgs), Givens rotations
 // (updateHcolumn :40-66), stop on |beta_k| < tol; x changes only on convergence.  With
 // m < maxit the Krylov space restarts every m iterations.
 __global__ void __launch_bounds__(kSolverThreads, kSolverBlocksPerSm) k_gmres(KArgs a) {
@@ -2332,46 +2331,32 @@ __global__ void __launch_bounds__(kSolverThreads, kSolverBlocksPerSm) k_gmres(KA
             if (global_pc && !grid_sync(a.bar, gridDim.x)) return;
             if (!precond_apply(a, a.q, vkp, r0, r1, apply++, ep_base)) return;
             __syncthreads();
-            if (a.gs == PF2_GS_CLASSICAL_TWICE) {
-                // h = V^T v_{k+1}, v_{k+1} -= V h; a second pass (its h added) unless the
-                // first kept ||v_{k+1}|| above 0.7 of its value (the DGKS test: then one
-                // pass is already orthogonal to working accuracy)
-                for (int pass = 0; pass < 2; ++pass) {
-                    double* hv = pass == 0 ? hcol : h2;
-                    block_dots(a.V, n, k + 1, vkp, r0, r1, hv, pass == 0);
-                    if (!grid_reduce_vec(a, hv, pass == 0 ? k + 2 : k + 1, sh)) return;
-                    for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
-                        double v = vkp[j];
-                        for (int i = 0; i <= k; ++i) v -= hv[i] * a.V[(size_t)i * n + j];
-                        vkp[j] = v;
-                    }
-                    __syncthreads();
-                    if (pass == 0) {
-                        double hh = 0.0;
-                        for (int i = 0; i <= k; ++i) hh += hv[i] * hv[i];
-                        const double ww = hv[k + 1];
-                        if (ww - hh > 0.49 * ww) {  // uniform: every block holds the same totals
-                            for (int i = threadIdx.x; i <= k; i += blockDim.x) h2[i] = 0.0;
-                            __syncthreads();
-                            break;
-                        }
-                    }
+            // h = V^T v_{k+1}, v_{k+1} -= V h; a second pass (its h added) unless the
+            // first kept ||v_{k+1}|| above 0.7 of its value (the DGKS test: then one
+            // pass is already orthogonal to working accuracy)
+            for (int pass = 0; pass < 2; ++pass) {
+                double* hv = pass == 0 ? hcol : h2;
+                block_dots(a.V, n, k + 1, vkp, r0, r1, hv, pass == 0);
+                if (!grid_reduce_vec(a, hv, pass == 0 ? k + 2 : k + 1, sh)) return;
+                for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
+                    double v = vkp[j];
+                    for (int i = 0; i <= k; ++i) v -= hv[i] * a.V[(size_t)i * n + j];
+                    vkp[j] = v;
                 }
-                for (int i = threadIdx.x; i <= k; i += blockDim.x) hcol[i] += h2[i];
                 __syncthreads();
-            } else {
-                // h_ik = v_{k+1} . v_i, then v_{k+1} -= h_ik v_i, i = 0..k (the reference's order)
-                for (int i = 0; i <= k; ++i) {
-                    const double* vi = a.V + (size_t)i * n;
-                    double d[1] = { 0.0 };
-                    for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) d[0] += __ldcg(&vkp[j]) * vi[j];
-                    if (!grid_reduce<1>(a.bar, d, sh)) return;
-                    const double h = d[0];
-                    if (threadIdx.x == 0) hcol[i] = h;
-                    for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) vkp[j] = __ldcg(&vkp[j]) - h * vi[j];
-                    __syncthreads();
+                if (pass == 0) {
+                    double hh = 0.0;
+                    for (int i = 0; i <= k; ++i) hh += hv[i] * hv[i];
+                    const double ww = hv[k + 1];
+                    if (ww - hh > 0.49 * ww) {  // uniform: every block holds the same totals
+                        for (int i = threadIdx.x; i <= k; i += blockDim.x) h2[i] = 0.0;
+                        __syncthreads();
+                        break;
+                    }
                 }
             }
+            for (int i = threadIdx.x; i <= k; i += blockDim.x) hcol[i] += h2[i];
+            __syncthreads();
             double nn[1] = { 0.0 };
             for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
                 const double v = __ldcg(&vkp[j]);
@@ -2430,6 +2415,12 @@ __global__ void __launch_bounds__(kSolverThreads, kSolverBlocksPerSm) k_gmres(KA
         a.out->status = conv ? DEV_OK : DEV_NOT_CONVERGED;
     }
 }
+
+}  // namespace pf2
+
+#include "gmres_mgs.cuh"
+
+namespace pf2 {
 
 // FP32 SpMV row (FP32 products summed in FP32 within the row; values read through L2
 // only where other blocks write them during the kernel).
@@ -2801,7 +2792,8 @@ struct pf2_solver {
     const pf2_mesh* mesh = nullptr;
     int n = 0, nnz = 0, blocks = 0, m = 0;
     long long barrier_polls = 0;  // PF2_BARRIER_POLLS (tests): a grid-barrier wait's poll limit
-    DevBuf<double> r, z, p, q, s, invd, partial, V, H, vpart, rhat, yv, tv;
+    DevBuf<double> r, z, p, q, s, invd, partial, V, H, vpart, rhat, yv, tv, gram;
+    DevBuf<unsigned long long> packets;  // GMRES: k_gmres_mgs
     DevBuf<unsigned> bar;  // count, gen
     DevBuf<int> err;
     DevBuf<int> rec;  // where a device wait gave up (5 ints)
@@ -2819,6 +2811,7 @@ struct pf2_solver {
     BandHost band[2];  // banded solve plan, forward and backward
     int band_P = 0, band_R = 0, band_K = 0;
     size_t smem = 0;  // dynamic shared memory of the solver kernels (banded window)
+    size_t extra_smem = 0;  // and of k_gmres_mgs behind it
     DevBuf<double> outB;
     DevBuf<float> fact32, tmp32, outB32;  // mixed precision with ILU/IC
     // FP64 CG on B (Tri::csr): A's values and the factors on B's pattern, x in B's
@@ -4027,7 +4020,8 @@ static int max_applies(const pf2_solver* S) {
 // no) preconditioner, k_pcg_csr (ILU/IC on B's CSR arrays, either variant) or k_pcg (the
 // standard iteration otherwise).
 static void* solve_kernel(const pf2_solver_options& o, bool csr) {
-    if (o.kind == PF2_SOLVER_GMRES) return (void*)k_gmres;
+    if (o.kind == PF2_SOLVER_GMRES)
+        return o.orthogonalization == PF2_GS_MODIFIED ? (void*)k_gmres_mgs : (void*)k_gmres;
     if (o.kind == PF2_SOLVER_BICGSTAB) return (void*)k_bicgstab;
     if (o.precision == PF2_PRECISION_MIXED) return (void*)k_pcg_mixed;
     const bool tri = o.precond == PF2_PRECOND_ILU || o.precond == PF2_PRECOND_IC;
@@ -4072,7 +4066,6 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     a.V = S->V.p;
     a.H = S->H.p;
     a.m = S->m;
-    a.gs = S->opt.orthogonalization;
     a.vpart = S->vpart.p;
     a.vtot = S->vpart.p ? S->vpart.p + (size_t)(S->m + 1) * S->blocks : nullptr;
     const bool mixed = S->opt.precision == PF2_PRECISION_MIXED && !precond_only;
@@ -4193,7 +4186,11 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     // iteration elsewhere
     if (!mixed && S->opt.kind == PF2_SOLVER_CG && S->opt.cg_variant == PF2_CG_PIPELINED && S->csr)
         fn = pipe_kernel();
-    PF2_COOP_LAUNCH(fn, dim3(S->blocks), dim3(kSolverThreads), args, S->smem, st);
+    GmresMgs gm{ S->gram.p, S->packets.p };
+    void* args_mgs[] = { &a, &gm };
+    if (S->packets.p) PF2_CUDA(cudaMemsetAsync(S->packets.p, 0, S->packets.bytes(), st));  // exchanges count from 1
+    PF2_COOP_LAUNCH(fn, dim3(S->blocks), dim3(kSolverThreads), S->packets.p ? args_mgs : args,
+                    S->smem + S->extra_smem, st);
     if (uses_tri(S)) {
         k_epoch_advance<<<1, 1, 0, st>>>(S->epoch.p, 2 * applies + 2);
         PF2_LAUNCH_CHECK();
@@ -4311,7 +4308,15 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
                                  (int)S->smem) != cudaSuccess)
             return fail(cuda_fail(cudaGetLastError(), "shared-memory attribute", __FILE__, __LINE__));
     }
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kSolverThreads, S->smem) != cudaSuccess || occ < 1)
+    const bool mgs = fn == (void*)k_gmres_mgs;
+    if (mgs) {
+        S->extra_smem = kGramBytes;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * kBandRows + kGramBytes)) != cudaSuccess)
+            return fail(cuda_fail(cudaGetLastError(), "shared-memory attribute", __FILE__, __LINE__));
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kSolverThreads, S->smem + S->extra_smem) != cudaSuccess ||
+        occ < 1)
         return fail(cuda_fail(cudaGetLastError(), "occupancy query", __FILE__, __LINE__));
     int occ_pc = occ;
     if (uses_tri(S) &&
@@ -4335,8 +4340,9 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
         occ = std::min(occ, occ_pp);
     }
     const int maxb = std::min(std::min(occ, occ_pc), bps) * num_sms();
-    // at least ~512 rows per block keeps the barrier count per unit of work low
-    S->blocks = std::max(1, std::min(maxb, (int)((S->n + 511) / 512)));
+    // at least ~512 rows per block keeps the barrier count per unit of work low (GMRES: kGmresRows)
+    const int min_rows = mgs ? kGmresRows : 512;
+    S->blocks = std::max(1, std::min(maxb, (S->n + min_rows - 1) / min_rows));
     if ((s = S->r.alloc(S->n)) || (s = S->z.alloc(S->n)) || (s = S->p.alloc(S->n)) || (s = S->q.alloc(S->n)) ||
         (opt->kind == PF2_SOLVER_CG && (s = S->s.alloc(S->n))) ||
         (opt->kind == PF2_SOLVER_CG && opt->cg_variant == PF2_CG_PIPELINED && (s = S->pipe.alloc(6 * S->n))) ||
@@ -4356,6 +4362,9 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
         if ((s = S->V.alloc((size_t)(m + 1) * S->n)) || (s = S->H.alloc((size_t)m * m))) return fail(s);
         if (opt->orthogonalization == PF2_GS_CLASSICAL_TWICE &&
             (s = S->vpart.alloc((size_t)(m + 1) * (S->blocks + 1))))
+            return fail(s);
+        if (opt->orthogonalization == PF2_GS_MODIFIED &&
+            ((s = S->gram.alloc((size_t)(m + 1) * (m + 1))) || (s = S->packets.alloc(gmres_packet_words(m, S->blocks)))))
             return fail(s);
     }
     if (uses_tri(S)) {

@@ -655,3 +655,31 @@ def test_level_sweeps_match_the_other_solves(cuda, monkeypatch, kind, pc):
         out[level] = (info.iterations, x6.cpu().numpy())
     assert abs(out["2"][0] - out["0"][0]) <= 1
     assert rel_err(out["2"][1], out["0"][1]) < 1e-11
+
+
+@pytest.mark.parametrize("nx,ny,pc,restart", [(12, 4, "none", 0), (48, 12, "jacobi", 0), (64, 24, "none", 0),
+                                              (256, 64, "jacobi", 0), (64, 24, "none", 33), (64, 24, "ilu", 7)])
+def test_gmres_low_synchronisation_follows_modified_gram_schmidt(cuda, nx, ny, pc, restart):
+    """GMRES whose projections share one exchange per iteration (h = (I + L)^{-1} V^T w) against the
+    oracle's one-after-another modified Gram-Schmidt: the coefficients are the same up to
+    rounding, so the iteration counts agree within 2 and both solutions meet ||r|| <= 1e-10, on
+    one block and on many, up to bases of more than 96 vectors (the blocks' own copy of L); with
+    restarts the residual alone is checked.  (A system of condition ~1e4: solutions within 1e-6.)"""
+    m, A, rp, col, val, rhs = _system(nx, ny)
+    b = torch.tensor(rhs, device="cuda")
+    x = torch.zeros_like(b)
+    info = g.LinearSolver(A, "gmres", pc, tol=1e-10, maxit=1000, restart=restart).solve(A, x, b)
+    assert info.converged == 1 and info.status == 0
+    xs = x.cpu().numpy()
+    if restart == 0:
+        ox, oinfo = O.gmres(rp, col, val, rhs, tol=1e-10, maxit=1000, precond=pc)
+        assert abs(info.iterations - oinfo.iterations) <= 2
+        assert rel_err(xs, ox) < 1e-6
+    diag = np.array([val[rp[i] + np.searchsorted(col[rp[i]:rp[i + 1]], i)] for i in range(rp.size - 1)])
+    r = rhs - O.spmv(rp, col, val, xs)
+    if pc == "none":
+        assert np.linalg.norm(r) <= 1.01e-10 + 1e-13 * np.linalg.norm(rhs)
+    elif pc == "jacobi":
+        assert np.linalg.norm(r / diag) <= 1.01e-10 + 1e-13 * np.linalg.norm(rhs / diag)
+    else:
+        assert np.linalg.norm(r) <= 1e-7 * np.linalg.norm(rhs)
