@@ -17,11 +17,11 @@
 // one warp beside that product, whose last one is thrown away.
 //
 // What bounds it: FP64 issue for large systems (3 multiply-adds per entry of V, 64 clocks per warp
-// instruction on a sub-partition: 22,000 of 59,000 clocks an iteration at 125,364 rows and a mean
+// instruction on a sub-partition: 25,000 of 63,000 clocks an iteration at 125,364 rows and a mean
 // basis of 17), the latency of its dependent steps for small ones.  Velocity prediction with
-// Jacobi, one reduction per projection -> this: 125,364 rows, 34 iterations, 4.69 -> 1.05 ms;
+// Jacobi, one reduction per projection -> this: 125,364 rows, 34 iterations, 4.69 -> 1.14 ms;
 // 16,705 rows, 23 iterations, 0.40 ms.  One block per SM (128 registers a thread) against two:
-// 1.14 / 1.49 ms at 125,364 rows, 9.5 / 9.3 at 499,288; 128 rows a block at least against 512:
+// 1.13 / 1.49 ms at 125,364 rows, 9.5 / 9.3 at 499,288 (v_k scaled, not divided); 128 rows a block at least against 512:
 // 0.40 / 0.59 ms at 16,705 rows.  Norms by packets and a fence against grid_reduce: 8,600 against
 // 11,500 clocks.
 #pragma once
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kSolverThreads, 1) k_gmres_mgs(KArgs a, GmresM
             } else {
                 const int skip = k > 0 ? 32 : 0;
                 for (int i = r0 + threadIdx.x - skip; i < r1; i += blockDim.x - skip) {
-                    vk[i] = __ldcg(&raw[i]) * inv;
+                    vk[i] = __ldcg(&raw[i]) / aux;
                     const double v = row_dot(a.A, i, raw) * inv;
                     out[i] = jacobi ? v * a.invd[i] : v;
                 }
