@@ -98,41 +98,62 @@ __device__ __forceinline__ double rhs_f(int kind, double x, double y) {
     return exp(-(x * x + 10 * y * y));
 }
 
-// cases/Poisson2D/main.cu:28-68
+// cases/Poisson2D/main.cu:28-68.  kPoissonLanes lanes per row: they share the row's cells for
+// the right-hand side (f at three points a cell; FP64 sines and exponentials are most of the
+// kernel, and a small mesh has too few rows to hide their chains), added in cell order, and the
+// first lane takes the matrix row.  4,225 nodes: 76 us with a thread per row, 35 now.
+constexpr int kPoissonLanes = 4;
+
 __global__ void k_poisson(int nv, RowMesh M, int kind, double lambda, double* __restrict__ val,
                           double* __restrict__ rhs, BcView bc) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kPoissonLanes;
+    const int sub = threadIdx.x % kPoissonLanes, first = threadIdx.x % 32 - sub;
+    const unsigned group = ((1u << kPoissonLanes) - 1) << first;
     if (i >= nv) return;
     const int s = M.rowptr[i], len = M.rowptr[i + 1] - s;
-    if (boundary_row(i, s, len, M.col, val, rhs, bc)) return;
+    if (bc.node_to_bc && bc.node_to_bc[i] >= 0) {
+        if (sub == 0) boundary_row(i, s, len, M.col, val, rhs, bc);
+        return;
+    }
     // 3-point rule of quadrature_formula_2d.cu:17-24 (z = 1 - x - y as there)
     const double q1 = 0.1666666666666667, q2 = 0.6666666666666667;
     const double QL[3][3] = { { q1, q1, 1.0 - q1 - q1 }, { q2, q1, 1.0 - q2 - q1 }, { q1, q2, 1.0 - q1 - q2 } };
     const double w = 0.3333333333333333;
+    const int q0 = M.inc_off[i], qe = M.inc_off[i + 1];
+    double r = 0.0;
+    for (int base = q0; base < qe; base += kPoissonLanes) {
+        double part = 0.0;
+        const int q = base + sub;
+        if (q < qe) {
+            const int e = M.inc[q], c = e >> 2, m = e & 3;
+            const int4 t = M.tri4[c];
+            const double2 P0 = M.xy[t.x], P1 = M.xy[t.y], P2 = M.xy[t.z];
+            double rr = 0.0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double x = QL[k][0] * P0.x + QL[k][1] * P1.x + QL[k][2] * P2.x;
+                const double y = QL[k][0] * P0.y + QL[k][1] * P1.y + QL[k][2] * P2.y;
+                const double Lm = m == 0 ? QL[k][0] : m == 1 ? QL[k][1] : QL[k][2];
+                rr += rhs_f(kind, x, y) * Lm * w;
+            }
+            part = rr * M.area[c];
+        }
+        for (int u = 0; u < min(kPoissonLanes, qe - base); ++u) r += __shfl_sync(group, part, first + u);
+    }
+    if (sub) return;
     double v[kMaxRow];
     for (int k = 0; k < len; ++k) v[k] = 0.0;
-    double r = 0.0;
-    for (int q = M.inc_off[i]; q < M.inc_off[i + 1]; ++q) {
+    for (int q = q0; q < qe; ++q) {
         const int e = M.inc[q], c = e >> 2, m = e & 3, pos = M.inc_pos[q];
-        const double4_32a J = M.invJ[c];
         const double A = M.area[c];
         double2 g[3];
-        shape_grads(J, g);
-        const int4 t = M.tri4[c];
-        const double2 P0 = M.xy[t.x], P1 = M.xy[t.y], P2 = M.xy[t.z];
+        shape_grads(M.invJ[c], g);
+        const double2 gm = m == 0 ? g[0] : m == 1 ? g[1] : g[2];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const int p = (pos >> (10 * j)) & 1023;
-            v[p] += lambda * (g[m].x * g[j].x + g[m].y * g[j].y) * A;
+            v[p] += lambda * (gm.x * g[j].x + gm.y * g[j].y) * A;
         }
-        double rr = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double x = QL[k][0] * P0.x + QL[k][1] * P1.x + QL[k][2] * P2.x;
-            const double y = QL[k][0] * P0.y + QL[k][1] * P1.y + QL[k][2] * P2.y;
-            rr += rhs_f(kind, x, y) * QL[k][m] * w;
-        }
-        r += rr * A;
     }
     eliminate_row(i, s, len, M.col, v, r, bc);
     for (int k = 0; k < len; ++k) val[s + k] = v[k];
@@ -140,6 +161,49 @@ __global__ void k_poisson(int nv, RowMesh M, int kind, double lambda, double* __
 }
 
 // ------------------------------------------------------------- flow systems
+// A cell as seen from its vertex m: gradients of N_m and of the other two vertices j, k, whose
+// nodes and places in m's row these are.  The gradients add up to zero, so the gradient of a
+// nodal field needs its differences to node m only, and a row's diagonal entry of every
+// gradient term is minus the sum of the others.
+//
+// The kernels below are bound by FP64 issue (64 clocks per warp instruction on an SM
+// sub-partition), and each of a cell's rows computes the cell's terms anew.  So sums over j come
+// first (gradients of u and p once per cell, mass on neighbours as one sum, factors common to a
+// row and diagonals at its end).  499,288 nodes, matrix and right-hand side, FP64 pipe 80 % busy:
+// k_prediction 514 -> 334 us, k_pressure 165 -> 147, k_correction 225 -> 133.  Differences to node m
+// also round less: the pressure of the quarter-size cylinder's first step agrees with the oracle's
+// to 6.5e-13 instead of 2.6e-12.
+struct CellAt {
+    double2 g, gj, gk;
+    int j, k, p, pj, pk;
+    __device__ __forceinline__ double2 grad(double dj, double dk) const {
+        return make_double2(fma(gj.x, dj, gk.x * dk), fma(gj.y, dj, gk.y * dk));
+    }
+};
+__device__ __forceinline__ CellAt cell_at(const double4_32a& J, const int4& t, int m, int pos) {
+    double2 g[3];
+    shape_grads(J, g);
+    const int p0 = pos & 1023, p1 = (pos >> 10) & 1023, p2 = (pos >> 20) & 1023;
+    CellAt C;
+    C.g = m == 0 ? g[0] : m == 1 ? g[1] : g[2];
+    C.gj = m == 0 ? g[1] : m == 1 ? g[2] : g[0];
+    C.gk = m == 0 ? g[2] : m == 1 ? g[0] : g[1];
+    C.j = m == 0 ? t.y : m == 1 ? t.z : t.x;
+    C.k = m == 0 ? t.z : m == 1 ? t.x : t.y;
+    C.p = m == 0 ? p0 : m == 1 ? p1 : p2;
+    C.pj = m == 0 ? p1 : m == 1 ? p2 : p0;
+    C.pk = m == 0 ? p2 : m == 1 ? p0 : p1;
+    return C;
+}
+
+// The sum of a row's other entries.
+__device__ __forceinline__ double others(const double* v, int len, int diag) {
+    double sum = 0.0;
+    for (int k = 0; k < len; ++k)
+        if (k != diag) sum += v[k];
+    return sum;
+}
+
 // `matrix` is a runtime flag, not a template parameter: the matrix values that feed the
 // elimination of a right-hand-side-only assembly then come from the same machine code
 // as a full assembly's, so both give the same bits (separate instantiations may fuse
@@ -164,33 +228,34 @@ __global__ void k_prediction(bool matrix, int nv, RowMesh M, FlowCoef P, const d
     double v0[kMaxRow], v1[kMaxRow];
     if (need)
         for (int k = 0; k < len; ++k) { v0[k] = 0.0; v1[k] = 0.0; }
-    double r0 = 0.0, r1 = 0.0;
-    const double visc = P.mu * P.dt;
-    const double third = 1.0 / 3.0;
+    double r0 = 0.0, r1 = 0.0, mass = 0.0;
+    const double visc = P.mu * P.dt, rho12 = P.rho / 12.0, dt3 = P.dt / 3.0;
+    const double uxi = ux[i], uyi = uy[i], pi = pold ? pold[i] : 0.0;
+    int diag = 0;
     for (int q = M.inc_off[i]; q < M.inc_off[i + 1]; ++q) {
         const int e = M.inc[q], c = e >> 2, m = e & 3, pos = M.inc_pos[q];
         const double A = M.area[c];
-        double2 g[3];
-        shape_grads(M.invJ[c], g);
-        const int4 t = M.tri4[c];
-        double c0 = 0.0, c1 = 0.0;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int nj = vtx(t, j), p = (pos >> (10 * j)) & 1023;
-            const double mass = P.rho * ((j == m) ? (1.0 / 6.0) : (1.0 / 12.0));
-            const double xx = g[m].x * g[j].x, yy = g[m].y * g[j].y;
-            const double xy_ = g[m].y * g[j].x, yx = g[m].x * g[j].y;
-            if (need) {
-                v0[p] += (mass + visc * (yy + 4.0 / 3.0 * xx)) * A;
-                v1[p] += (mass + visc * (xx + 4.0 / 3.0 * yy)) * A;
-            }
-            c0 += mass * uxo[nj] - visc * (xy_ - 2.0 / 3.0 * yx) * uy[nj];
-            c1 += mass * uyo[nj] - visc * (yx - 2.0 / 3.0 * xy_) * ux[nj];
-            if (pold) {
-                const double a = third * pold[nj] * P.dt;
-                c0 -= a * g[j].x;
-                c1 -= a * g[j].y;
-            }
+        const CellAt C = cell_at(M.invJ[c], M.tri4[c], m, pos);
+        diag = C.p;
+        const double Am = rho12 * A, Av = visc * A;
+        const double ax = Av * C.g.x, ay = Av * C.g.y;
+        if (need) {
+            const double ax43 = 4.0 / 3.0 * ax, ay43 = 4.0 / 3.0 * ay;
+            v0[C.pj] += fma(ay, C.gj.y, fma(ax43, C.gj.x, Am));
+            v0[C.pk] += fma(ay, C.gk.y, fma(ax43, C.gk.x, Am));
+            v1[C.pj] += fma(ax, C.gj.x, fma(ay43, C.gj.y, Am));
+            v1[C.pk] += fma(ax, C.gk.x, fma(ay43, C.gk.y, Am));
+        }
+        mass += Am;
+        r0 = fma(Am, uxo[C.j] + uxo[C.k], r0);
+        r1 = fma(Am, uyo[C.j] + uyo[C.k], r1);
+        const double2 dx = C.grad(ux[C.j] - uxi, ux[C.k] - uxi), dy = C.grad(uy[C.j] - uyi, uy[C.k] - uyi);
+        r0 = fma(-ay, dy.x, fma(2.0 / 3.0 * ax, dy.y, r0));
+        r1 = fma(-ax, dx.y, fma(2.0 / 3.0 * ay, dx.x, r1));
+        if (pold) {
+            const double2 d = C.grad(pold[C.j] - pi, pold[C.k] - pi);
+            r0 = fma(-(dt3 * A), d.x, r0);
+            r1 = fma(-(dt3 * A), d.y, r1);
         }
         // outlet edges (id 1) that contain local vertex m
         const int e0 = M.edge_ids[3 * c], e1 = M.edge_ids[3 * c + 1], e2 = M.edge_ids[3 * c + 2];
@@ -199,23 +264,33 @@ __global__ void k_prediction(bool matrix, int nv, RowMesh M, FlowCoef P, const d
         for (int ed = 0; ed < 3; ++ed) {
             if (ids[ed] != 1) continue;
             if (m != ed && m != (ed + 1) % 3) continue;
+            const int4 t = M.tri4[c];
+            double2 g[3];
+            shape_grads(M.invJ[c], g);
             const double2 S = M.xy[vtx(t, ed)], E = M.xy[vtx(t, (ed + 1) % 3)];
             const double half = 0.5 * sqrt((S.x - E.x) * (S.x - E.x) + (S.y - E.y) * (S.y - E.y));
             const double w = visc * half;
             const double nx = 1.0, ny = 0.0;
+            double c0 = 0.0, c1 = 0.0;
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 const int nj = vtx(t, j), p = (pos >> (10 * j)) & 1023;
-                if (need) {
+                if (need && j != m) {
                     v0[p] -= w * ((4.0 / 3.0) * g[j].x * nx + g[j].y * ny) * A;
                     v1[p] -= w * (g[j].x * nx + (4.0 / 3.0) * g[j].y * ny) * A;
                 }
                 c0 += w * uy[nj] * ((-2.0 / 3.0) * g[j].y * nx + g[j].x * ny);
                 c1 += w * ux[nj] * (g[j].y * nx + (-2.0 / 3.0) * g[j].x * ny);
             }
+            r0 += c0 * A;
+            r1 += c1 * A;
         }
-        r0 += c0 * A;
-        r1 += c1 * A;
+    }
+    r0 = fma(2.0 * mass, uxo[i], r0);
+    r1 = fma(2.0 * mass, uyo[i], r1);
+    if (need) {
+        v0[diag] = 4.0 * mass - others(v0, len, diag);
+        v1[diag] = 4.0 * mass - others(v1, len, diag);
     }
     if (!bx) {
         if (need) eliminate_row(i, s, len, M.col, v0, r0, bcx);
@@ -239,28 +314,34 @@ __global__ void k_pressure(bool matrix, int nv, RowMesh M, FlowCoef P, const dou
     if (i >= nv) return;
     const int s = M.rowptr[i], len = M.rowptr[i + 1] - s;
     if (boundary_row(i, s, len, M.col, val, rhs, bc, matrix)) return;
-    const bool need = matrix || has_bc_column(i, s, len, M.col, bc);
+    const bool need = matrix || has_bc_column(i, s, len, M.col, bc), entries = need || pold;
     double v[kMaxRow];
-    if (need)
+    if (entries)
         for (int k = 0; k < len; ++k) v[k] = 0.0;
     double r = 0.0;
-    const double fdiv = -P.rho / P.dt / 3.0;
+    const double pxi = px[i], pyi = py[i];
+    int diag = 0;
     for (int q = M.inc_off[i]; q < M.inc_off[i + 1]; ++q) {
         const int e = M.inc[q], c = e >> 2, m = e & 3, pos = M.inc_pos[q];
         const double A = M.area[c];
-        double2 g[3];
-        shape_grads(M.invJ[c], g);
-        const int4 t = M.tri4[c];
-        double cr = 0.0, div = 0.0;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int nj = vtx(t, j), p = (pos >> (10 * j)) & 1023;
-            const double K = g[m].x * g[j].x + g[m].y * g[j].y;
-            if (need) v[p] += K * A;
-            if (pold) cr += K * pold[nj];
-            div += g[j].x * px[nj] + g[j].y * py[nj];
+        const CellAt C = cell_at(M.invJ[c], M.tri4[c], m, pos);
+        diag = C.p;
+        if (entries) {
+            const double ax = A * C.g.x, ay = A * C.g.y;
+            v[C.pj] = fma(ax, C.gj.x, fma(ay, C.gj.y, v[C.pj]));
+            v[C.pk] = fma(ax, C.gk.x, fma(ay, C.gk.y, v[C.pk]));
         }
-        r += (cr + fdiv * div) * A;
+        const double div = fma(C.gj.x, px[C.j] - pxi, fma(C.gk.x, px[C.k] - pxi,
+                           fma(C.gj.y, py[C.j] - pyi, C.gk.y * (py[C.k] - pyi))));
+        r = fma(A, div, r);
+    }
+    r *= -P.rho / P.dt / 3.0;
+    if (entries) {
+        v[diag] = -others(v, len, diag);
+        if (pold) {
+            const double pi = pold[i];
+            for (int k = 0; k < len; ++k) r = fma(v[k], pold[M.col[s + k]] - pi, r);
+        }
     }
     if (need) eliminate_row(i, s, len, M.col, v, r, bc);
     if (matrix)
@@ -281,28 +362,30 @@ __global__ void k_correction(bool matrix, int nv, RowMesh M, FlowCoef P, const d
     if (bx && by) return;
     const bool need = matrix || has_bc_column(i, s, len, M.col, bcx) || has_bc_column(i, s, len, M.col, bcy);
     double v[kMaxRow];
-    if (need)
-        for (int k = 0; k < len; ++k) v[k] = 0.0;
+    for (int k = 0; k < len; ++k) v[k] = 0.0;
     double r0 = 0.0, r1 = 0.0;
-    const double gdt = P.dt / 3.0;
+    const double dpi = pold ? pres[i] - pold[i] : pres[i];
+    int diag = 0;
     for (int q = M.inc_off[i]; q < M.inc_off[i + 1]; ++q) {
         const int e = M.inc[q], c = e >> 2, m = e & 3, pos = M.inc_pos[q];
         const double A = M.area[c];
-        double2 g[3];
-        shape_grads(M.invJ[c], g);
-        const int4 t = M.tri4[c];
-        double c0 = 0.0, c1 = 0.0;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int nj = vtx(t, j), p = (pos >> (10 * j)) & 1023;
-            const double mass = P.rho * ((j == m) ? (1.0 / 6.0) : (1.0 / 12.0));
-            if (need) v[p] += mass * A;
-            const double dp = pold ? (pres[nj] - pold[nj]) : pres[nj];
-            c0 += mass * px[nj] - gdt * g[j].x * dp;
-            c1 += mass * py[nj] - gdt * g[j].y * dp;
-        }
-        r0 += c0 * A;
-        r1 += c1 * A;
+        const CellAt C = cell_at(M.invJ[c], M.tri4[c], m, pos);
+        diag = C.p;
+        v[C.pj] += A;
+        v[C.pk] += A;
+        const double dpj = pold ? pres[C.j] - pold[C.j] : pres[C.j], dpk = pold ? pres[C.k] - pold[C.k] : pres[C.k];
+        const double2 d = C.grad(dpj - dpi, dpk - dpi);
+        r0 = fma(A, d.x, r0);
+        r1 = fma(A, d.y, r1);
+    }
+    r0 *= -P.dt / 3.0;
+    r1 *= -P.dt / 3.0;
+    v[diag] = others(v, len, diag);  // each cell's area once for j and once for k
+    for (int k = 0; k < len; ++k) {
+        const int j = M.col[s + k];
+        v[k] *= P.rho / 12.0;
+        r0 = fma(v[k], px[j], r0);
+        r1 = fma(v[k], py[j], r1);
     }
     double w[kMaxRow];
     if (need)
@@ -546,7 +629,7 @@ pf2_status pf2_assemble_poisson(const pf2_mesh* m, pf2_csr* A, double* rhs, int 
     PF2_TRY(check_csr(m, A));
     PF2_TRY(check_bc(m, bc));
     PF2_REQUIRE(rhs, PF2_BAD_INPUT, "null rhs");
-    k_poisson<<<blocks_for(m->nv), kThreads, 0, as_stream(stream)>>>(m->nv, row_mesh(m), kind, lambda, A->val.p, rhs,
+    k_poisson<<<blocks_for((long long)m->nv * kPoissonLanes), kThreads, 0, as_stream(stream)>>>(m->nv, row_mesh(m), kind, lambda, A->val.p, rhs,
                                                                       bc_view(bc));
     PF2_LAUNCH_CHECK();
     return PF2_OK;

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import gpupfem2_gb300 as g
+from gpupfem2_gb300 import meshgen as mg
 from oracle import oracle as O
 from tests.helpers import poisson_square, rel_err
 
@@ -86,3 +87,33 @@ def test_not_converged_is_reported(cuda):
     x = torch.zeros(m.nv, dtype=torch.float64, device="cuda")
     info = g.LinearSolver(A, "cg", "jacobi", tol=1e-12, maxit=3).solve(A, x, rhs)
     assert info.converged == 0 and info.iterations == 3
+
+
+@pytest.mark.parametrize("dims", [(1, 1), (2, 1), (3, 5), (9, 4), (1, 1, 1), (2, 3, 1), (5, 4, 3)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_assembly_on_the_smallest_meshes(cuda, dims, kind):
+    """Rows shared by a few lanes: last warps and blocks that are partly filled, rows of fewer cells than
+    lanes, boundary rows beside inner ones.  A row sums at most ~40 cells' terms of ~30 roundings
+    each: 1200 x 1.1e-16 = 1.3e-13 of the largest entry; 1e-12 as above."""
+    if len(dims) == 2:
+        xy, tri = mg.channel(dims[0], dims[1])
+        m = g.Mesh2D.from_arrays(xy, tri)
+        area, invJ = O.mesh_geometry(xy, tri)
+        rp, col = O.csr_structure(xy.shape[0], tri)
+        val, orhs = O.assemble_poisson(xy, tri, area, invJ, rp, col, kind, 0.7)
+        assemble = g.assemble_poisson
+    else:
+        xy, tet = mg.box_tets(*dims)
+        m = g.Mesh3D.from_arrays(xy, tet)
+        vol, invJ = O.mesh3d_geometry(xy, tet)
+        rp, col = O.csr_structure_3d(xy.shape[0], tet)
+        val, orhs = O.assemble_poisson_3d(xy, tet, vol, invJ, rp, col, kind, 0.7)
+        assemble = g.assemble_poisson_3d
+    A = g.SparseMatrixCSR(m)
+    rhs = torch.full((m.nv,), 7.0, dtype=torch.float64, device="cuda")
+    assemble(m, A, rhs, kind, 0.7)
+    assert rel_err(A.download()[2], val) < ASM_TOL and rel_err(rhs.cpu().numpy(), orhs) < ASM_TOL
+    bcs = [(i, 0.1 * i - 0.3) for i in range(0, m.nv, 3)]
+    val, orhs = O.apply_bcs(rp, col, val, orhs, np.array([b for b, _ in bcs], np.int32), np.array([v for _, v in bcs]))
+    assemble(m, A, rhs, kind, 0.7, g.DirichletBCs(m.nv, bcs))
+    assert rel_err(A.download()[2], val) < ASM_TOL and rel_err(rhs.cpu().numpy(), orhs) < ASM_TOL
