@@ -58,6 +58,20 @@ __global__ void k_seed(int nc, int ppc, Centers C, const double2* __restrict__ x
     if (g == 0) seg[nc] = nc * ppc;
 }
 
+// determine_subcell by FP32 where that is certain: the coordinates are within 2e-6 of [0, 1], so
+// each of the three FP32 values below is within 2e-6 of what the FP64 rule compares or truncates,
+// and one farther than 1e-5 from the nearest integer or bound decides alike.  (14 FP64
+// instructions, 64 clocks each, otherwise.)
+__device__ __forceinline__ int subcell_of(int n, double step, double l0, double l1, double l2) {
+    const float fn = (float)n, a = (1.0f - (float)l1) * fn, b = (float)l0 * fn;
+    const int i = (int)a, j = (int)b;
+    const float d = ((float)l2 * fn - (float)(i - j));
+    const float g = 1e-5f;
+    const bool sure = fabsf(a - rintf(a)) > g && fabsf(b - rintf(b)) > g && (i == j || fabsf(d) > g);
+    if (!sure) return determine_subcell(n, step, l0, l1, l2);
+    return i * i + 2 * j + (i != j && d < 0.0f ? 1 : 0);
+}
+
 struct MeshRefs {
     const int4* tri;
     const double4_32a* invJ;
@@ -226,7 +240,7 @@ __global__ void __launch_bounds__(256) k_advect(const int* __restrict__ np_ptr, 
                 // a located particle loses its centroid flag; with no substeps it keeps it
                 P.cw[p] = substeps > 0 ? c : cw;
                 key = c;
-                sub = determine_subcell(level, step, l0, l1, l2);
+                sub = subcell_of(level, step, l0, l1, l2);
             }
         }
         // one atomic per (warp, cell); each lane's rank = group base + lanes below it
@@ -309,21 +323,29 @@ struct PartialStage {
     int bs[8], bn[8];
 };
 
-__device__ __forceinline__ void block_partials(PartialStage& G, int c0, int nc, PState S, const Centers& C,
-                                               Partials part) {
-    const int t = threadIdx.x;
-    __syncthreads();  // bs, bn and the block's slots are in place
-    const int S0 = G.bs[0];
-    int total = 0;
+
+// Whether the block's cells (bs, bn) can be staged, and how many slots they hold.
+__device__ __forceinline__ bool stage_fits(const PartialStage& G, int c0, int nc, int& total) {
     bool contiguous = true;
+    total = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         if (c0 + i >= nc) break;
-        if (G.bn[i] < 0 || G.bs[i] != S0 + total) contiguous = false;
+        if (G.bn[i] < 0 || G.bs[i] != G.bs[0] + total) contiguous = false;
         total += max(G.bn[i], 0);
     }
-    const bool staged = contiguous && total <= kStageSlots;  // uniform over the block
-    if (staged) {
+    return contiguous && total <= kStageSlots;
+}
+
+// filled: the caller has written the stage of a block that stage_fits.
+__device__ __forceinline__ void block_partials(PartialStage& G, int c0, int nc, PState S, const Centers& C,
+                                               Partials part, bool filled = false) {
+    const int t = threadIdx.x;
+    __syncthreads();  // bs, bn and the block's slots are in place
+    const int S0 = G.bs[0];
+    int total;
+    const bool staged = stage_fits(G, c0, nc, total);  // uniform over the block
+    if (staged && !filled) {
         for (int k = t; k < total; k += blockDim.x) {
             const int o = S0 + k;
             const int w = S.cw[o];
@@ -335,7 +357,7 @@ __device__ __forceinline__ void block_partials(PartialStage& G, int c0, int nc, 
             G.v[k] = S.v[o];
         }
     }
-    __syncthreads();
+    if (!filled) __syncthreads();
     // thread t: coordinate a (grouped so that the L2 threads of the unstaged path share
     // warps), cell i, factor j (u, v, 1), third q
     const int a = t / 72, rem = t % 72, i = rem / 9, j = (rem % 9) / 3, q = rem % 3;
@@ -371,9 +393,15 @@ __device__ __forceinline__ void block_partials(PartialStage& G, int c0, int nc, 
 // Per cell, one warp: stable order, move, reseed (kAddParticlesToCell :197-236); then the
 // block's partial sums.  The cell's particles arrive in perm[s, s + n) in the order the
 // atomics handed out ranks; each lane ranks its particle by old index against all n (the
-// old order is the order the cell keeps), moves it to slot s + rank, then lanes fill the
-// missing sub-cells after them.  The partial sums are formed over the slots after the
+// old order is the order the cell keeps) and moves it to slot s + rank; the missing
+// sub-cells follow them.  The partial sums are formed over the slots after the
 // moves, so they do not depend on the atomics' order.
+//
+// What bounds it: the chain of dependent loads (segment, order, particle), and FP64 issue in the
+// reseeds and sums.  A warp's particles go to the stage of the sums as they are moved, without a
+// second trip through L2, and the block's reseeds (a few per cell) are made together, so that
+// their FP64 instructions serve full warps.  17.6 million particles: 2,340 us with the reseeds
+// per warp and the stage read back -> GATHER_NEW us.
 __global__ void __launch_bounds__(256, 5) k_gather(int nc, const int* __restrict__ seg, int* count, int* mask,
                                                 const int* __restrict__ perm, PState S, PState D, Centers C,
                                                 int level, int reseed, const double2* __restrict__ xy,
@@ -381,6 +409,9 @@ __global__ void __launch_bounds__(256, 5) k_gather(int nc, const int* __restrict
                                                 const double* __restrict__ uy, Partials part, long long cap,
                                                 int* cnt) {
     __shared__ PartialStage G;
+    __shared__ int add[8];          // the cells' missing sub-cells: their number,
+    __shared__ unsigned gone[8];    // which, and the slot of the first one
+    __shared__ int add_at[8];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     const int c0 = blockIdx.x * 8;
     const int c = c0 + wi;
@@ -405,51 +436,82 @@ __global__ void __launch_bounds__(256, 5) k_gather(int nc, const int* __restrict
     if (lane == 0) {
         G.bs[wi] = s;
         G.bn[wi] = fits ? n + nadd : -1;
+        add[wi] = fits ? nadd : 0;
+        gone[wi] = ~m & ((1u << ppc) - 1u);
+        add_at[wi] = s + n;
     }
+    __syncthreads();
+    int total;
+    const bool staged = stage_fits(G, c0, nc, total);
+    const int S0 = G.bs[0];
+    auto stage = [&](int o, int w, double l0, double l1, double u, double v) {
+        const int k = o - S0;
+        G.l[0][k] = l0;
+        G.l[1][k] = l1;
+        G.l[2][k] = third_coord(w, l0, l1, C);
+        G.u[k] = u;
+        G.v[k] = v;
+    };
     if (fits) {
         // existing particles: lane handles entries base + lane of perm[s, s + n)
         for (int base = 0; base < n; base += 32) {
             const int i = base + lane;
             const int v = i < n ? perm[s + i] : 0x7fffffff;
+            const bool mine = i < n;
+            double px, py, pl0, pl1, pu, pv;
+            int pw;
+            if (mine) {  // (on their way while the warp ranks)
+                px = S.x[v];
+                py = S.y[v];
+                pl0 = S.l0[v];
+                pl1 = S.l1[v];
+                pu = S.u[v];
+                pv = S.v[v];
+                pw = S.cw[v];
+            }
             int r = 0;
             for (int cb = 0; cb < n; cb += 32) {
-                const int w = cb + lane < n ? perm[s + cb + lane] : 0x7fffffff;
+                const int w = cb == base ? v : cb + lane < n ? perm[s + cb + lane] : 0x7fffffff;
                 const int lim = min(32, n - cb);
                 for (int j = 0; j < lim; ++j) r += (__shfl_sync(0xffffffffu, w, j) < v) ? 1 : 0;
             }
-            if (i < n) {
+            if (mine) {
                 const int o = s + r;
-                D.x[o] = S.x[v];
-                D.y[o] = S.y[v];
-                D.l0[o] = S.l0[v];
-                D.l1[o] = S.l1[v];
-                D.u[o] = S.u[v];
-                D.v[o] = S.v[v];
-                D.cw[o] = S.cw[v];
-            }
-        }
-        // reseed: the q-th missing sub-cell goes to slot s + n + q
-        if (nadd) {
-            const int4 t = tri[c];
-            const double2 A = xy[t.x], B = xy[t.y], E = xy[t.z];
-            const double u0 = ux[t.x], u1 = ux[t.y], u2 = ux[t.z];
-            const double w0 = uy[t.x], w1 = uy[t.y], w2 = uy[t.z];
-            const unsigned missing = ~m & ((1u << ppc) - 1u);
-            for (int q = lane; q < nadd; q += 32) {
-                const int k = (int)__fns(missing, 0, q + 1);
-                const int o = s + n + q;
-                const double L0 = C.c[k][0], L1 = C.c[k][1], L2 = C.c[k][2];
-                D.x[o] = local_to_global(L0, L1, L2, A.x, B.x, E.x);
-                D.y[o] = local_to_global(L0, L1, L2, A.y, B.y, E.y);
-                D.l0[o] = L0;
-                D.l1[o] = L1;
-                D.u[o] = interp3(L0, L1, L2, u0, u1, u2);
-                D.v[o] = interp3(L0, L1, L2, w0, w1, w2);
-                D.cw[o] = c | ((k + 1) << kCellBits);
+                D.x[o] = px;
+                D.y[o] = py;
+                D.l0[o] = pl0;
+                D.l1[o] = pl1;
+                D.u[o] = pu;
+                D.v[o] = pv;
+                D.cw[o] = pw;
+                if (staged) stage(o, pw, pl0, pl1, pu, pv);
             }
         }
     }
-    block_partials(G, c0, nc, D, C, part);
+    // reseed: the q-th missing sub-cell of a cell goes to the q-th slot after its particles
+    int adds = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) adds += add[i];
+    for (int t = threadIdx.x; t < adds; t += blockDim.x) {
+        int i = 0, q = t;
+        while (q >= add[i]) q -= add[i++];
+        const int4 v = tri[c0 + i];
+        const double2 A = xy[v.x], B = xy[v.y], E = xy[v.z];
+        const int k = (int)__fns(gone[i], 0, q + 1);
+        const int o = add_at[i] + q;
+        const double L0 = C.c[k][0], L1 = C.c[k][1], L2 = C.c[k][2];
+        const double u = interp3(L0, L1, L2, ux[v.x], ux[v.y], ux[v.z]), w = interp3(L0, L1, L2, uy[v.x], uy[v.y], uy[v.z]);
+        const int cw = (c0 + i) | ((k + 1) << kCellBits);
+        D.x[o] = local_to_global(L0, L1, L2, A.x, B.x, E.x);
+        D.y[o] = local_to_global(L0, L1, L2, A.y, B.y, E.y);
+        D.l0[o] = L0;
+        D.l1[o] = L1;
+        D.u[o] = u;
+        D.v[o] = w;
+        D.cw[o] = cw;
+        if (staged) stage(o, cw, L0, L1, u, w);
+    }
+    block_partials(G, c0, nc, D, C, part, staged);
 }
 
 // Partial sums of every cell from the current (cell-ordered) particles, eight cells per
@@ -487,24 +549,29 @@ __global__ void k_project_nodes(int nv, const int* __restrict__ inc_off, const i
     if (uxo) { uxo[i] = a; uyo[i] = b; }
 }
 
-// kCorrectParticleVelocity (:72-88); old == nullptr gives initParticleVelocity.
+// The change of the grid velocity, once per node for k_correct (a particle's cell has three nodes,
+// a node ~35 particles).
+__global__ void k_node_change(int nv, const double* __restrict__ ux, const double* __restrict__ uy,
+                              const double* __restrict__ uxo, const double* __restrict__ uyo, double* dx, double* dy) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nv) return;
+    dx[i] = __dsub_rn(ux[i], uxo[i]);
+    dy[i] = __dsub_rn(uy[i], uyo[i]);
+}
+
+// kCorrectParticleVelocity (:72-88) with the nodes' change of velocity; with the velocity itself
+// initParticleVelocity.  Bound by FP64 issue (80 % of the pipe): 10 instructions per particle, 16
+// when each particle subtracted its nodes' old velocities; 17.6 million particles: 698 -> CORRECT_NEW us.
 __global__ void k_correct(const int* __restrict__ np_ptr, PState P, Centers C, const int4* __restrict__ tri,
-                          const double* __restrict__ ux, const double* __restrict__ uy,
-                          const double* __restrict__ uxo, const double* __restrict__ uyo) {
+                          const double* __restrict__ dx, const double* __restrict__ dy) {
     const int np = *np_ptr;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
         const int w = P.cw[p];
         if (w < 0) continue;
         const int4 t = tri[w & kCellMask];
         const double l0 = P.l0[p], l1 = P.l1[p], l2 = third_coord(w, l0, l1, C);
-        double dx0 = ux[t.x], dx1 = ux[t.y], dx2 = ux[t.z];
-        double dy0 = uy[t.x], dy1 = uy[t.y], dy2 = uy[t.z];
-        if (uxo) {
-            dx0 = __dsub_rn(dx0, uxo[t.x]); dx1 = __dsub_rn(dx1, uxo[t.y]); dx2 = __dsub_rn(dx2, uxo[t.z]);
-            dy0 = __dsub_rn(dy0, uyo[t.x]); dy1 = __dsub_rn(dy1, uyo[t.y]); dy2 = __dsub_rn(dy2, uyo[t.z]);
-        }
-        P.u[p] = __dadd_rn(P.u[p], interp3(l0, l1, l2, dx0, dx1, dx2));
-        P.v[p] = __dadd_rn(P.v[p], interp3(l0, l1, l2, dy0, dy1, dy2));
+        P.u[p] = __dadd_rn(P.u[p], interp3(l0, l1, l2, dx[t.x], dx[t.y], dx[t.z]));
+        P.v[p] = __dadd_rn(P.v[p], interp3(l0, l1, l2, dy[t.x], dy[t.y], dy[t.z]));
     }
 }
 
@@ -522,7 +589,7 @@ struct pf2_particles {
     DevBuf<int> cw[2];
     int cur = 0;
     DevBuf<int> rank, perm, count, mask, seg, segsz, scratch, cnt, err;
-    DevBuf<double> part;
+    DevBuf<double> part, change;  // projection partial sums; k_node_change
     PinnedBuf<int> h_cnt;
     bool partials_valid = false;
     bool seeded = false;
@@ -614,8 +681,14 @@ pf2_status particles_project(pf2_particles* H, double* ux, double* uy, double* u
 
 pf2_status particles_correct(pf2_particles* H, const double* ux, const double* uy, const double* uxo,
                              const double* uyo, cudaStream_t st) {
-    k_correct<<<particle_grid(), kThreads, 0, st>>>(H->cnt.p, H->state(H->cur), H->C, H->mesh->tri4.p, ux, uy, uxo,
-                                                    uyo);
+    if (uxo) {
+        const int nv = H->mesh->nv;
+        k_node_change<<<blocks_for(nv), kThreads, 0, st>>>(nv, ux, uy, uxo, uyo, H->change.p, H->change.p + nv);
+        PF2_LAUNCH_CHECK();
+        ux = H->change.p;
+        uy = H->change.p + nv;
+    }
+    k_correct<<<particle_grid(), kThreads, 0, st>>>(H->cnt.p, H->state(H->cur), H->C, H->mesh->tri4.p, ux, uy);
     PF2_LAUNCH_CHECK();
     H->partials_valid = false;
     return PF2_OK;
@@ -745,7 +818,7 @@ pf2_status pf2_particles_create(const pf2_mesh* m, int level, double capacity_fa
     if ((s = H->rank.alloc(H->cap)) || (s = H->perm.alloc(H->cap)) || (s = H->count.alloc(nc + 1)) ||
         (s = H->mask.alloc(nc + 1)) || (s = H->seg.alloc(nc + 1)) || (s = H->segsz.alloc(nc + 1)) ||
         (s = H->scratch.alloc(scan_scratch_ints(nc))) || (s = H->cnt.alloc(2)) || (s = H->err.alloc(1)) ||
-        (s = H->part.alloc(9 * (size_t)nc)) || (s = H->h_cnt.alloc(2)))
+        (s = H->part.alloc(9 * (size_t)nc)) || (s = H->change.alloc(2 * (size_t)m->nv)) || (s = H->h_cnt.alloc(2)))
         return fail(s);
     if (cudaMemset(H->count.p, 0, sizeof(int) * (nc + 1)) != cudaSuccess ||
         cudaMemset(H->mask.p, 0, sizeof(int) * (nc + 1)) != cudaSuccess ||
