@@ -29,7 +29,7 @@
 namespace pf2 {
 
 struct GmresMgs {
-    double* L;                 // (i, j) at j (m + 1) + i: v_i.v_j, j < i (written by block 0)
+    // (the rows of L, written by block 0, lie in H's unused triangle: v_i.v_j, j < i, at m j + i)
     unsigned long long* part;  // packets (zeroed before the launch): 2 x (2 m + 2) x G parts, 2 x (2 m + 2)
                                // totals, 2 x G parts of norms; then the counter of norm parts
 };
@@ -367,12 +367,12 @@ __global__ void __launch_bounds__(kSolverThreads, 1) k_gmres_mgs(KArgs a, GmresM
                     } else {
                         g[v - k - 1] = d;
                         if (k < kGramRows) Ls[(v - k - 1) * (kGramRows + 1) + k] = d;
-                        if (blockIdx.x == 0) __stcg(&C.L[(size_t)(v - k - 1) * (m + 1) + k], d);
+                        if (blockIdx.x == 0) __stcg(&a.H[(size_t)(v - k - 1) * m + k], d);
                     }
                 }
             }
             __syncthreads();
-            gmres_solve_lower(h, g, Ls, C.L, m + 1, k);
+            gmres_solve_lower(h, g, Ls, a.H, m, k);
             nn = 0.0;
             for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
                 double v = w[j];

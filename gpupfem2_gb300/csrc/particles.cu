@@ -401,7 +401,7 @@ __device__ __forceinline__ void block_partials(PartialStage& G, int c0, int nc, 
 // reseeds and sums.  A warp's particles go to the stage of the sums as they are moved, without a
 // second trip through L2, and the block's reseeds (a few per cell) are made together, so that
 // their FP64 instructions serve full warps.  17.6 million particles: 2,340 us with the reseeds
-// per warp and the stage read back -> GATHER_NEW us.
+// per warp and the stage read back -> 1,757 us.
 __global__ void __launch_bounds__(256, 5) k_gather(int nc, const int* __restrict__ seg, int* count, int* mask,
                                                 const int* __restrict__ perm, PState S, PState D, Centers C,
                                                 int level, int reseed, const double2* __restrict__ xy,
@@ -561,7 +561,7 @@ __global__ void k_node_change(int nv, const double* __restrict__ ux, const doubl
 
 // kCorrectParticleVelocity (:72-88) with the nodes' change of velocity; with the velocity itself
 // initParticleVelocity.  Bound by FP64 issue (80 % of the pipe): 10 instructions per particle, 16
-// when each particle subtracted its nodes' old velocities; 17.6 million particles: 698 -> CORRECT_NEW us.
+// when each particle subtracted its nodes' old velocities; 17.6 million particles: 698 -> 436 us.
 __global__ void k_correct(const int* __restrict__ np_ptr, PState P, Centers C, const int4* __restrict__ tri,
                           const double* __restrict__ dx, const double* __restrict__ dy) {
     const int np = *np_ptr;

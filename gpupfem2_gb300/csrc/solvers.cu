@@ -11,8 +11,13 @@
 // identical bits.  The ILU(0)/IC(0) factorisation and triangular solves walk the rows
 // in level order; a row waits (bounded) until the rows it depends on are done.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
+#include <exception>
+#include <functional>
 #include <mutex>
+#include <system_error>
+#include <thread>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -2792,7 +2797,7 @@ struct pf2_solver {
     const pf2_mesh* mesh = nullptr;
     int n = 0, nnz = 0, blocks = 0, m = 0;
     long long barrier_polls = 0;  // PF2_BARRIER_POLLS (tests): a grid-barrier wait's poll limit
-    DevBuf<double> r, z, p, q, s, invd, partial, V, H, vpart, rhat, yv, tv, gram;
+    DevBuf<double> r, z, p, q, s, invd, partial, V, H, vpart, rhat, yv, tv;
     DevBuf<unsigned long long> packets;  // GMRES: k_gmres_mgs
     DevBuf<unsigned> bar;  // count, gen
     DevBuf<int> err;
@@ -2844,9 +2849,10 @@ struct pf2_solver {
     int halo_RL = 0, halo_TL = 0, halo_E = 0;
     bool halo_res = false;
     long long halo_ne = 0, halo_nd = 0;  // stream entries, diagonals
-    DevBuf<int> h_hoff, h_hq, h_foff, h_fg, h_zoff, h_zg, h_r1off, h_ioff, h_wit, h_went, h_gsl, h_dmap;
-    DevBuf<unsigned short> h_fl, h_zl, h_r1, h_col;
-    DevBuf<unsigned char> h_pub, h_item;
+    DevBuf<unsigned char> h_plan;  // the arrays below, one after another
+    int *h_hoff, *h_hq, *h_foff, *h_fg, *h_zoff, *h_zg, *h_r1off, *h_ioff, *h_wit, *h_went, *h_gsl, *h_dmap;
+    unsigned short *h_fl, *h_zl, *h_r1, *h_col;
+    unsigned char *h_pub, *h_item;
     DevBuf<unsigned long long> h_gq, h_gt;  // packets of the exchanges
     DevBuf<double> h_diag;
     // CG with level sweeps in one block (k_pcg_level): streams, units and what their values are
@@ -2986,15 +2992,18 @@ static int multicolour_order(int n, const int* rp, const int* col, bool kempe, s
 // node (the last node a breadth-first search from the subset's first node reaches; a
 // disconnected subset continues from its next unreached node) and cut after the rows of
 // its first P / 2 parts.  part[i] receives the part of row i.
-static void graph_parts(int n, const std::vector<int>& rp, const std::vector<int>& col, int P, std::vector<int>& part) {
-    part.assign(n, 0);
-    std::vector<int> order(n), tmp(n), subset(n, -1), seen(n, -1);
-    for (int i = 0; i < n; ++i) order[i] = i;
-    struct Job { int lo, hi, P, first; };
-    std::vector<Job> jobs{ { 0, n, P, 0 } };
-    int sid = 0, stamp = 0;
-    auto bfs = [&](int lo, int hi, int start) {
-        ++stamp;
+// Subsets are independent, so the larger half of a cut goes to another thread as long as both
+// are worth one (the result is the same; 499,288 rows into 152 parts: 55 -> 27 ms).
+constexpr int kPlanThreads = 8;
+
+struct GraphCut {
+    const std::vector<int>&rp, &col;
+    std::vector<int>& part;
+    std::vector<int> order, tmp, subset, seen;
+    std::atomic<int> subsets{ 0 };
+
+    // breadth-first order of the rows order[lo .. hi) of subset sid into tmp
+    int bfs(int lo, int hi, int sid, int stamp, int start) {
         int w = lo, next = lo;
         tmp[w++] = start;
         seen[start] = stamp;
@@ -3007,31 +3016,66 @@ static void graph_parts(int n, const std::vector<int>& rp, const std::vector<int
             const int v = tmp[h];
             for (int k = rp[v]; k < rp[v + 1]; ++k) {
                 const int u = col[k];
-                if (subset[u] == sid && seen[u] != stamp) {
+                // (another thread may be moving u to a subset of its own, never to this one)
+                if (__atomic_load_n(&subset[u], __ATOMIC_RELAXED) == sid && seen[u] != stamp) {
                     seen[u] = stamp;
                     tmp[w++] = u;
                 }
             }
         }
         return tmp[hi - 1];
-    };
-    while (!jobs.empty()) {
-        const Job j = jobs.back();
-        jobs.pop_back();
-        if (j.P <= 1 || j.hi - j.lo <= 1) {
-            for (int q = j.lo; q < j.hi; ++q) part[order[q]] = j.first;
-            continue;
-        }
-        ++sid;
-        for (int q = j.lo; q < j.hi; ++q) subset[order[q]] = sid;
-        const int far = bfs(j.lo, j.hi, order[j.lo]);
-        bfs(j.lo, j.hi, far);
-        std::copy(tmp.begin() + j.lo, tmp.begin() + j.hi, order.begin() + j.lo);
-        const int P1 = j.P / 2;
-        const int mid = j.lo + (int)((long long)(j.hi - j.lo) * P1 / j.P);
-        jobs.push_back({ mid, j.hi, j.P - P1, j.first + P1 });
-        jobs.push_back({ j.lo, mid, P1, j.first });
     }
+    void cut(int lo, int hi, int P, int first, int threads) {
+        if (P <= 1 || hi - lo <= 1) {
+            for (int q = lo; q < hi; ++q) part[order[q]] = first;
+            return;
+        }
+        const int sid = subsets++;
+        for (int q = lo; q < hi; ++q) __atomic_store_n(&subset[order[q]], sid, __ATOMIC_RELAXED);
+        const int far = bfs(lo, hi, sid, 2 * sid, order[lo]);
+        bfs(lo, hi, sid, 2 * sid + 1, far);
+        std::copy(tmp.begin() + lo, tmp.begin() + hi, order.begin() + lo);
+        const int P1 = P / 2;
+        const int mid = lo + (int)((long long)(hi - lo) * P1 / P);
+        std::thread other;
+        if (threads > 1 && hi - lo >= 4096) {
+            try {
+                other = std::thread([=] { cut(mid, hi, P - P1, first + P1, threads / 2); });
+            } catch (const std::system_error&) {}  // no thread to be had
+        }
+        cut(lo, mid, P1, first, threads / 2);
+        if (other.joinable()) other.join();
+        else cut(mid, hi, P - P1, first + P1, threads / 2);
+    }
+};
+
+static void graph_parts(int n, const std::vector<int>& rp, const std::vector<int>& col, int P, std::vector<int>& part) {
+    part.assign(n, 0);
+    GraphCut G{ rp, col, part, std::vector<int>(n), std::vector<int>(n), std::vector<int>(n, -1), std::vector<int>(n, -1) };
+    for (int i = 0; i < n; ++i) G.order[i] = i;
+    G.cut(0, n, P, 0, std::min<int>(kPlanThreads, std::max(1u, std::thread::hardware_concurrency())));
+}
+
+// f(worker, first, last) for `workers` ranges of 0 .. n, each on a thread of its own where one can
+// be had; the first exception of any is thrown here.
+template <class F>
+static void parallel_ranges(int n, int workers, F&& f) {
+    std::vector<std::thread> t;
+    std::vector<std::exception_ptr> err(workers);
+    auto run = [&](int w) {
+        try {
+            f(w, (int)((long long)n * w / workers), (int)((long long)n * (w + 1) / workers));
+        } catch (...) { err[w] = std::current_exception(); }
+    };
+    t.reserve(workers);
+    int w = 0;
+    try {
+        for (; w + 1 < workers; ++w) t.emplace_back(run, w);
+    } catch (const std::system_error&) {}
+    for (; w < workers; ++w) run(w);
+    for (std::thread& x : t) x.join();
+    for (const std::exception_ptr& e : err)
+        if (e) std::rethrow_exception(e);
 }
 
 // The partitioned CG plan (k_pcg_part) for the pattern of B = P A P^T (brp, bcol; bmap:
@@ -3065,9 +3109,10 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
         if (atoi(e) == 3) return PF2_OK;  // tests: the kernel with waits inside the sweeps
     if (const char* e = getenv("PF2_CG_PART_LOCAL"))
         if (mixed && tri && atoi(e) != 0) return PF2_OK;
-    // pid: the part of a row of B; cls: the row's membership in the halo of part stamp
-    std::vector<int> pid(n), local(n, -1), stamp(n, -1);
-    std::vector<unsigned char> cls(n, 0), pub(n, 0), pub_t(n, 0);
+    // pid: the part of a row of B
+    std::vector<int> pid(n);
+    std::vector<unsigned char> pub(n, 0), pub_t(n, 0);
+    const int workers = std::max(1, std::min({ kPlanThreads, (int)std::thread::hardware_concurrency(), n / 4096, P }));
     for (int r = 0; r < n; ++r) pid[r] = part[perm[r]];
     enum { F = 1, Z = 2 };
     struct Halo {
@@ -3076,179 +3121,228 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
         std::vector<unsigned char> cls;
     };
     std::vector<Halo> H(P);
-    std::vector<std::vector<int>> bucket(ng);
-    int RL = 0;
-    for (int k = 0; k < P; ++k) {
-        Halo& h = H[k];
-        const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0;
-        // ring 1, the F rows among it (read by an own row's lower entries) and the closures
-        for (auto& b : bucket) b.clear();
-        int nh = 0;
-        auto add = [&](int j, int bits) {
-            if (stamp[j] != k) {
-                stamp[j] = k;
-                cls[j] = 0;
-                bucket[grp[j]].push_back(j);
-                ++nh;
-            }
-            cls[j] |= bits;
-        };
-        for (int q = p0; q < p0 + np; ++q) {
-            const int i = qb[q];
-            for (int e = brp[i]; e < brp[i + 1]; ++e) {
-                const int j = bcol[e];
-                if (pid[j] == k) continue;
-                if (stamp[j] != k) h.ring.push_back(j);
-                add(j, !tri ? F : (e < bdiag[i] ? F | Z : Z));
-            }
-        }
-        if (tri) {
-            for (int g = ng - 1; g >= 0; --g)  // rows added have lower groups
-                for (size_t c = 0; c < bucket[g].size(); ++c) {
-                    const int i = bucket[g][c];
-                    if (!(cls[i] & F)) continue;
-                    for (int e = brp[i]; e < bdiag[i]; ++e)
-                        if (pid[bcol[e]] != k) add(bcol[e], F);
+    std::vector<int> rl(workers, 0);
+    std::atomic<bool> too_many{ false };
+    parallel_ranges(P, workers, [&](int worker, int k0, int k1) {
+        std::vector<int> stamp(n, -1);  // cls: the row's membership in the halo of part stamp
+        std::vector<unsigned char> cls(n, 0);
+        std::vector<std::vector<int>> bucket(ng);
+        for (int k = k0; k < k1 && !too_many; ++k) {
+            Halo& h = H[k];
+            const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0;
+            // ring 1, the F rows among it (read by an own row's lower entries) and the closures
+            for (auto& b : bucket) b.clear();
+            int nh = 0;
+            auto add = [&](int j, int bits) {
+                if (stamp[j] != k) {
+                    stamp[j] = k;
+                    cls[j] = 0;
+                    bucket[grp[j]].push_back(j);
+                    ++nh;
                 }
-            for (int g = 0; g < ng; ++g)  // rows added have higher groups
-                for (size_t c = 0; c < bucket[g].size(); ++c) {
-                    const int i = bucket[g][c];
-                    if (!(cls[i] & Z)) continue;
-                    for (int e = bdiag[i] + 1; e < brp[i + 1]; ++e)
-                        if (pid[bcol[e]] != k) add(bcol[e], Z);
-                }
-        }
-        if (nh > std::max(4 * np, 64) || np + nh >= kHaloMaxLocal) {
-            S->part_why = "the halo rows outnumber a part's rows";
-            return PF2_OK;
-        }
-        RL = std::max(RL, np + nh);
-        h.f0.resize(ng);
-        h.f1.resize(ng);
-        h.z0.resize(ng);
-        h.z1.resize(ng);
-        for (int g = 0; g < ng; ++g) {
-            auto& b = bucket[g];
-            std::sort(b.begin(), b.end());
-            auto put = [&](int want) {
-                for (int i : b)
-                    if (cls[i] == want) h.rows.push_back(i);
+                cls[j] |= bits;
             };
-            h.f0[g] = (int)h.rows.size();
-            put(F);
-            h.z0[g] = (int)h.rows.size();
-            put(F | Z);
-            h.f1[g] = (int)h.rows.size();
-            put(Z);
-            h.z1[g] = (int)h.rows.size();
-        }
-        h.cls.resize(nh);
-        for (int c = 0; c < nh; ++c) {
-            h.cls[c] = cls[h.rows[c]];
-            (h.cls[c] & F ? pub : pub_t)[bq[h.rows[c]]] = 1;
-        }
-    }
-    std::vector<int> hoff(P + 1, 0), hq, foff(P + 1, 0), fg, zoff(P + 1, 0), zg, r1off(P + 1, 0), ioff(P + 1, 0), wit, went,
-        gsl, map, dmap;
-    std::vector<unsigned char> item;
-    std::vector<unsigned short> fl, zl, r1, col;
-    int TL = 0;
-    const size_t guess = (size_t)S->nnz * (tri ? 9 : 5) / 4;
-    col.reserve(guess);
-    map.reserve(guess);
-    const std::vector<int> none;
-    for (int k = 0; k < P; ++k) {
-        const Halo& h = H[k];
-        const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0, nh = (int)h.rows.size();
-        for (int q = p0; q < p0 + np; ++q) local[qb[q]] = q - p0;
-        for (int c = 0; c < nh; ++c) {
-            const int i = h.rows[c];
-            local[i] = np + c;
-            hq.push_back(bq[i]);
-            if (h.cls[c] & F) {
-                fl.push_back((unsigned short)local[i]);
-                fg.push_back(bq[i]);
-            } else {
-                zl.push_back((unsigned short)local[i]);
-                zg.push_back(bq[i]);
-            }
-        }
-        for (int i : h.ring) r1.push_back((unsigned short)local[i]);
-        if (!tri) {
-            for (int q = p0; q < p0 + np; ++q) dmap.push_back(bmap[bdiag[qb[q]]]);
-            for (int i : h.rows) dmap.push_back(bmap[bdiag[i]]);
-        }
-        // the slice of rows row(s .. min(s + 32, m) - 1), entries [lo(i), hi(i)) of row i, cut into
-        // items; a padding entry has the value 0 and a column that is safe to read: the row's
-        // first entry, or the row itself.  set 0: SpMV (values of A), 1: forward, 2: backward
-        // (factor values, flagged in the map; the first entry row holds the pivots)
-        auto emit = [&](int m, int s, auto row, auto lo, auto hi, int set) {
-            const int wd = std::min(32, m - s);
-            int len = 0;
-            for (int j = 0; j < wd; ++j) len = std::max(len, hi(row(s + j)) - lo(row(s + j)));
-            const int lead = set ? 1 : 0, rows = len + lead;
-            const size_t at = col.size();
-            col.resize(at + 32 * (size_t)rows, 0);
-            map.resize(col.size(), -1);
-            for (int j = 0; j < wd; ++j) {
-                const int i = row(s + j), e0 = lo(i), n_i = hi(i) - e0;
-                if (lead) {
-                    const bool publish = set == 1 && local[i] < np && pub_t[bq[i]];
-                    col[at + j] = (unsigned short)(local[i] | (publish ? kHaloPubT : 0));
-                    map[at + j] = bdiag[i] | kHaloFactor;
+            for (int q = p0; q < p0 + np; ++q) {
+                const int i = qb[q];
+                for (int e = brp[i]; e < brp[i + 1]; ++e) {
+                    const int j = bcol[e];
+                    if (pid[j] == k) continue;
+                    if (stamp[j] != k) h.ring.push_back(j);
+                    add(j, !tri ? F : (e < bdiag[i] ? F | Z : Z));
                 }
-                for (int e = 0; e < len; ++e) {
-                    const size_t o = at + 32 * (size_t)(e + lead) + j;
-                    if (e < n_i) {
-                        col[o] = (unsigned short)local[bcol[e0 + e]];
-                        map[o] = set ? (e0 + e) | kHaloFactor : bmap[e0 + e];
-                    } else {
-                        col[o] = (unsigned short)local[n_i ? bcol[e0] : i];
+            }
+            if (tri) {
+                for (int g = ng - 1; g >= 0; --g)  // rows added have lower groups
+                    for (size_t c = 0; c < bucket[g].size(); ++c) {
+                        const int i = bucket[g][c];
+                        if (!(cls[i] & F)) continue;
+                        for (int e = brp[i]; e < bdiag[i]; ++e)
+                            if (pid[bcol[e]] != k) add(bcol[e], F);
                     }
-                }
+                for (int g = 0; g < ng; ++g)  // rows added have higher groups
+                    for (size_t c = 0; c < bucket[g].size(); ++c) {
+                        const int i = bucket[g][c];
+                        if (!(cls[i] & Z)) continue;
+                        for (int e = bdiag[i] + 1; e < brp[i + 1]; ++e)
+                            if (pid[bcol[e]] != k) add(bcol[e], Z);
+                    }
             }
-            if (lead)
-                for (int j = wd; j < 32; ++j) col[at + j] = kHaloNone;
-            for (int e = 0; e < rows; e += kHaloItem) {
-                const int c = std::min(kHaloItem, rows - e);
-                item.push_back((unsigned char)(c | (e + c == rows ? kHaloLast : 0)));
+            if (nh > std::max(4 * np, 64) || np + nh >= kHaloMaxLocal) {
+                too_many = true;
+                return;
             }
-        };
-        auto row_lo = [&](int i) { return brp[i]; };
-        auto row_hi = [&](int i) { return brp[i + 1]; };
-        auto low_hi = [&](int i) { return bdiag[i]; };
-        auto up_lo = [&](int i) { return bdiag[i] + 1; };
-        for (int dir = 0; dir < 2; ++dir)
+            rl[worker] = std::max(rl[worker], np + nh);
+            h.f0.resize(ng);
+            h.f1.resize(ng);
+            h.z0.resize(ng);
+            h.z1.resize(ng);
             for (int g = 0; g < ng; ++g) {
-                const int no = qs[(size_t)k * ng + g + 1] - qs[(size_t)k * ng + g];
-                const int nc = dir == 0 ? h.f1[g] - h.f0[g] : h.z1[g] - h.z0[g];
-                gsl.push_back(tri ? (no + nc + 31) / 32 : 0);
+                auto& b = bucket[g];
+                std::sort(b.begin(), b.end());
+                auto put = [&](int want) {
+                    for (int i : b)
+                        if (cls[i] == want) h.rows.push_back(i);
+                };
+                h.f0[g] = (int)h.rows.size();
+                put(F);
+                h.z0[g] = (int)h.rows.size();
+                put(F | Z);
+                h.f1[g] = (int)h.rows.size();
+                put(Z);
+                h.z1[g] = (int)h.rows.size();
             }
-        for (int w = 0; w < kHaloWarps; ++w) {
-            went.push_back((int)(col.size() / 32));
-            wit.push_back((int)item.size() - ioff[k]);
-            for (int dir = 0; dir < 2 && tri; ++dir)
-                for (int gi = 0; gi < ng; ++gi) {
-                    const int g = dir == 0 ? gi : ng - 1 - gi;
-                    const int o0 = qs[(size_t)k * ng + g], no = qs[(size_t)k * ng + g + 1] - o0;
-                    const int c0 = dir == 0 ? h.f0[g] : h.z0[g], nc = (dir == 0 ? h.f1[g] : h.z1[g]) - c0;
-                    auto row = [&](int c) { return c < no ? qb[o0 + c] : h.rows[c0 + c - no]; };
-                    for (int s = 32 * w; s < no + nc; s += 32 * kHaloWarps) {
-                        if (dir == 0) emit(no + nc, s, row, row_lo, low_hi, 1);
-                        else emit(no + nc, s, row, up_lo, row_hi, 2);
+            h.cls.resize(nh);
+            for (int c = 0; c < nh; ++c) {
+                h.cls[c] = cls[h.rows[c]];
+                __atomic_store_n(&(h.cls[c] & F ? pub : pub_t)[bq[h.rows[c]]], (unsigned char)1, __ATOMIC_RELAXED);
+            }
+        }
+    });
+    if (too_many) {
+        S->part_why = "the halo rows outnumber a part's rows";
+        return PF2_OK;
+    }
+    const int RL = *std::max_element(rl.begin(), rl.end());
+    // each worker's parts, one after another; put together below
+    struct Piece {
+        std::vector<int> hq, fg, zg, wit, went, gsl, map, dmap, hoff, foff, zoff, r1off, ioff;
+        std::vector<unsigned char> item;
+        std::vector<unsigned short> fl, zl, r1, col;
+        int TL = 0;
+    };
+    std::vector<Piece> piece(workers);
+    parallel_ranges(P, workers, [&](int worker, int k0, int k1) {
+        auto& [hq, fg, zg, wit, went, gsl, map, dmap, hoff, foff, zoff, r1off, ioff, item, fl, zl, r1, col, TL] = piece[worker];
+        std::vector<int> local(n, -1);
+        const size_t guess = (size_t)S->nnz * (tri ? 9 : 5) / 4 / P * (k1 - k0);
+        col.reserve(guess);
+        map.reserve(guess);
+        for (int k = k0; k < k1; ++k) {
+            const Halo& h = H[k];
+            const int item0 = (int)item.size();
+            const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0, nh = (int)h.rows.size();
+            for (int q = p0; q < p0 + np; ++q) local[qb[q]] = q - p0;
+            for (int c = 0; c < nh; ++c) {
+                const int i = h.rows[c];
+                local[i] = np + c;
+                hq.push_back(bq[i]);
+                if (h.cls[c] & F) {
+                    fl.push_back((unsigned short)local[i]);
+                    fg.push_back(bq[i]);
+                } else {
+                    zl.push_back((unsigned short)local[i]);
+                    zg.push_back(bq[i]);
+                }
+            }
+            for (int i : h.ring) r1.push_back((unsigned short)local[i]);
+            if (!tri) {
+                for (int q = p0; q < p0 + np; ++q) dmap.push_back(bmap[bdiag[qb[q]]]);
+                for (int i : h.rows) dmap.push_back(bmap[bdiag[i]]);
+            }
+            // the slice of rows row(s .. min(s + 32, m) - 1), entries [lo(i), hi(i)) of row i, cut into
+            // items; a padding entry has the value 0 and a column that is safe to read: the row's
+            // first entry, or the row itself.  set 0: SpMV (values of A), 1: forward, 2: backward
+            // (factor values, flagged in the map; the first entry row holds the pivots)
+            auto emit = [&](int m, int s, auto row, auto lo, auto hi, int set) {
+                const int wd = std::min(32, m - s);
+                int len = 0;
+                for (int j = 0; j < wd; ++j) len = std::max(len, hi(row(s + j)) - lo(row(s + j)));
+                const int lead = set ? 1 : 0, rows = len + lead;
+                const size_t at = col.size();
+                col.resize(at + 32 * (size_t)rows, 0);
+                map.resize(col.size(), -1);
+                for (int j = 0; j < wd; ++j) {
+                    const int i = row(s + j), e0 = lo(i), n_i = hi(i) - e0;
+                    if (lead) {
+                        const bool publish = set == 1 && local[i] < np && pub_t[bq[i]];
+                        col[at + j] = (unsigned short)(local[i] | (publish ? kHaloPubT : 0));
+                        map[at + j] = bdiag[i] | kHaloFactor;
+                    }
+                    for (int e = 0; e < len; ++e) {
+                        const size_t o = at + 32 * (size_t)(e + lead) + j;
+                        if (e < n_i) {
+                            col[o] = (unsigned short)local[bcol[e0 + e]];
+                            map[o] = set ? (e0 + e) | kHaloFactor : bmap[e0 + e];
+                        } else {
+                            col[o] = (unsigned short)local[n_i ? bcol[e0] : i];
+                        }
                     }
                 }
-            wit.push_back((int)item.size() - ioff[k]);
-            for (int s = 32 * w; s < np; s += 32 * kHaloWarps)
-                emit(np, s, [&](int c) { return qb[p0 + c]; }, row_lo, row_hi, 0);
+                if (lead)
+                    for (int j = wd; j < 32; ++j) col[at + j] = kHaloNone;
+                for (int e = 0; e < rows; e += kHaloItem) {
+                    const int c = std::min(kHaloItem, rows - e);
+                    item.push_back((unsigned char)(c | (e + c == rows ? kHaloLast : 0)));
+                }
+            };
+            auto row_lo = [&](int i) { return brp[i]; };
+            auto row_hi = [&](int i) { return brp[i + 1]; };
+            auto low_hi = [&](int i) { return bdiag[i]; };
+            auto up_lo = [&](int i) { return bdiag[i] + 1; };
+            for (int dir = 0; dir < 2; ++dir)
+                for (int g = 0; g < ng; ++g) {
+                    const int no = qs[(size_t)k * ng + g + 1] - qs[(size_t)k * ng + g];
+                    const int nc = dir == 0 ? h.f1[g] - h.f0[g] : h.z1[g] - h.z0[g];
+                    gsl.push_back(tri ? (no + nc + 31) / 32 : 0);
+                }
+            for (int w = 0; w < kHaloWarps; ++w) {
+                went.push_back((int)(col.size() / 32));
+                wit.push_back((int)item.size() - item0);
+                for (int dir = 0; dir < 2 && tri; ++dir)
+                    for (int gi = 0; gi < ng; ++gi) {
+                        const int g = dir == 0 ? gi : ng - 1 - gi;
+                        const int o0 = qs[(size_t)k * ng + g], no = qs[(size_t)k * ng + g + 1] - o0;
+                        const int c0 = dir == 0 ? h.f0[g] : h.z0[g], nc = (dir == 0 ? h.f1[g] : h.z1[g]) - c0;
+                        auto row = [&](int c) { return c < no ? qb[o0 + c] : h.rows[c0 + c - no]; };
+                        for (int s = 32 * w; s < no + nc; s += 32 * kHaloWarps) {
+                            if (dir == 0) emit(no + nc, s, row, row_lo, low_hi, 1);
+                            else emit(no + nc, s, row, up_lo, row_hi, 2);
+                        }
+                    }
+                wit.push_back((int)item.size() - item0);
+                for (int s = 32 * w; s < np; s += 32 * kHaloWarps)
+                    emit(np, s, [&](int c) { return qb[p0 + c]; }, row_lo, row_hi, 0);
+            }
+            TL = std::max(TL, (int)item.size() - item0);
+            ioff.push_back((int)item.size());
+            hoff.push_back((int)hq.size());
+            foff.push_back((int)fl.size());
+            zoff.push_back((int)zl.size());
+            r1off.push_back((int)r1.size());
         }
-        TL = std::max(TL, (int)item.size() - ioff[k]);
-        ioff[k + 1] = (int)item.size();
-        hoff[k + 1] = (int)hq.size();
-        foff[k + 1] = (int)fl.size();
-        zoff[k + 1] = (int)zl.size();
-        r1off[k + 1] = (int)r1.size();
+    });
+    Piece all;
+    for (std::vector<int>* v : { &all.hoff, &all.foff, &all.zoff, &all.r1off, &all.ioff }) v->push_back(0);
+    for (Piece& w : piece) {
+        // offsets count from the pieces before (the last entry of what is there; went: its entry rows)
+        auto add = [](std::vector<int>& to, const std::vector<int>& v, int base) {
+            for (int x : v) to.push_back(base + x);
+        };
+        add(all.hoff, w.hoff, all.hoff.back());
+        add(all.foff, w.foff, all.foff.back());
+        add(all.zoff, w.zoff, all.zoff.back());
+        add(all.r1off, w.r1off, all.r1off.back());
+        add(all.ioff, w.ioff, all.ioff.back());
+        add(all.went, w.went, (int)(all.col.size() / 32));
+        auto join = [](auto& to, auto& v) {
+            if (to.empty()) to = std::move(v);
+            else to.insert(to.end(), v.begin(), v.end());
+        };
+        join(all.hq, w.hq);
+        join(all.fg, w.fg);
+        join(all.zg, w.zg);
+        join(all.wit, w.wit);
+        join(all.gsl, w.gsl);
+        join(all.map, w.map);
+        join(all.dmap, w.dmap);
+        join(all.item, w.item);
+        join(all.fl, w.fl);
+        join(all.zl, w.zl);
+        join(all.r1, w.r1);
+        join(all.col, w.col);
+        all.TL = std::max(all.TL, w.TL);
     }
+    auto& [hq, fg, zg, wit, went, gsl, map, dmap, hoff, foff, zoff, r1off, ioff, item, fl, zl, r1, col, TL] = all;
     went.push_back((int)(col.size() / 32));
     int E = 0;
     for (int k = 0; k < P; ++k) E = std::max(E, went[(size_t)(k + 1) * kHaloWarps] - went[(size_t)k * kHaloWarps]);
@@ -3268,25 +3362,36 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
     };
     PF2_TRY(up(S->q_s, qs));
     PF2_TRY(up(S->q_a, qa));
-    PF2_TRY(up(S->h_dmap, dmap));
-    PF2_TRY(up(S->h_hoff, hoff));
-    PF2_TRY(up(S->h_hq, hq));
-    PF2_TRY(up(S->h_foff, foff));
-    PF2_TRY(up(S->h_fl, fl));
-    PF2_TRY(up(S->h_fg, fg));
-    PF2_TRY(up(S->h_zoff, zoff));
-    PF2_TRY(up(S->h_zl, zl));
-    PF2_TRY(up(S->h_zg, zg));
-    PF2_TRY(up(S->h_r1off, r1off));
-    PF2_TRY(up(S->h_r1, r1));
-    PF2_TRY(up(S->h_ioff, ioff));
-    PF2_TRY(up(S->h_item, item));
-    PF2_TRY(up(S->h_wit, wit));
-    PF2_TRY(up(S->h_went, went));
-    PF2_TRY(up(S->h_gsl, gsl));
-    PF2_TRY(up(S->h_col, col));
     PF2_TRY(up(S->q_amap, map));
-    PF2_TRY(up(S->h_pub, pub));
+    // one allocation and one copy for the rest: a small system's plan is mostly their calls
+    std::vector<unsigned char> plan;
+    std::vector<std::function<void(unsigned char*)>> place;
+    auto pack = [&](auto*& d, const auto& v) {
+        const size_t at = (plan.size() + 255) / 256 * 256, bytes = sizeof(v[0]) * v.size();
+        plan.resize(at + std::max<size_t>(bytes, 1));
+        if (bytes) memcpy(plan.data() + at, v.data(), bytes);
+        place.push_back([&d, at](unsigned char* base) { d = reinterpret_cast<std::decay_t<decltype(d)>>(base + at); });
+    };
+    pack(S->h_col, col);
+    pack(S->h_dmap, dmap);
+    pack(S->h_hoff, hoff);
+    pack(S->h_hq, hq);
+    pack(S->h_foff, foff);
+    pack(S->h_fl, fl);
+    pack(S->h_fg, fg);
+    pack(S->h_zoff, zoff);
+    pack(S->h_zl, zl);
+    pack(S->h_zg, zg);
+    pack(S->h_r1off, r1off);
+    pack(S->h_r1, r1);
+    pack(S->h_ioff, ioff);
+    pack(S->h_item, item);
+    pack(S->h_wit, wit);
+    pack(S->h_went, went);
+    pack(S->h_gsl, gsl);
+    pack(S->h_pub, pub);
+    PF2_TRY(up(S->h_plan, plan));
+    for (auto& put : place) put(S->h_plan.p);
     PF2_TRY(S->q_val.alloc(col.size()));
     PF2_TRY(S->q_x.alloc(n));
     PF2_TRY(S->h_diag.alloc(dmap.size()));
@@ -4114,7 +4219,7 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
         PF2_CUDA(cudaMemsetAsync(S->rec.p, 0, 5 * sizeof(int), st));
         if (S->halo_nd) {
             k_gather_values<<<std::min((int)blocks_for(S->halo_nd), num_sms() * 8), kThreads, 0, st>>>(
-                S->halo_nd, a.A.val, S->h_dmap.p, S->h_diag.p);
+                S->halo_nd, a.A.val, S->h_dmap, S->h_diag.p);
             PF2_LAUNCH_CHECK();
         }
         if (S->halo) {  // exchange numbers start at 1
@@ -4125,9 +4230,9 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
         PartHalo h{};
         if (S->halo)
             h = PartHalo{ S->part_P, S->part_ng, S->part_R, S->halo_RL, S->halo_TL, S->halo_E, S->q_s.p,
-                          S->h_hoff.p, S->h_hq.p, S->h_foff.p, S->h_fl.p, S->h_fg.p, S->h_zoff.p, S->h_zl.p,
-                          S->h_zg.p, S->h_r1off.p, S->h_r1.p, S->h_pub.p, S->h_ioff.p, S->h_item.p, S->h_wit.p,
-                          S->h_went.p, S->h_gsl.p, S->h_col.p, S->q_val.p, S->q_a.p, S->h_diag.p, S->q_x.p,
+                          S->h_hoff, S->h_hq, S->h_foff, S->h_fl, S->h_fg, S->h_zoff, S->h_zl,
+                          S->h_zg, S->h_r1off, S->h_r1, S->h_pub, S->h_ioff, S->h_item, S->h_wit,
+                          S->h_went, S->h_gsl, S->h_col, S->q_val.p, S->q_a.p, S->h_diag.p, S->q_x.p,
                           S->q_val32.p, S->h_gq.p, S->h_gt.p };
         void* args[] = { &a, &h };
         PF2_COOP_LAUNCH(part_kernel(S), dim3(S->part_P), dim3(part_threads(S)), args, S->part_smem,
@@ -4186,7 +4291,7 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     // iteration elsewhere
     if (!mixed && S->opt.kind == PF2_SOLVER_CG && S->opt.cg_variant == PF2_CG_PIPELINED && S->csr)
         fn = pipe_kernel();
-    GmresMgs gm{ S->gram.p, S->packets.p };
+    GmresMgs gm{ S->packets.p };
     void* args_mgs[] = { &a, &gm };
     if (S->packets.p) PF2_CUDA(cudaMemsetAsync(S->packets.p, 0, S->packets.bytes(), st));  // exchanges count from 1
     PF2_COOP_LAUNCH(fn, dim3(S->blocks), dim3(kSolverThreads), S->packets.p ? args_mgs : args,
@@ -4364,7 +4469,7 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
             (s = S->vpart.alloc((size_t)(m + 1) * (S->blocks + 1))))
             return fail(s);
         if (opt->orthogonalization == PF2_GS_MODIFIED &&
-            ((s = S->gram.alloc((size_t)(m + 1) * (m + 1))) || (s = S->packets.alloc(gmres_packet_words(m, S->blocks)))))
+            (s = S->packets.alloc(gmres_packet_words(m, S->blocks))))
             return fail(s);
     }
     if (uses_tri(S)) {
