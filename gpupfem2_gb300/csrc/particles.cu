@@ -559,21 +559,36 @@ __global__ void k_node_change(int nv, const double* __restrict__ ux, const doubl
     dy[i] = __dsub_rn(uy[i], uyo[i]);
 }
 
-// kCorrectParticleVelocity (:72-88) with the nodes' change of velocity; with the velocity itself
-// initParticleVelocity.  Bound by FP64 issue (80 % of the pipe): 10 instructions per particle, 16
-// when each particle subtracted its nodes' old velocities; 17.6 million particles: 698 -> 436 us.
+// kCorrectParticleVelocity (:72-88): the particle's cell's change of velocity, from the nodes' old
+// velocity uxo, uyo (OLD) or from the change itself; with the velocity itself in its place
+// initParticleVelocity.  Same bits either way.  Bound by FP64 issue (80 % of the pipe): 10
+// instructions per particle with k_node_change, 16 without.  17.6 million particles: 698 us
+// without, 436 + 6 with.
+template <bool OLD>
 __global__ void k_correct(const int* __restrict__ np_ptr, PState P, Centers C, const int4* __restrict__ tri,
-                          const double* __restrict__ dx, const double* __restrict__ dy) {
+                          const double* __restrict__ ux, const double* __restrict__ uy,
+                          const double* __restrict__ uxo, const double* __restrict__ uyo) {
     const int np = *np_ptr;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
         const int w = P.cw[p];
         if (w < 0) continue;
         const int4 t = tri[w & kCellMask];
         const double l0 = P.l0[p], l1 = P.l1[p], l2 = third_coord(w, l0, l1, C);
-        P.u[p] = __dadd_rn(P.u[p], interp3(l0, l1, l2, dx[t.x], dx[t.y], dx[t.z]));
-        P.v[p] = __dadd_rn(P.v[p], interp3(l0, l1, l2, dy[t.x], dy[t.y], dy[t.z]));
+        double dx0 = ux[t.x], dx1 = ux[t.y], dx2 = ux[t.z];
+        double dy0 = uy[t.x], dy1 = uy[t.y], dy2 = uy[t.z];
+        if (OLD) {
+            dx0 = __dsub_rn(dx0, uxo[t.x]); dx1 = __dsub_rn(dx1, uxo[t.y]); dx2 = __dsub_rn(dx2, uxo[t.z]);
+            dy0 = __dsub_rn(dy0, uyo[t.x]); dy1 = __dsub_rn(dy1, uyo[t.y]); dy2 = __dsub_rn(dy2, uyo[t.z]);
+        }
+        P.u[p] = __dadd_rn(P.u[p], interp3(l0, l1, l2, dx0, dx1, dx2));
+        P.v[p] = __dadd_rn(P.v[p], interp3(l0, l1, l2, dy0, dy1, dy2));
     }
 }
+
+// Particles (as seeded) from which on the launch of k_node_change pays.  Three advections with
+// sort and correction, without / with it: 294,912 particles 522 / 522 us; 32,768 particles
+// 187 / 194.
+constexpr long long kNodeChangeMin = 1 << 19;
 
 }  // namespace pf2
 
@@ -681,14 +696,16 @@ pf2_status particles_project(pf2_particles* H, double* ux, double* uy, double* u
 
 pf2_status particles_correct(pf2_particles* H, const double* ux, const double* uy, const double* uxo,
                              const double* uyo, cudaStream_t st) {
-    if (uxo) {
-        const int nv = H->mesh->nv;
+    const int nv = H->mesh->nv;
+    if (uxo && (long long)H->mesh->nc * H->ppc >= kNodeChangeMin) {
         k_node_change<<<blocks_for(nv), kThreads, 0, st>>>(nv, ux, uy, uxo, uyo, H->change.p, H->change.p + nv);
         PF2_LAUNCH_CHECK();
         ux = H->change.p;
         uy = H->change.p + nv;
+        uxo = nullptr;
     }
-    k_correct<<<particle_grid(), kThreads, 0, st>>>(H->cnt.p, H->state(H->cur), H->C, H->mesh->tri4.p, ux, uy);
+    auto* correct = uxo ? k_correct<true> : k_correct<false>;
+    correct<<<particle_grid(), kThreads, 0, st>>>(H->cnt.p, H->state(H->cur), H->C, H->mesh->tri4.p, ux, uy, uxo, uyo);
     PF2_LAUNCH_CHECK();
     H->partials_valid = false;
     return PF2_OK;
