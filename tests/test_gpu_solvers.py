@@ -683,3 +683,35 @@ def test_gmres_low_synchronisation_follows_modified_gram_schmidt(cuda, nx, ny, p
         assert np.linalg.norm(r / diag) <= 1.01e-10 + 1e-13 * np.linalg.norm(rhs / diag)
     else:
         assert np.linalg.norm(r) <= 1e-7 * np.linalg.norm(rhs)
+
+
+@pytest.mark.parametrize("pc", ["ic", "ilu"])
+@pytest.mark.parametrize("kind", ["channel", "box", "wide", "ring", "hub", "star"])
+def test_factors_of_odd_patterns_match_the_oracle(cuda, kind, pc):
+    """ILU(0) / IC(0) of a warp per row (rows of up to 32 entries held by its lanes) against the
+    oracle's, through one preconditioner apply: the same sums in the same order up to fused
+    multiply-adds.  Factors and solves of a matrix whose off-diagonal sums stay within 1/1.05 of
+    the diagonal amplify rounding by at most ~41 (32 operations a row: 41 x 32 x 1.1e-16 =
+    1.4e-13); 1e-12 allowed."""
+    xy, cells = _odd_mesh(kind)
+    m = (g.Mesh3D if kind == "box" else g.Mesh2D).from_arrays(xy, cells)
+    A = g.SparseMatrixCSR(m)
+    rp, col, _ = A.download()
+    n = rp.size - 1
+    row = np.repeat(np.arange(n), np.diff(rp))
+    val = np.where(row == col, 0.0, -1.0 - 0.3 * np.cos(row + col.astype(np.float64)))
+    sums = np.zeros(n)
+    np.add.at(sums, row, -val)
+    val[row == col] = 1.05 * sums
+    A.upload_values(val)
+    s = g.LinearSolver(A, "cg", pc)
+    s.setup(A)
+    src = np.sin(1.0 + np.arange(n))
+    dst = torch.empty(n, dtype=torch.float64, device="cuda")
+    s.apply_preconditioner(dst, torch.tensor(src, device="cuda"))
+    f = O.ilu0(rp, col, val) if pc == "ilu" else O.ic0(rp, col, val)
+    ref, tmp = np.empty(n), np.empty(n)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    O.lib().or_precond_apply.argtypes = [C.c_int, C.c_int] + [C.c_void_p] * 7
+    O.lib().or_precond_apply(O.PRECOND[pc], n, p(rp), p(col), p(f), None, p(src), p(ref), p(tmp))
+    assert rel_err(dst.cpu().numpy(), ref) < 1e-12
