@@ -20,7 +20,7 @@
 //
 // Rows are taken in slices of 32 by warps (slice i of the SpMV, and of each group of a sweep, by
 // warp i mod kHaloWarps).  A slice's entries, entry k of its rows side by side, lie in items of
-// at most KC entry rows, and a warp's items lie in the order in which it uses them (forward
+// at most kHaloItem entry rows, and a warp's items lie in the order in which it uses them (forward
 // sweep, backward sweep, SpMV).  A sweep slice's first entry row holds the inverse pivots and, as
 // columns, the rows themselves.  Two forms (RES): a part whose values and columns fit in shared
 // memory beside its vectors (up to ~900 rows of a triangular mesh) loads them once, by bulk
