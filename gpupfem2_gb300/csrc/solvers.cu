@@ -16,7 +16,6 @@
 #include <exception>
 #include <functional>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <cmath>
 #include <cstring>
@@ -3112,7 +3111,7 @@ struct GraphCut {
         if (threads > 1 && hi - lo >= 4096) {
             try {
                 other = std::thread([=] { cut(mid, hi, P - P1, first + P1, threads / 2); });
-            } catch (const std::system_error&) {}  // no thread to be had
+            } catch (...) {}  // no thread to be had
         }
         cut(lo, mid, P1, first, threads / 2);
         if (other.joinable()) other.join();
@@ -3142,7 +3141,7 @@ static void parallel_ranges(int n, int workers, F&& f) {
     int w = 0;
     try {
         for (; w + 1 < workers; ++w) t.emplace_back(run, w);
-    } catch (const std::system_error&) {}
+    } catch (...) {}  // no thread to be had
     for (; w < workers; ++w) run(w);
     for (std::thread& x : t) x.join();
     for (const std::exception_ptr& e : err)
