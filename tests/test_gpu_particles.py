@@ -116,3 +116,40 @@ def test_capacity_overflow_is_reported(cuda):
     with pytest.raises(g.Pf2Error) as e:
         ph.upload(big)
     assert e.value.status == g.OVERFLOW
+
+
+@pytest.mark.parametrize("level", [1, 2, 3, 4])
+def test_sub_cells_at_their_borders_bitwise(cuda, level):
+    """The occupied sub-cell is found in FP32 where that is certain: particles on the borders between
+    sub-cells, a rounding beside them, and on either side of the band in which the FP64 rule
+    decides (1e-5 in level units), at rest.  Which sub-cells the next sort reseeds, and so every
+    particle, is the oracle's bit for bit."""
+    xy, tri, m = _mesh(64, 32)
+    area, invJ = O.mesh_geometry(xy, tri)
+    off, idx = O.neighbors(xy.shape[0], tri)
+    eps = np.array([0.0, 1e-16, 1e-12, 1e-9, 1e-7, 1e-6, 2.4e-6, 4e-6, 9e-6, 1.1e-5, 3e-5, 1e-4])
+    eps = np.concatenate([eps, -eps[1:]]) / level
+    rng = np.random.default_rng(level)
+    per = 3
+    nc = tri.shape[0]
+    cell = np.repeat(np.arange(nc, dtype=np.int32), per)
+    i, j = rng.integers(0, level + 1, cell.size), rng.integers(0, level + 1, cell.size)
+    a = i / level + rng.choice(eps, cell.size)
+    b = np.where(rng.random(cell.size) < 0.5, j / level + rng.choice(eps, cell.size), rng.random(cell.size))
+    third = rng.random(cell.size) < 0.34  # (the third coordinate on a border instead)
+    b = np.where(third, 1.0 - a - (j / level + rng.choice(eps, cell.size)), b)
+    inside = (a >= 0) & (b >= 0) & (1.0 - a - b >= 0)
+    l0, l1 = np.where(inside, a, 0.3), np.where(inside, b, 0.4)
+    l2 = (1.0 - l0) - l1
+    P = xy[tri[cell]]
+    x = P[:, 0, 0] * l0 + P[:, 1, 0] * l1 + P[:, 2, 0] * l2
+    y = P[:, 0, 1] * l0 + P[:, 1, 1] * l1 + P[:, 2, 1] * l2
+    zero = np.zeros(cell.size)
+    R = dict(x=x, y=y, l0=l0, l1=l1, l2=l2, u=zero, v=zero.copy(), cell=cell)
+    ph = g.ParticleHandler2D(m, level, capacity_factor=6.0)
+    ph.upload(R)
+    still = np.zeros(xy.shape[0])
+    t = torch.zeros(xy.shape[0], dtype=torch.float64, device="cuda")
+    ph.advect(t, t, 0.1, 1)
+    R, _, _ = O.advect(R, xy, tri, invJ, off, idx, still, still, 0.1, 1, level, cap=8 * level * level * nc)
+    _assert_same(ph.download(), R)
