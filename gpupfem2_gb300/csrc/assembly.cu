@@ -1,6 +1,6 @@
 // assembly.cu - finite element assembly of the CSR systems and the Dirichlet rule.
 //
-// Every kernel is row-centric: thread i owns CSR row i, walks the cells around node i
+// Every kernel is row-centric: thread i (Poisson: four lanes) owns CSR row i, walks the cells around node i
 // (ascending cell order, so sums are deterministic), adds row "local vertex of i" of
 // each cell's 3x3 matrix and rhs into a per-thread row buffer, applies the Dirichlet
 // rule to the finished row and writes it once.  No atomics and no clearing pass are

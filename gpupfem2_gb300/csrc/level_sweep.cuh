@@ -20,8 +20,8 @@
 //
 // What bounds it: the chain.  16,705 rows (257 x 65 nodes, 321 levels of ~52 rows): 160 us per
 // ILU(0) iteration, 1,046 with the banded solve; a unit takes ~440 clocks, of which the barrier
-// 43, the ring 30, two late products 128 and, wide meshes, the FP64 pipe (64 clocks per warp
-// instruction, 20 per slice of 32 rows).  Before the three steps were split: 449 (units through a
+// 43, the ring 30 and two late products 128 (64 clocks per FP64 warp instruction); on wide meshes
+// the FP64 pipe.  Before the three steps were split: 449 (units through a
 // bulk-copy ring, two groups; its mbarriers cost ~300 clocks a unit), 328 (loads issued beside the
 // late products), 212 (the generic sums on the path of the common ones).
 #pragma once

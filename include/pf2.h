@@ -306,8 +306,8 @@ typedef struct pf2_solver_options {
     int precision;     /* PF2_PRECISION_* (CG only; MIXED always stops on ||b - A x|| <= tol ||b||) */
     int restart;       /* GMRES Krylov dimension; 0 = max_iterations (no restart, as the reference) */
     int ordering;      /* PF2_ORDERING_* of ILU(0)/IC(0) */
-    int orthogonalization; /* GMRES: PF2_GS_MODIFIED (the reference's, one reduction per basis
-                              vector) or PF2_GS_CLASSICAL_TWICE (two batched reductions) */
+    int orthogonalization; /* GMRES: PF2_GS_MODIFIED (the reference's, its sums in one exchange per
+                              iteration) or PF2_GS_CLASSICAL_TWICE (two batched reductions) */
     int cg_variant;        /* CG: PF2_CG_* */
 } pf2_solver_options;
 

@@ -598,7 +598,7 @@ def _odd_mesh(kind):
     """channel: ordinary levels; box: up to 13 dependencies a row; wide: few levels, of several units; ring: an
     annulus numbered around, whose last rows depend on ones that have left the sweeps' window of
     solved values; hub / star: a last row of 30 / 20 neighbours, solved one after the other / in the
-    two levels before."""
+    two levels before; axis: tetrahedra around an edge, rows of 43 entries."""
     if kind == "channel":
         return mg.channel(64, 16, 4.0, 1.0)
     if kind == "box":
@@ -614,6 +614,12 @@ def _odd_mesh(kind):
         xy = np.stack([np.stack([r * np.cos(t), r * np.sin(t)], 1) for r in (1.0, 1.01)], 1).reshape(-1, 2)
         a, b = 2 * k, 2 * ((k + 1) % n)
         return xy, np.concatenate([np.stack([a, a + 1, b], 1), np.stack([b, a + 1, b + 1], 1)]).astype(np.int32)
+    if kind == "axis":
+        n = 40
+        t = 2 * np.pi * np.arange(n) / n
+        xyz = np.concatenate([np.stack([np.cos(t), np.sin(t), 0 * t], 1), [[0, 0, -1.0], [0, 0, 1.0]]])
+        k = np.arange(n)
+        return xyz, np.stack([np.full(n, n), k, (k + 1) % n, np.full(n, n + 1)], 1).astype(np.int32)
     n = 30 if kind == "hub" else 20
     t = 2 * np.pi * np.arange(n) / n
     xy = np.concatenate([np.stack([np.cos(t), np.sin(t)], 1), np.zeros((1, 2))])
@@ -626,7 +632,7 @@ def _odd_mesh(kind):
 
 
 @pytest.mark.parametrize("pc", ["ic", "ilu"])
-@pytest.mark.parametrize("kind", ["channel", "box", "wide", "ring", "hub", "star"])
+@pytest.mark.parametrize("kind", ["channel", "box", "wide", "ring", "hub", "star", "axis"])
 def test_level_sweeps_match_the_other_solves(cuda, monkeypatch, kind, pc):
     """CG in the natural order with one block's level sweeps (PF2_CG_LEVEL=2) against the banded, slot
     or ticket solve (0).  After 6 iterations only rounding differs: off-diagonal sums within 1/1.05
@@ -634,7 +640,8 @@ def test_level_sweeps_match_the_other_solves(cuda, monkeypatch, kind, pc):
     differ by at most some 6 x 20 operations x 41 x 1.1e-16 = 5.4e-13 relative; 1e-11 allowed.  To
     convergence, the iteration counts agree within one."""
     xy, cells = _odd_mesh(kind)
-    m = (g.Mesh3D if kind == "box" else g.Mesh2D).from_arrays(xy, cells)
+    cells = np.asarray(cells)
+    m = (g.Mesh3D if cells.shape[1] == 4 else g.Mesh2D).from_arrays(xy, cells)
     A = g.SparseMatrixCSR(m)
     rp, col, _ = A.download()
     n = rp.size - 1
@@ -686,7 +693,7 @@ def test_gmres_low_synchronisation_follows_modified_gram_schmidt(cuda, nx, ny, p
 
 
 @pytest.mark.parametrize("pc", ["ic", "ilu"])
-@pytest.mark.parametrize("kind", ["channel", "box", "wide", "ring", "hub", "star"])
+@pytest.mark.parametrize("kind", ["channel", "box", "wide", "ring", "hub", "star", "axis"])
 def test_factors_of_odd_patterns_match_the_oracle(cuda, kind, pc):
     """ILU(0) / IC(0) of a warp per row (rows of up to 32 entries held by its lanes) against the
     oracle's, through one preconditioner apply: the same sums in the same order up to fused
@@ -694,7 +701,8 @@ def test_factors_of_odd_patterns_match_the_oracle(cuda, kind, pc):
     the diagonal amplify rounding by at most ~41 (32 operations a row: 41 x 32 x 1.1e-16 =
     1.4e-13); 1e-12 allowed."""
     xy, cells = _odd_mesh(kind)
-    m = (g.Mesh3D if kind == "box" else g.Mesh2D).from_arrays(xy, cells)
+    cells = np.asarray(cells)
+    m = (g.Mesh3D if cells.shape[1] == 4 else g.Mesh2D).from_arrays(xy, cells)
     A = g.SparseMatrixCSR(m)
     rp, col, _ = A.download()
     n = rp.size - 1
