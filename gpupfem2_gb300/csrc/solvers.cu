@@ -509,6 +509,7 @@ __global__ void k_factor(Tri T, const int* __restrict__ order, unsigned* ticket,
             int ok = 1;
             if (lane == 0) ok = wait_flag(&T.done_f[k], epoch, err, T.rec, i, k);
             if (!__shfl_sync(0xffffffffu, ok, 0)) return;
+            __syncwarp();  // lane 0's wait and fence order the other lanes' loads (a shuffle orders none)
             const double ak = lane < nk ? __ldcg(&a[k0 + lane]) : 0.0;
             const double pivot = __shfl_sync(0xffffffffu, ak, ilu ? 0 : nk - 1);
             double match = 0.0;  // row k's entry in this lane's column

@@ -723,3 +723,20 @@ def test_factors_of_odd_patterns_match_the_oracle(cuda, kind, pc):
     O.lib().or_precond_apply.argtypes = [C.c_int, C.c_int] + [C.c_void_p] * 7
     O.lib().or_precond_apply(O.PRECOND[pc], n, p(rp), p(col), p(f), None, p(src), p(ref), p(tmp))
     assert rel_err(dst.cpu().numpy(), ref) < 1e-12
+
+
+@pytest.mark.parametrize("pc", ["ic", "ilu"])
+@pytest.mark.parametrize("ordering", [0, 1])
+def test_factorisations_are_repeatable_bit_for_bit(cuda, pc, ordering):
+    """Rows of a factorisation wait for the rows that they depend on and then read them with all lanes of
+    a warp: whatever the order in which rows finish, every factorisation gives the same bits
+    (compared through one preconditioner apply; 64 of them on 4,257 rows in 160 levels, or in
+    a few colours)."""
+    m, A, rp, col, val, rhs = _system(128, 32)
+    src = torch.tensor(np.sin(1.0 + np.arange(rp.size - 1)), device="cuda")
+    s = g.LinearSolver(A, "cg", pc, ordering=ordering)
+    first, dst = torch.empty_like(src), torch.empty_like(src)
+    for k in range(64):
+        s.setup(A)
+        s.apply_preconditioner(dst if k else first, src)
+        assert k == 0 or torch.equal(dst.view(torch.int64), first.view(torch.int64))
