@@ -166,13 +166,11 @@ __global__ void k_poisson(int nv, RowMesh M, int kind, double lambda, double* __
 // nodal field needs its differences to node m only, and a row's diagonal entry of every
 // gradient term is minus the sum of the others.
 //
-// The kernels below are bound by FP64 issue (64 clocks per warp instruction on an SM
+// k_prediction and k_correction are bound by FP64 issue (64 clocks per warp instruction on an SM
 // sub-partition), and each of a cell's rows computes the cell's terms anew.  So sums over j come
 // first (gradients of u and p once per cell, mass on neighbours as one sum, factors common to a
 // row and diagonals at its end).  499,288 nodes, matrix and right-hand side, FP64 pipe 80 % busy:
-// k_prediction 514 -> 334 us, k_pressure 165 -> 147, k_correction 225 -> 133.  Differences to node m
-// also round less: the pressure of the quarter-size cylinder's first step agrees with the oracle's
-// to 6.5e-13 instead of 2.6e-12.
+// k_prediction 514 -> 334 us, k_correction 225 -> 133.
 struct CellAt {
     double2 g, gj, gk;
     int j, k, p, pj, pk;
@@ -307,6 +305,13 @@ __global__ void k_prediction(bool matrix, int nv, RowMesh M, FlowCoef P, const d
 }
 
 // kIntegratePressureEquation, cases/Cylinder2D/main.cu:169-211
+//
+// Every entry, the diagonal too, adds its cells' terms in ascending order, as K = fma(gx_i, gx_j,
+// gy_i gy_j) and fma(K, area, v); the right-hand side takes K p from the same terms.  Sums by CellAt
+// would cost 147 instead of 165 us (499,288 nodes) and are not taken: other roundings of the matrix
+// stop the mixed-precision solve elsewhere (its answer moved by 1.9e-9), and with rows that do
+// not add up to zero alike, differences in the right-hand side lose what they gain (pressure of the
+// quarter-size cylinder's first step against the oracle's: 4.1e-12, 2.1e-12 as it is).
 __global__ void k_pressure(bool matrix, int nv, RowMesh M, FlowCoef P, const double* __restrict__ px,
                            const double* __restrict__ py, const double* __restrict__ pold, double* __restrict__ val,
                            double* __restrict__ rhs, BcView bc) {
@@ -314,34 +319,28 @@ __global__ void k_pressure(bool matrix, int nv, RowMesh M, FlowCoef P, const dou
     if (i >= nv) return;
     const int s = M.rowptr[i], len = M.rowptr[i + 1] - s;
     if (boundary_row(i, s, len, M.col, val, rhs, bc, matrix)) return;
-    const bool need = matrix || has_bc_column(i, s, len, M.col, bc), entries = need || pold;
+    const bool need = matrix || has_bc_column(i, s, len, M.col, bc);
     double v[kMaxRow];
-    if (entries)
+    if (need)
         for (int k = 0; k < len; ++k) v[k] = 0.0;
     double r = 0.0;
-    const double pxi = px[i], pyi = py[i];
-    int diag = 0;
+    const double fdiv = -P.rho / P.dt / 3.0;
     for (int q = M.inc_off[i]; q < M.inc_off[i + 1]; ++q) {
         const int e = M.inc[q], c = e >> 2, m = e & 3, pos = M.inc_pos[q];
         const double A = M.area[c];
-        const CellAt C = cell_at(M.invJ[c], M.tri4[c], m, pos);
-        diag = C.p;
-        if (entries) {
-            const double ax = A * C.g.x, ay = A * C.g.y;
-            v[C.pj] = fma(ax, C.gj.x, fma(ay, C.gj.y, v[C.pj]));
-            v[C.pk] = fma(ax, C.gk.x, fma(ay, C.gk.y, v[C.pk]));
+        double2 g[3];
+        shape_grads(M.invJ[c], g);
+        const int4 t = M.tri4[c];
+        double cr = 0.0, div = 0.0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int nj = vtx(t, j), p = (pos >> (10 * j)) & 1023;
+            const double K = g[m].x * g[j].x + g[m].y * g[j].y;
+            if (need) v[p] += K * A;
+            if (pold) cr += K * pold[nj];
+            div += g[j].x * px[nj] + g[j].y * py[nj];
         }
-        const double div = fma(C.gj.x, px[C.j] - pxi, fma(C.gk.x, px[C.k] - pxi,
-                           fma(C.gj.y, py[C.j] - pyi, C.gk.y * (py[C.k] - pyi))));
-        r = fma(A, div, r);
-    }
-    r *= -P.rho / P.dt / 3.0;
-    if (entries) {
-        v[diag] = -others(v, len, diag);
-        if (pold) {
-            const double pi = pold[i];
-            for (int k = 0; k < len; ++k) r = fma(v[k], pold[M.col[s + k]] - pi, r);
-        }
+        r += (cr + fdiv * div) * A;
     }
     if (need) eliminate_row(i, s, len, M.col, v, r, bc);
     if (matrix)

@@ -1,5 +1,7 @@
 """Whole PFEM-2 steps (cases/Cylinder2D/main.cu:793-880) on the GPU against the oracle,
 and the flow systems' assembly kernels one by one."""
+from fractions import Fraction
+
 import numpy as np
 import pytest
 import torch
@@ -216,3 +218,33 @@ def test_particles_reserve_keeps_the_particles(cuda):
     after = h.download()
     for k in before:
         assert np.array_equal(before[k], after[k]), k
+
+
+@pytest.mark.parametrize("pold", [False, True])
+def test_pressure_matrix_bits(cuda, pold):
+    """The pressure matrix bit for bit: row i adds, cell by cell in ascending order, fma(K, area, v)
+    with K = fma(gx_i, gx_j, gy_i gy_j), the diagonal entry among them.  (An iteration on the
+    matrix rounded to FP32 stops at another place for every rounding of it: with a diagonal formed
+    as minus the sum of the others the mixed pressure solve's answer moved by 1.9e-9.)"""
+    def fma(a, b, c):
+        return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+    xy, tri = mg.cylinder_channel(nxh=24, nyh=24, nr=2)
+    m = g.Mesh2D.from_arrays(xy, tri)
+    area, invJ = O.mesh_geometry(xy, tri)
+    rp, col = O.csr_structure(xy.shape[0], tri)
+    ref = np.zeros(col.size)
+    for c, t in enumerate(np.asarray(tri)):
+        d = [float(v) for v in np.asarray(invJ)[c].reshape(-1)]
+        gr = [(d[0], d[2]), (d[1], d[3]), (-d[0] - d[1], -d[2] - d[3])]
+        for i in range(3):
+            for j in range(3):
+                K = fma(gr[i][0], gr[j][0], gr[i][1] * gr[j][1])
+                at = rp[t[i]] + np.searchsorted(col[rp[t[i]]:rp[t[i] + 1]], t[j])
+                ref[at] = fma(K, float(area[c]), float(ref[at]))
+    n = xy.shape[0]
+    v = [torch.tensor(mg.uniform_pm1(k, n), device="cuda") for k in range(3)]
+    A, b = g.SparseMatrixCSR(m), torch.empty(n, dtype=torch.float64, device="cuda")
+    g.assemble_pressure(m, g.default_params(), v[0], v[1], v[2] if pold else None, A, b)
+    val = A.download()[2]
+    assert np.array_equal(val.view(np.int64), ref.view(np.int64))
