@@ -4379,6 +4379,19 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     return PF2_OK;
 }
 
+// Lets fn take all the dynamic shared memory that a block can have.  The limit belongs to the
+// function, for all solvers of the process: one set to what a solver needs would refuse the launches
+// of every larger solver that is alive.
+static pf2_status allow_smem(void* fn) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes at;
+    PF2_CUDA(cudaGetDevice(&dev));
+    PF2_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    PF2_CUDA(cudaFuncGetAttributes(&at, fn));
+    PF2_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes));
+    return PF2_OK;
+}
+
 // The partitioned CG plan of a Jacobi / no-preconditioner solve: B = A, one group.
 static pf2_status build_part_plan_local(pf2_solver* S) {
     const pf2_mesh* M = S->mesh;
@@ -4459,9 +4472,8 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
     if (S->part) {
         int occ_p = 0;
         void* pf = part_kernel(S);
-        if (cudaFuncSetAttribute(pf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->part_smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, pf, part_threads(S),
-                                                          S->part_smem) != cudaSuccess)
+        if ((s = allow_smem(pf))) return fail(s);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, pf, part_threads(S), S->part_smem) != cudaSuccess)
             return fail(cuda_fail(cudaGetLastError(), "partitioned CG attributes", __FILE__, __LINE__));
         if (occ_p < 1) {  // the other kernels then
             S->part = false;
@@ -4476,26 +4488,16 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
             return fail(PF2_BAD_INPUT);
         }
     if (S->level) {
-        if (cudaFuncSetAttribute((void*)k_pcg_level, cudaFuncAttributeMaxDynamicSharedMemorySize, kLevelSmem) != cudaSuccess)
-            return fail(cuda_fail(cudaGetLastError(), "level sweep attributes", __FILE__, __LINE__));
+        if ((s = allow_smem((void*)k_pcg_level))) return fail(s);
         S->level_blocks = std::max(1, std::min(num_sms(), (S->n + kLevelThreads - 1) / kLevelThreads));
     }
     // the banded triangular solve keeps a range of the solution in shared memory
     S->smem = S->band_P ? sizeof(double) * (size_t)S->band_R : 0;
     void* fn = solve_kernel(*opt, S->csr);
-    if (S->smem) {
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem) != cudaSuccess ||
-            cudaFuncSetAttribute((void*)k_precond_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)S->smem) != cudaSuccess)
-            return fail(cuda_fail(cudaGetLastError(), "shared-memory attribute", __FILE__, __LINE__));
-    }
     const bool mgs = fn == (void*)k_gmres_mgs;
-    if (mgs) {
-        S->extra_smem = kGramBytes;
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(double) * kBandRows + kGramBytes)) != cudaSuccess)
-            return fail(cuda_fail(cudaGetLastError(), "shared-memory attribute", __FILE__, __LINE__));
-    }
+    if (mgs) S->extra_smem = kGramBytes;
+    if (S->smem + S->extra_smem && (s = allow_smem(fn))) return fail(s);
+    if (S->smem && (s = allow_smem((void*)k_precond_apply))) return fail(s);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kSolverThreads, S->smem + S->extra_smem) != cudaSuccess ||
         occ < 1)
         return fail(cuda_fail(cudaGetLastError(), "occupancy query", __FILE__, __LINE__));

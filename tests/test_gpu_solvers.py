@@ -740,3 +740,34 @@ def test_factorisations_are_repeatable_bit_for_bit(cuda, pc, ordering):
         s.setup(A)
         s.apply_preconditioner(dst if k else first, src)
         assert k == 0 or torch.equal(dst.view(torch.int64), first.view(torch.int64))
+
+
+@pytest.mark.parametrize("kind,pc,ordering,precision,gs,level", [
+    ("cg", "jacobi", 0, 0, 0, None), ("cg", "none", 0, 0, 0, None), ("cg", "ic", 1, 0, 0, None),
+    ("cg", "ilu", 1, 0, 0, None), ("cg", "ic", 1, 1, 0, None), ("cg", "ilu", 1, 1, 0, None),
+    ("cg", "ic", 0, 0, 0, None), ("cg", "ic", 0, 0, 0, "0"), ("cg", "ilu", 0, 1, 0, "0"),
+    ("gmres", "ilu", 0, 0, 0, None), ("gmres", "ilu", 0, 0, 1, None)])
+def test_a_smaller_solver_leaves_a_larger_one_alone(cuda, monkeypatch, kind, pc, ordering, precision, gs, level):
+    """Two solvers of the same kernel alive at once, the smaller created last: the larger one still
+    solves, to the bits it gave before, and its preconditioner applies.  (How much shared memory a
+    kernel may take is a property of the kernel, not of a solver.)"""
+    if level is not None:
+        monkeypatch.setenv("PF2_CG_LEVEL", level)
+    systems = [_system(256, 64), _system(32, 16)]
+    mk = lambda A: g.LinearSolver(A, kind, pc, tol=1e-6, maxit=2000, ordering=ordering, precision=precision,  # noqa: E731
+                                  orthogonalization=gs, criterion=g.CRITERION_REL if kind == "cg" else 0)
+
+    def solve(s, system):
+        A, b = system[1], torch.tensor(system[5], device="cuda")
+        x, z = torch.zeros_like(b), torch.empty_like(b)
+        assert s.solve(A, x, b).converged == 1
+        s.apply_preconditioner(z, b)
+        return x, z
+
+    large = mk(systems[0][1])
+    before = solve(large, systems[0])
+    small = mk(systems[1][1])
+    solve(small, systems[1])
+    after = solve(large, systems[0])
+    for u, v in zip(before, after):
+        assert torch.equal(u.view(torch.int64), v.view(torch.int64))
