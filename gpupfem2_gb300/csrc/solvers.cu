@@ -3753,6 +3753,41 @@ static pf2_status build_level_plan(pf2_solver* S, const std::vector<int> (&level
     return PF2_OK;
 }
 
+// Whether one block's level sweeps are faster than the kernels that share the triangles among all
+// SMs: a question of rows per level, since one SM works through a level alone while each level
+// costs the others ~20 us and more (9 where a numbering by colours puts it side by side).
+// Dependencies that have left the ring are read through L2, one after another, and rows of more than
+// kBandMaxDeps of them wait for each.  us per IC(0) iteration, the kernel on B's CSR arrays (under 128
+// levels) or the banded or ticket solve -> level sweeps; far: dependencies outside the ring:
+//   a mesher's sweep over the mesh (none far): triangles 4,257 rows 434 -> 80, 16,705 rows 1,033 ->
+//     143, 125,479 rows 7,977 -> 859, 500,157 rows 50,387 -> 3,091; tetrahedra 9,471 rows 3,676 -> 128,
+//     211,191 rows (1,106 a level) 11,752 -> 1,747
+//   numbered by colours (4 levels): 536 rows a level 36 -> 35, 1,046 39 -> 47, 3,937 37 -> 102,
+//     125,039 62 -> 7,093
+//   few far: shuffled triangles, 1,193 a level 287 -> 137; nested dissection, 1,719 a level (3.5 % far)
+//     46,198 -> 10,812; shuffled tetrahedra, 659 a level (2.7 %) 632 -> 478
+//   many far, triangles: 497 a level (12 %) 2,191 -> 1,319, 1,126 (16 %) 588 -> 533, 1,257 (22 %)
+//     601 -> 723, 27,786 (shuffled, 500,157 rows) 1,351 -> 14,745
+//   many far, tetrahedra: 313 a level (28 %) 2,482 -> 2,207, 417 (17 %) 10,638 -> 18,479, 1,281 (35 %)
+//     649 -> 1,374, 6,212 (83 %) 2,460 -> 12,278
+template <class Deps>
+static bool level_sweeps_pay(int n, int K, int levels, const std::vector<int> (&order)[2], Deps&& deps) {
+    const int rows = n / std::max(levels, 1);
+    if (levels < 10) return rows <= 256;
+    if (rows <= 400 || rows > 2048) return rows <= 400;
+    std::vector<int> pos(n);
+    long long far = 0, all = 0;
+    for (int dir = 0; dir < 2; ++dir) {
+        for (int q = 0; q < n; ++q) pos[order[dir][q]] = q;
+        for (int i = 0; i < n; ++i)
+            deps(dir, i, [&](int j, int) {
+                far += pos[i] - pos[j] > kLevelRing - 32 * kLevelSlices;
+                ++all;
+            });
+    }
+    return far <= all / 10 || (K <= kBandMaxDeps && rows <= 1000);
+}
+
 static pf2_status build_tri_plan(pf2_solver* S) {
     const pf2_mesh* M = S->mesh;
     const int n = M->nv, nnz = M->nnz;
@@ -3897,18 +3932,16 @@ static pf2_status build_tri_plan(pf2_solver* S) {
     // CG with few levels: the whole iteration on B's CSR arrays (pcg_csr, pcg_csr_mixed)
     S->csr = std::max(S->levels_fwd, S->levels_bwd) < band_min && S->opt.kind == PF2_SOLVER_CG;
     if (const char* e = getenv("PF2_CG_SLOTS")) S->csr = S->csr && atoi(e) == 0;  // tuning: keep the slot sweeps
-    // FP64 CG in the natural order, or on any order with long chains: one block's level sweeps.
-    // us per IC(0) iteration, the banded, slot or ticket solve -> level sweeps:
-    //   triangles   4,355 rows 375 -> 68; 16,705 rows 1,040 -> 152; 36,042 rows 2,181 -> 294;
-    //               125,364 rows 8,927 -> 1,008; 499,288 rows 53,594 -> 4,241
-    //   tetrahedra  1,617 rows 2,109 -> 54; 9,471 rows 3,730 -> 131; 77,531 rows 2,997 -> 684;
-    //               251,991 rows 15,972 -> 2,095
-    // The other CG variants keep their kernels.  PF2_CG_LEVEL=0, or an override of the banded or slot
-    // solve, keeps those (tests and tuning); PF2_CG_LEVEL=2 (tests) requires the level sweeps.
+    // FP64 CG in the natural order: one block's level sweeps, where level_sweeps_pay.  Few levels:
+    // the standard variant (the other variants have their kernels on B's CSR arrays); 128 levels
+    // and more: every variant (all run the standard iteration there).  PF2_CG_LEVEL=0, or an override of
+    // the banded or slot solve, keeps the other kernels (tests and tuning); PF2_CG_LEVEL=2 (tests)
+    // requires the level sweeps, wherever they pay.
     const char* le = getenv("PF2_CG_LEVEL");
     const bool want = le ? atoi(le) != 0 : !getenv("PF2_BAND_ROWS") && !getenv("PF2_BAND_MIN_LEVELS") && !getenv("PF2_CG_SLOTS");
     if (want && S->opt.kind == PF2_SOLVER_CG && S->opt.precision == PF2_PRECISION_FP64 &&
-        (S->csr ? S->opt.ordering == PF2_ORDERING_NATURAL && S->opt.cg_variant == PF2_CG_STANDARD : banded || K > kBandMaxDeps))
+        (S->csr ? S->opt.ordering == PF2_ORDERING_NATURAL && S->opt.cg_variant == PF2_CG_STANDARD : banded || K > kBandMaxDeps) &&
+        ((le && atoi(le) == 2) || level_sweeps_pay(n, K, std::max(S->levels_fwd, S->levels_bwd), level_order, deps)))
         PF2_TRY(build_level_plan(S, level, level_order, bdiag, perm, ic, deps));
     if (le && atoi(le) == 2 && !S->level) {
         set_error("the level sweeps do not apply");

@@ -771,3 +771,53 @@ def test_a_smaller_solver_leaves_a_larger_one_alone(cuda, monkeypatch, kind, pc,
     after = solve(large, systems[0])
     for u, v in zip(before, after):
         assert torch.equal(u.view(torch.int64), v.view(torch.int64))
+
+
+def _numbered(xy, cells, key):
+    order = np.argsort(key, kind="stable")
+    return np.asarray(xy)[order], np.argsort(order)[np.asarray(cells)].astype(np.int32)
+
+
+@pytest.mark.parametrize("kind,sweeps", [("own", True), ("shuffled small", True), ("coloured", False),
+                                         ("shuffled", False), ("tetrahedra", True), ("shuffled tetrahedra", False)])
+def test_wide_levels_keep_the_solve_on_all_sms(cuda, monkeypatch, kind, sweeps):
+    """CG with IC(0) in the natural order takes one block's level sweeps where levels are narrow, and the
+    kernels that share the triangles among all SMs where they are wide (a mesh numbered by colours, or
+    without any order): bit for bit the iterates of the forced kernel, which differ between the two."""
+    rng = np.random.default_rng(5)
+    if "tetrahedra" in kind:
+        xy, cells = mg.box_tets(*((20, 10, 8) if kind == "tetrahedra" else (60, 30, 20)))
+    else:
+        xy, cells = mg.channel(*{"coloured": (180, 86), "shuffled": (400, 120)}.get(kind, (64, 16)), 4.0, 1.0)
+    if "shuffled" in kind:
+        xy, cells = _numbered(xy, cells, rng.random(len(xy)))
+    M = g.Mesh3D if np.asarray(cells).shape[1] == 4 else g.Mesh2D
+    if kind == "coloured":
+        rp, col, _ = g.SparseMatrixCSR(M.from_arrays(xy, cells)).download()
+        colour = []
+        for i in range(rp.size - 1):
+            used = {colour[j] for j in col[rp[i]:rp[i + 1]] if j < i}
+            colour.append(next(c for c in range(len(used) + 1) if c not in used))
+        xy, cells = _numbered(xy, cells, np.array(colour))
+    m = M.from_arrays(xy, cells)
+    A = g.SparseMatrixCSR(m)
+    rp, col, _ = A.download()
+    n = rp.size - 1
+    row = np.repeat(np.arange(n), np.diff(rp))
+    val = np.where(row == col, 0.0, -1.0 - 0.3 * np.cos(row + col.astype(np.float64)))
+    sums = np.zeros(n)
+    np.add.at(sums, row, -val)
+    val[row == col] = 1.05 * sums
+    A.upload_values(val)
+    b = torch.tensor(np.sin(1.0 + np.arange(n)), device="cuda")
+    out = {}
+    for level in ("2", "0", None):
+        if level is None:
+            monkeypatch.delenv("PF2_CG_LEVEL")
+        else:
+            monkeypatch.setenv("PF2_CG_LEVEL", level)
+        x = torch.zeros_like(b)
+        g.LinearSolver(A, "cg", "ic", tol=0.0, maxit=6, criterion=g.CRITERION_REL).solve(A, x, b, check=False)
+        out[level] = x.view(torch.int64)
+    assert not torch.equal(out["2"], out["0"])
+    assert torch.equal(out[None], out["2" if sweeps else "0"])
