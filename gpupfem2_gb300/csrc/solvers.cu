@@ -3193,12 +3193,12 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
     };
     std::vector<Halo> H(P);
     std::vector<int> rl(workers, 0);
-    std::atomic<bool> too_many{ false };
+    std::atomic<bool> too_many{ false }, too_large{ false };
     parallel_ranges(P, workers, [&](int worker, int k0, int k1) {
         std::vector<int> stamp(n, -1);  // cls: the row's membership in the halo of part stamp
         std::vector<unsigned char> cls(n, 0);
         std::vector<std::vector<int>> bucket(ng);
-        for (int k = k0; k < k1 && !too_many; ++k) {
+        for (int k = k0; k < k1 && !too_many && !too_large; ++k) {
             Halo& h = H[k];
             const int p0 = qs[(size_t)k * ng], np = qs[(size_t)(k + 1) * ng] - p0;
             // ring 1, the F rows among it (read by an own row's lower entries) and the closures
@@ -3239,7 +3239,7 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
                     }
             }
             if (nh > std::max(4 * np, 64) || np + nh >= kHaloMaxLocal) {
-                too_many = true;
+                (np + nh >= kHaloMaxLocal ? too_large : too_many) = true;
                 return;
             }
             rl[worker] = std::max(rl[worker], np + nh);
@@ -3269,8 +3269,8 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
             }
         }
     });
-    if (too_many) {
-        S->part_why = "the halo rows outnumber a part's rows";
+    if (too_many || too_large) {
+        S->part_why = too_large ? "a part and its halo are too many rows" : "the halo rows outnumber a part's rows";
         return PF2_OK;
     }
     const int RL = *std::max_element(rl.begin(), rl.end());
@@ -4513,13 +4513,20 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
             S->part_why = "no block of the partitioned kernel fits on an SM";
         }
     }
-    // PF2_CG_PART=2 (tests): require the partitioned kernel
-    if (const char* e = getenv("PF2_CG_PART"))
-        if (atoi(e) == 2 && !S->part) {
+    // tests: PF2_CG_PART=2 requires a partitioned kernel, 4 the one with halo rows, its entries
+    // resident in shared memory (PF2_HALO_RESIDENT=1) or read from L2 (0)
+    if (const char* e = getenv("PF2_CG_PART")) {
+        const char* res = getenv("PF2_HALO_RESIDENT");
+        if ((atoi(e) == 2 && !S->part) || (atoi(e) == 4 && !(S->part && S->halo))) {
             set_error("the partitioned CG kernel does not apply: %s", part_eligible(S) ? S->part_why :
                       "solver kind, variant, precision or preconditioner");
             return fail(PF2_BAD_INPUT);
         }
+        if (atoi(e) == 4 && res && S->halo_res != (atoi(res) != 0)) {
+            set_error("a part's entries do not fit in the shared memory of a block");
+            return fail(PF2_BAD_INPUT);
+        }
+    }
     if (S->level) {
         if ((s = allow_smem((void*)k_pcg_level))) return fail(s);
         S->level_blocks = std::max(1, std::min(num_sms(), (S->n + kLevelThreads - 1) / kLevelThreads));

@@ -821,3 +821,62 @@ def test_wide_levels_keep_the_solve_on_all_sms(cuda, monkeypatch, kind, sweeps):
         out[level] = x.view(torch.int64)
     assert not torch.equal(out["2"], out["0"])
     assert torch.equal(out[None], out["2" if sweeps else "0"])
+
+
+@pytest.mark.parametrize("pc,precision", [("none", 0), ("jacobi", 0), ("ic", 0), ("ilu", 0), ("ic", 1), ("ilu", 1)])
+@pytest.mark.parametrize("parts,resident", [("1", "0"), ("2", "1"), ("7", "1"), ("23", "1"), ("70", "1"), ("7", "0")])
+def test_the_halo_form_is_the_one_compared(cuda, monkeypatch, pc, precision, parts, resident):
+    """The systems and parts of the comparison with the waiting sweeps are solved by the kernel with
+    halo rows, with resident entries or (one part of 2,193 rows, or where asked) with entries read from
+    L2: creation that requires it (PF2_CG_PART=4) succeeds, and its solve gives the bits of the one
+    that requires some partitioned kernel (2)."""
+    m, A, rp, col, val, rhs = _system(128, 16)
+    b = torch.tensor(rhs, device="cuda")
+    monkeypatch.setenv("PF2_CG_PARTS", parts)
+    monkeypatch.setenv("PF2_HALO_RESIDENT", resident)
+    out = []
+    for part in ("4", "2"):
+        monkeypatch.setenv("PF2_CG_PART", part)
+        x = torch.zeros_like(b)
+        s = g.LinearSolver(A, "cg", pc, ordering=1 if pc in ("ic", "ilu") else 0, precision=precision,
+                           tol=1e-8 if precision else 1e-12, maxit=5000, criterion=g.CRITERION_REL)
+        assert s.solve(A, x, b).converged == 1
+        out.append(x.view(torch.int64))
+    assert torch.equal(*out)
+
+
+def test_requiring_the_halo_form_where_it_does_not_apply_is_refused(cuda, monkeypatch):
+    """Parts of a dozen rows of a tetrahedral mesh in eight colours, whose halos are many times as large,
+    and a solver kind that has no parts."""
+    m = g.Mesh3D.from_arrays(*mg.box_tets(12, 10, 8))
+    A = g.SparseMatrixCSR(m)
+    monkeypatch.setenv("PF2_CG_PART", "4")
+    monkeypatch.setenv("PF2_CG_PARTS", "100")
+    for kind in ("cg", "gmres"):
+        with pytest.raises(g.Pf2Error) as e:
+            g.LinearSolver(A, kind, "ic", ordering=1)
+        assert e.value.status == g.BAD_INPUT
+    monkeypatch.setenv("PF2_CG_PART", "2")
+    g.LinearSolver(A, "cg", "ic", ordering=1)
+
+
+@pytest.mark.parametrize("kind,pc", [("gmres", "jacobi"), ("gmres", "ilu"), ("cg", "ic")])
+def test_waits_of_gmres_and_of_the_level_sweeps_that_run_out_return_timeout(cuda, monkeypatch, kind, pc):
+    """As above for the exchanges of GMRES with modified Gram-Schmidt and for the blocks that wait for the
+    level sweeps: one poll is not enough, the solve returns PF2_TIMEOUT, and the next solver works."""
+    m, A, rp, col, val, rhs = _system(128, 32)
+    b = torch.tensor(rhs, device="cuda")
+    if kind == "cg":
+        monkeypatch.setenv("PF2_CG_LEVEL", "2")
+    monkeypatch.setenv("PF2_BARRIER_POLLS", "1")
+    s = g.LinearSolver(A, kind, pc, tol=1e-8, maxit=1000)
+    monkeypatch.delenv("PF2_BARRIER_POLLS")
+    with pytest.raises(g.Pf2Error) as e:
+        s.solve(A, torch.zeros_like(b), b)
+    assert e.value.status == g.TIMEOUT
+    torch.cuda.synchronize()  # the context is still usable
+    x = torch.zeros_like(b)
+    info = g.LinearSolver(A, kind, pc, tol=1e-8, maxit=1000).solve(A, x, b)
+    assert info.converged == 1 and info.status == 0
+    ox, _ = O.pcg(rp, col, val, rhs, tol=1e-10, maxit=1000, precond="jacobi")
+    assert rel_err(x.cpu().numpy(), ox) < 1e-6
