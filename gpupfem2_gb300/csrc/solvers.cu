@@ -3157,8 +3157,11 @@ static void parallel_ranges(int n, int workers, F&& f) {
 // depend on one another, or a part too large for the shared-memory vectors.
 // Rows per part at least: fewer rows share less FP64 work per SM but more halo and more blocks
 // in a reduction.  Measured, us per IC(0) iteration at 512 / 256 / 170 / 128 rows: 4,355 rows
-// 12.7 / 10.9 / 10.7 / 10.5, 16,705 rows 13.1 / 11.5 / 11.2 / 11.4.
-constexpr int kPartMinRows = 170;
+// 12.7 / 10.9 / 10.7 / 10.5, 16,705 rows 13.1 / 11.5 / 11.2 / 11.4.  With many groups (the eight
+// colours of a tetrahedral mesh) parts of 170 rows have more halo than the halo form takes, and the
+// form with waits gains nothing from small parts: at 512 rows 9,471 nodes in 3D take 28.2 us (halo),
+// with waits at 170 / 512 rows 75.8 / 74.2 (mixed 74.5 / 67.8), 19,125 nodes 76.6 / 76.2 (78.9 / 74.9).
+constexpr int kPartMinRows = 170, kPartMinRowsWaits = 512, kPartFewGroups = 6;
 constexpr int kHaloFactor = 1 << 30;  // flag of a factor value in the streams' value map
 
 // The halo form of the plan (part_halo.cuh) on the parts and the order Q of build_part_plan
@@ -3504,38 +3507,46 @@ static pf2_status build_part_plan(pf2_solver* S, const std::vector<int>& rp, con
                     S->part_why = "a sweep group's rows depend on one another";
                     return PF2_OK;
                 }
-    int P = std::max(1, std::min(num_sms(), n / kPartMinRows));
-    if (const char* e = getenv("PF2_CG_PARTS")) P = std::max(1, std::min(num_sms(), atoi(e)));  // tests, tuning
-    std::vector<int> part;
-    graph_parts(n, rp, col, P, part);
-    // boundary rows (a neighbour in another part), in A's numbering
-    std::vector<unsigned char> bnd_a(n, 0);
-    for (int i = 0; i < n; ++i)
-        for (int k = rp[i]; k < rp[i + 1]; ++k)
-            if (part[col[k]] != part[i]) bnd_a[i] = 1;
-    // Q: by part, then group, then the group's boundary rows before its interior rows (the
-    // threads that wait on other parts' values share warps with as few others as possible),
-    // then B's order
-    std::vector<int> cls((size_t)P * ng * 2 + 1, 0);
-    auto cell = [&](int r) { return ((size_t)part[perm[r]] * ng + grp[r]) * 2 + (bnd_a[perm[r]] ? 0 : 1); };
-    for (int r = 0; r < n; ++r) cls[cell(r) + 1]++;
-    for (size_t c = 0; c + 1 < cls.size(); ++c) cls[c + 1] += cls[c];
-    std::vector<int> qs((size_t)P * ng + 1);
-    for (size_t c = 0; c < qs.size(); ++c) qs[c] = cls[2 * c];
-    std::vector<int> fill(cls.begin(), cls.end() - 1), bq(n), qa(n), qb(n);
-    for (int r = 0; r < n; ++r) {
-        const int q = fill[cell(r)]++;
-        bq[r] = q;
-        qb[q] = r;
-        qa[q] = perm[r];
-    }
-    int R = 0;
-    for (int p = 0; p < P; ++p) R = std::max(R, qs[(size_t)(p + 1) * ng] - qs[(size_t)p * ng]);
     int optin = 0;
     PF2_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
     const bool mixed = S->opt.precision == PF2_PRECISION_MIXED;
-    PF2_TRY(build_halo_plan(S, brp, bcol, bmap, bdiag, perm, part, grp, qs, bq, qb, qa, P, ng, R, optin, tri, mixed));
-    if (S->halo) return PF2_OK;
+    const char* parts = getenv("PF2_CG_PARTS");  // tests, tuning
+    int P = 0, R = 0;
+    std::vector<int> part, qs, bq(n), qa(n), qb(n);
+    // the halo form on the smallest parts first; where it is refused, cut again, and the form with
+    // waits takes the last cut
+    for (int rows : { kPartMinRows, kPartMinRowsWaits }) {
+        if (rows == kPartMinRows && ng > kPartFewGroups) continue;
+        const int cut = std::max(1, std::min(num_sms(), parts ? atoi(parts) : n / rows));
+        if (cut == P) break;
+        P = cut;
+        graph_parts(n, rp, col, P, part);
+        // boundary rows (a neighbour in another part), in A's numbering
+        std::vector<unsigned char> bnd_a(n, 0);
+        for (int i = 0; i < n; ++i)
+            for (int k = rp[i]; k < rp[i + 1]; ++k)
+                if (part[col[k]] != part[i]) bnd_a[i] = 1;
+        // Q: by part, then group, then the group's boundary rows before its interior rows (the
+        // threads that wait on other parts' values share warps with as few others as possible),
+        // then B's order
+        std::vector<int> cls((size_t)P * ng * 2 + 1, 0);
+        auto cell = [&](int r) { return ((size_t)part[perm[r]] * ng + grp[r]) * 2 + (bnd_a[perm[r]] ? 0 : 1); };
+        for (int r = 0; r < n; ++r) cls[cell(r) + 1]++;
+        for (size_t c = 0; c + 1 < cls.size(); ++c) cls[c + 1] += cls[c];
+        qs.resize((size_t)P * ng + 1);
+        for (size_t c = 0; c < qs.size(); ++c) qs[c] = cls[2 * c];
+        std::vector<int> fill(cls.begin(), cls.end() - 1);
+        for (int r = 0; r < n; ++r) {
+            const int q = fill[cell(r)]++;
+            bq[r] = q;
+            qb[q] = r;
+            qa[q] = perm[r];
+        }
+        R = 0;
+        for (int p = 0; p < P; ++p) R = std::max(R, qs[(size_t)(p + 1) * ng] - qs[(size_t)p * ng]);
+        PF2_TRY(build_halo_plan(S, brp, bcol, bmap, bdiag, perm, part, grp, qs, bq, qb, qa, P, ng, R, optin, tri, mixed));
+        if (S->halo) return PF2_OK;
+    }
     const size_t smem = (part_smem_bytes(R, tri, mixed ? sizeof(float) : sizeof(double), mixed) + 15) / 16 * 16;
     if (smem + 2048 > (size_t)optin) {
         S->part_why = "a part's vectors exceed the shared memory of a block";

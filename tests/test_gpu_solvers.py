@@ -880,3 +880,32 @@ def test_waits_of_gmres_and_of_the_level_sweeps_that_run_out_return_timeout(cuda
     assert info.converged == 1 and info.status == 0
     ox, _ = O.pcg(rp, col, val, rhs, tol=1e-10, maxit=1000, precond="jacobi")
     assert rel_err(x.cpu().numpy(), ox) < 1e-6
+
+
+@pytest.mark.parametrize("pc,precision", [("ic", 0), ("ilu", 0), ("ic", 1)])
+@pytest.mark.parametrize("dims,halo", [((40, 20, 10), True), ((44, 24, 16), False)])
+def test_parts_of_a_tetrahedral_mesh(cuda, monkeypatch, dims, halo, pc, precision):
+    """Eight colours: parts of at least 512 rows, by the form with halo rows where it applies and by the
+    form with waits otherwise; bit for bit the iterates of the form and the parts asked for."""
+    xyz, tet = mg.box_tets(*dims)
+    m = g.Mesh3D.from_arrays(xyz, tet)
+    A = g.SparseMatrixCSR(m)
+    rp, col, _ = A.download()
+    n = rp.size - 1
+    row = np.repeat(np.arange(n), np.diff(rp))
+    val = np.where(row == col, 0.0, -1.0 - 0.3 * np.cos(row + col.astype(np.float64)))
+    sums = np.zeros(n)
+    np.add.at(sums, row, -val)
+    val[row == col] = 1.05 * sums
+    A.upload_values(val)
+    b = torch.tensor(np.sin(1.0 + np.arange(n)), device="cuda")
+    out = []
+    for part, parts in ((None, None), ("4" if halo else "3", str(n // 512))):
+        if part:
+            monkeypatch.setenv("PF2_CG_PART", part)
+            monkeypatch.setenv("PF2_CG_PARTS", parts)
+        x = torch.zeros_like(b)
+        g.LinearSolver(A, "cg", pc, ordering=1, precision=precision, tol=0.0, maxit=6,
+                       criterion=g.CRITERION_REL).solve(A, x, b, check=False)
+        out.append(x.view(torch.int64))
+    assert torch.equal(*out)
