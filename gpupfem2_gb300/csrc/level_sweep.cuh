@@ -162,6 +162,16 @@ __device__ __forceinline__ void level_sweep(const LevelSweep& S, const double* i
     for (int i = g; i < kLevelGroups; ++i) __syncthreads();
 }
 
+// z = M^{-1} r, by one block.
+__global__ void __launch_bounds__(kLevelThreads, 1) k_level_apply(KArgs a, LevelCg C) {
+    extern __shared__ __align__(128) unsigned char level_ring[];
+    for (int i = threadIdx.x; i < a.A.n; i += blockDim.x) __stcg(&C.rf[__ldg(&C.slot_f[i])], a.r[i]);
+    __syncthreads();
+#pragma unroll 1
+    for (int d = 0; d < 2; ++d)
+        level_sweep(d ? C.b : C.f, d ? C.tb : C.rf, d ? a.z : C.tb, d || a.precond == PF2_PRECOND_IC, level_ring);
+}
+
 // SolverCG::solve with ILU(0)/IC(0), k_pcg's iteration: q = A p with p.q; x, r; z = M^{-1} r by
 // block 0; r.z and r.r; p.
 __global__ void __launch_bounds__(kLevelThreads, 1) k_pcg_level(KArgs a, LevelCg C) {

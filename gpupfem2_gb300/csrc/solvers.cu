@@ -2929,10 +2929,12 @@ struct pf2_solver {
     // CG with level sweeps in one block (k_pcg_level): streams, units and what their values are
     bool level = false;
     int level_blocks = 0, level_units[2] = { 0, 0 };
-    DevBuf<unsigned char> level_stream[2];
-    DevBuf<int4> level_unit[2], level_src[2];  // src: double of the stream, factor position, pivot position (-1 = none)
-    DevBuf<int> level_slot;
-    DevBuf<double> level_rf, level_tb;
+    long long level_sources[2] = { 0, 0 };
+    DevBuf<unsigned char> level_plan;  // the arrays below, one after another
+    unsigned char* level_stream[2];
+    int4 *level_unit[2], *level_src[2];  // src: double of the stream, factor position, pivot position (-1 = none)
+    int* level_slot;
+    double* level_rhs[2];  // right-hand sides of the two sweeps, by slot
     bool factored = false;
     const pf2_csr* last = nullptr;  // matrix of the last setup / solve
 };
@@ -3659,107 +3661,149 @@ static void* part_kernel(const pf2_solver* S) {
 }
 
 // The streams and units of k_pcg_level (level_sweep.cuh).  level[dir], order[dir]: level and level
-// order of B's rows; deps(dir, row, f): f(dependency, factor position).
+// order of B's rows; deps(dir, row, f): f(dependency, factor position).  The two directions are built
+// side by side and go to the device in one allocation.  Creating a solver of 16,705 rows: 4.4 ms with
+// lists per row, nine allocations and the banded plan built as well (for k_precond_apply, whose place
+// k_level_apply takes: 1,000 -> 144 us an apply); 2.5 ms as it is, 2.1 with the banded plan alone.
 template <class Deps>
 static pf2_status build_level_plan(pf2_solver* S, const std::vector<int> (&level)[2], const std::vector<int> (&order)[2],
                                    const std::vector<int>& bdiag, const std::vector<int>& perm, bool ic, Deps&& deps) {
     const int n = S->n;
-    std::vector<std::vector<int>> units[2];  // rows
-    std::vector<int> unit_of[2], slot[2], first[2];
-    int slots[2];
-    for (int dir = 0; dir < 2; ++dir) {
-        unit_of[dir].assign(n, -1);
-        slot[dir].assign(n, -1);
-        int next = 0;
-        std::vector<std::vector<int>>& U = units[dir];
-        auto add = [&](const std::vector<int>& r) {
-            first[dir].push_back(next);
-            for (size_t q = 0; q < r.size(); ++q) {
-                unit_of[dir][r[q]] = (int)U.size();
-                slot[dir][r[q]] = next + (int)q;
-            }
-            next += ((int)r.size() + 31) / 32 * 32;
-            U.push_back(r);
-        };
-        const std::vector<int>& o = order[dir];
-        for (int i0 = 0; i0 < n;) {
-            int i1 = i0;
-            while (i1 < n && level[dir][o[i1]] == level[dir][o[i0]]) ++i1;
-            // rows with more late dependencies than registers come a unit later
-            std::vector<int> part[2];
-            const int last = (int)U.size() - 1;
-            for (int q = i0; q < i1; ++q) {
-                int late = 0;
-                deps(dir, o[q], [&](int j, int) { late += unit_of[dir][j] == last; });
-                part[late > kLevelCase].push_back(o[q]);
-            }
-            if (part[0].empty()) add(part[0]);
-            for (const std::vector<int>& r : part)
-                for (size_t q = 0; q < r.size(); q += 32 * kLevelSlices)
-                    add(std::vector<int>(r.begin() + q, r.begin() + std::min(r.size(), q + 32 * kLevelSlices)));
-            i0 = i1;
-        }
-        while (U.size() % kLevelGroups) add({});
-        slots[dir] = next;
-    }
-    for (int dir = 0; dir < 2; ++dir) {
+    struct Dir {
+        std::vector<int> rows, start, first;  // rows by unit; a unit's first row there, its first slot
+        std::vector<int> unit_of, slot;       // by row
         std::vector<unsigned char> stream;
         std::vector<int4> unit, src;
-        std::vector<std::pair<int, int>> list[2][32 * kLevelSlices];  // early, late: dependency, factor position
-        const bool pivot = dir == 1 || ic;
-        for (size_t u = 0; u < units[dir].size(); ++u) {
-            const std::vector<int>& r = units[dir][u];
-            const int at = first[dir][u], ns = ((int)r.size() + 31) / 32;
-            int K[2] = { 0, 0 };
-            for (size_t q = 0; q < r.size(); ++q) {
-                list[0][q].clear();
-                list[1][q].clear();
-                deps(dir, r[q], [&](int j, int k) { list[unit_of[dir][j] == (int)u - 1][q].emplace_back(j, k); });
-                for (int e = 0; e < 2; ++e) K[e] = std::max(K[e], (int)list[e][q].size());
+        int slots = 0;
+        bool fits = true;
+    } D[2];
+    const int workers = n >= 2048 ? 2 : 1;
+    parallel_ranges(2, workers, [&](int, int d0, int d1) {
+        for (int dir = d0; dir < d1; ++dir) {
+            Dir& L = D[dir];
+            L.unit_of.assign(n, -1);
+            L.slot.resize(n);
+            L.rows.reserve(n);
+            auto add = [&](const int* r, int count) {
+                L.start.push_back((int)L.rows.size());
+                L.first.push_back(L.slots);
+                for (int q = 0; q < count; ++q) {
+                    L.unit_of[r[q]] = (int)L.first.size() - 1;
+                    L.slot[r[q]] = L.slots + q;
+                }
+                L.rows.insert(L.rows.end(), r, r + count);
+                L.slots += (count + 31) / 32 * 32;
+            };
+            const std::vector<int>& o = order[dir];
+            std::vector<int> part[2];
+            for (int i0 = 0; i0 < n;) {
+                // rows with more late dependencies than registers come a unit later
+                const int last = (int)L.first.size() - 1, l = level[dir][o[i0]];
+                part[0].clear();
+                part[1].clear();
+                for (; i0 < n && level[dir][o[i0]] == l; ++i0) {
+                    int late = 0;
+                    deps(dir, o[i0], [&](int j, int) { late += L.unit_of[j] == last; });
+                    part[late > kLevelCase].push_back(o[i0]);
+                }
+                if (part[0].empty()) add(nullptr, 0);
+                for (const std::vector<int>& r : part)
+                    for (int q = 0; q < (int)r.size(); q += 32 * kLevelSlices)
+                        add(r.data() + q, std::min((int)r.size() - q, 32 * kLevelSlices));
             }
-            const int sb = level_slice_bytes(K[0] + K[1]);
-            const size_t off = stream.size();
-            if (K[0] > 255 || (off + (size_t)ns * sb) / 8 > 0x7fffffffull) return PF2_OK;  // (no plan)
-            stream.resize(off + (size_t)ns * sb, 0);
-            int flags = 0;
-            for (int q = 0; q < 32 * ns; ++q) {
-                const size_t base = off + (size_t)(q / 32) * sb, v0 = base / 8 + q % 32;
-                int* word = reinterpret_cast<int*>(stream.data() + base) + q % 32;
-                const bool real = q < (int)r.size();
-                word[64] = (at + q) % kLevelRing * 8;
-                word[96] = !real ? -1 : dir == 0 ? slot[1][r[q]] : perm[r[q]];
-                if (!real) continue;
-                const int dpos = pivot ? bdiag[r[q]] : -1;
-                if (pivot) src.push_back(make_int4((int)v0, -1, dpos, 0));
-                for (int e = 0; e < 2; ++e)
-                    for (size_t k = 0; k < list[e][q].size(); ++k) {
-                        const int j = list[e][q][k].first, c = (e ? K[0] : 0) + (int)k;
-                        // the ring holds it until the row's unit is solved; else where the sweep writes it
-                        const bool near = slot[dir][j] >= at + 32 * ns - kLevelRing;
-                        word[192 + 96 * c] = near ? slot[dir][j] % kLevelRing * 8 : ~(dir == 0 ? slot[1][j] : perm[j]);
-                        if (!near) flags = kLevelFar;
-                        src.push_back(make_int4((int)(v0 + 64 + 48 * c), list[e][q][k].second, e ? dpos : -1, 0));
-                    }
-            }
-            unit.push_back(make_int4((int)(off / 16), K[0] | K[1] << 8 | ns << 16 | flags, at, 0));
+            while (L.first.size() % kLevelGroups) add(nullptr, 0);
+            L.start.push_back(n);
         }
-        if (src.empty()) src.push_back(make_int4(0, -1, -1, 0));  // (an inverse pivot that no row reads)
-        S->level_units[dir] = (int)unit.size();
-        PF2_TRY(S->level_stream[dir].alloc(stream.size()));
-        PF2_CUDA(cudaMemcpy(S->level_stream[dir].p, stream.data(), stream.size(), cudaMemcpyHostToDevice));
-        PF2_TRY(S->level_unit[dir].alloc(unit.size()));
-        PF2_CUDA(cudaMemcpy(S->level_unit[dir].p, unit.data(), sizeof(int4) * unit.size(), cudaMemcpyHostToDevice));
-        PF2_TRY(S->level_src[dir].alloc(src.size()));
-        PF2_CUDA(cudaMemcpy(S->level_src[dir].p, src.data(), sizeof(int4) * src.size(), cudaMemcpyHostToDevice));
-    }
+    });
+    parallel_ranges(2, workers, [&](int, int d0, int d1) {
+        for (int dir = d0; dir < d1; ++dir) {
+            Dir& L = D[dir];
+            const bool pivot = dir == 1 || ic;
+            const int units = (int)L.first.size();
+            std::vector<int> early(units, 0), late(units, 0);
+            size_t bytes = 0, sources = pivot ? n : 0;
+            for (int u = 0; u < units; ++u) {
+                for (int q = L.start[u]; q < L.start[u + 1]; ++q) {
+                    int e = 0, l = 0;
+                    deps(dir, L.rows[q], [&](int j, int) { ++(L.unit_of[j] == u - 1 ? l : e); });
+                    early[u] = std::max(early[u], e);
+                    late[u] = std::max(late[u], l);
+                    sources += e + l;
+                }
+                bytes += (size_t)((L.start[u + 1] - L.start[u] + 31) / 32) * level_slice_bytes(early[u] + late[u]);
+                if (early[u] > 255 || bytes / 8 > 0x7fffffffull) {
+                    L.fits = false;
+                    return;
+                }
+            }
+            L.stream.assign(bytes, 0);
+            L.unit.reserve(units);
+            L.src.reserve(sources + 1);
+            size_t off = 0;
+            for (int u = 0; u < units; ++u) {
+                const int at = L.first[u], count = L.start[u + 1] - L.start[u], ns = (count + 31) / 32;
+                const int sb = level_slice_bytes(early[u] + late[u]);
+                int flags = 0;
+                for (int q = 0; q < 32 * ns; ++q) {
+                    const size_t base = off + (size_t)(q / 32) * sb, v0 = base / 8 + q % 32;
+                    int* word = reinterpret_cast<int*>(L.stream.data() + base) + q % 32;
+                    word[64] = (at + q) % kLevelRing * 8;
+                    word[96] = -1;
+                    if (q >= count) continue;
+                    const int r = L.rows[L.start[u] + q], dpos = pivot ? bdiag[r] : -1;
+                    word[96] = dir == 0 ? D[1].slot[r] : perm[r];
+                    if (pivot) L.src.push_back(make_int4((int)v0, -1, dpos, 0));
+                    int c[2] = { 0, early[u] };
+                    deps(dir, r, [&](int j, int k) {
+                        const bool is_late = L.unit_of[j] == u - 1;
+                        const int e = c[is_late]++, s = L.slot[j];
+                        // the ring holds it until the row's unit is solved; else where the sweep writes it
+                        const bool near = s >= at + 32 * ns - kLevelRing;
+                        word[192 + 96 * e] = near ? s % kLevelRing * 8 : ~(dir == 0 ? D[1].slot[j] : perm[j]);
+                        if (!near) flags = kLevelFar;
+                        L.src.push_back(make_int4((int)(v0 + 64 + 48 * e), k, is_late ? dpos : -1, 0));
+                    });
+                }
+                L.unit.push_back(make_int4((int)(off / 16), early[u] | late[u] << 8 | ns << 16 | flags, at, 0));
+                off += (size_t)ns * sb;
+            }
+            if (L.src.empty()) L.src.push_back(make_int4(0, -1, -1, 0));  // (an inverse pivot that no row reads)
+        }
+    });
+    if (!D[0].fits || !D[1].fits) return PF2_OK;  // (no plan)
     std::vector<int> slot_a(n);  // by A's rows
-    for (int i = 0; i < n; ++i) slot_a[perm[i]] = slot[0][i];
-    PF2_TRY(S->level_slot.alloc(n));
-    PF2_CUDA(cudaMemcpy(S->level_slot.p, slot_a.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    PF2_TRY(S->level_rf.alloc(slots[0]));
-    PF2_TRY(S->level_tb.alloc(slots[1]));
-    PF2_CUDA(cudaMemset(S->level_rf.p, 0, S->level_rf.bytes()));
-    PF2_CUDA(cudaMemset(S->level_tb.p, 0, S->level_tb.bytes()));
+    for (int i = 0; i < n; ++i) slot_a[perm[i]] = D[0].slot[i];
+    size_t size = 0;
+    auto room = [&](size_t bytes) {
+        const size_t at = size;
+        size += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    size_t at_stream[2], at_unit[2], at_src[2], at_rhs[2];
+    for (int d = 0; d < 2; ++d) {
+        at_rhs[d] = room(sizeof(double) * D[d].slots);
+        at_stream[d] = room(D[d].stream.size());
+        at_unit[d] = room(sizeof(int4) * D[d].unit.size());
+        at_src[d] = room(sizeof(int4) * D[d].src.size());
+    }
+    const size_t at_slot = room(sizeof(int) * n);
+    PF2_TRY(S->level_plan.alloc(size));
+    unsigned char* p = S->level_plan.p;
+    auto up = [&](auto*& d, size_t at, const auto& v) -> pf2_status {
+        d = reinterpret_cast<std::decay_t<decltype(d)>>(p + at);
+        PF2_CUDA(cudaMemcpy(d, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice));
+        return PF2_OK;
+    };
+    for (int d = 0; d < 2; ++d) {
+        PF2_TRY(up(S->level_stream[d], at_stream[d], D[d].stream));
+        PF2_TRY(up(S->level_unit[d], at_unit[d], D[d].unit));
+        PF2_TRY(up(S->level_src[d], at_src[d], D[d].src));
+        S->level_rhs[d] = reinterpret_cast<double*>(p + at_rhs[d]);
+        PF2_CUDA(cudaMemset(S->level_rhs[d], 0, sizeof(double) * D[d].slots));
+        S->level_units[d] = (int)D[d].unit.size();
+        S->level_sources[d] = (long long)D[d].src.size();
+    }
+    PF2_TRY(up(S->level_slot, at_slot, slot_a));
     S->level = true;
     return PF2_OK;
 }
@@ -3994,7 +4038,7 @@ static pf2_status build_tri_plan(pf2_solver* S) {
         else
             S->part_why = "ILU(0) / IC(0) in the natural order";
     }
-    if (K <= kBandMaxDeps) {
+    if (K <= kBandMaxDeps && !S->level) {  // (the level sweeps apply the preconditioner too)
         const int R = banded ? std::min(n, band_rows) : n;
         const int P = banded ? (n + R - 1) / R : 0;
         std::vector<int> rs(P + 1);
@@ -4197,9 +4241,9 @@ static pf2_status factorize(pf2_solver* S, const pf2_csr* A, cudaStream_t st) {
         }
     }
     for (int d = 0; d < 2 && S->level; ++d) {
-        const long long ne = (long long)S->level_src[d].n;
+        const long long ne = S->level_sources[d];
         k_level_values<<<std::min((int)blocks_for(ne), num_sms() * 8), kThreads, 0, st>>>(
-            ne, S->level_src[d].p, S->fact.p, reinterpret_cast<double*>(S->level_stream[d].p));
+            ne, S->level_src[d], S->fact.p, reinterpret_cast<double*>(S->level_stream[d]));
         PF2_LAUNCH_CHECK();
     }
     if (S->csr) {
@@ -4359,13 +4403,18 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
                         st);
         return PF2_OK;
     }
-    if (S->level && !precond_only) {
+    if (S->level) {
         LevelCg c{};
         for (int d = 0; d < 2; ++d)
-            (d ? c.b : c.f) = LevelSweep{ S->level_stream[d].p, S->level_unit[d].p, S->level_units[d] };
-        c.slot_f = S->level_slot.p;
-        c.rf = S->level_rf.p;
-        c.tb = S->level_tb.p;
+            (d ? c.b : c.f) = LevelSweep{ S->level_stream[d], S->level_unit[d], S->level_units[d] };
+        c.slot_f = S->level_slot;
+        c.rf = S->level_rhs[0];
+        c.tb = S->level_rhs[1];
+        if (precond_only) {
+            k_level_apply<<<1, kLevelThreads, kLevelSmem, st>>>(a, c);
+            PF2_LAUNCH_CHECK();
+            return PF2_OK;
+        }
         PF2_CUDA(cudaMemsetAsync(S->bar.p, 0, 2 * sizeof(unsigned), st));
         PF2_CUDA(cudaMemsetAsync(S->err.p, 0, sizeof(int), st));
         PF2_CUDA(cudaMemsetAsync(S->rec.p, 0, 5 * sizeof(int), st));
@@ -4539,7 +4588,7 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
         }
     }
     if (S->level) {
-        if ((s = allow_smem((void*)k_pcg_level))) return fail(s);
+        if ((s = allow_smem((void*)k_pcg_level)) || (s = allow_smem((void*)k_level_apply))) return fail(s);
         S->level_blocks = std::max(1, std::min(num_sms(), (S->n + kLevelThreads - 1) / kLevelThreads));
     }
     // the banded triangular solve keeps a range of the solution in shared memory
