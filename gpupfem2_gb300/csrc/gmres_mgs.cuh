@@ -41,6 +41,36 @@ __host__ __device__ constexpr size_t gmres_packet_words(int m, int G) {
 constexpr int kGramRows = 96;                                            // rows of L that each block keeps
 constexpr size_t kGramBytes = sizeof(double) * (kGramRows + 1) * (kGramRows + 1);  // (dynamic shared memory)
 constexpr int kGmresRows = 128;                                          // rows per block at least
+// Rows per block from which on the basis no longer stays in L2 and a block's loads in flight set
+// the pace: rows then go four (product) and two (update) at a time, and all 16 warps take part in
+// the dot products of a short basis.  1,997,113 rows, Jacobi, ms per solve, one reduction per projection
+// with two blocks per SM / without this / with it: 8 iterations 1.52 / 1.70 / 1.53, 40 iterations
+// 17.3 / 15.9 / 13.3, 40 restarted after 10 7.96 / 8.88 / 7.67.  Below, the loads cost more than they
+// hide: 125,364 rows, 40 iterations 1.34 without, 1.45 with.
+constexpr int kGmresMany = 4096;
+
+// f(i, (A x)_i) for rows i0, i0 + step, .. below r1, N of them with their loads in flight together
+// (each row's entries in order, as row_dot).
+template <int N, class F>
+__device__ __forceinline__ void gmres_rows(const Csr& A, const double* x, int i0, int step, int r1, F f) {
+    int s[N], e[N], len = 0;
+    double sum[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const int i = i0 + u * step;
+        s[u] = i < r1 ? __ldg(&A.rowptr[i]) : 0;
+        e[u] = i < r1 ? __ldg(&A.rowptr[i + 1]) : 0;
+        sum[u] = 0.0;
+        len = max(len, e[u] - s[u]);
+    }
+    for (int k = 0; k < len; ++k)
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+            if (s[u] + k < e[u]) sum[u] += __ldg(&A.val[s[u] + k]) * __ldcg(&x[__ldg(&A.col[s[u] + k])]);
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+        if (i0 + u * step < r1) f(i0 + u * step, sum[u]);
+}
 
 // Sums over this block's rows j = lo + lane, ... of w V_i and u V_i for C vectors i: lane 4 q's
 // low bits zero, bits 2..4 = q: value q (w V_0, ..; from C on u V_0, ..).
@@ -175,6 +205,8 @@ __device__ __forceinline__ void gmres_solve_upper(double* s, double* inv, const 
     }
 }
 
+// MANY: kGmresMany rows per block and more.
+template <bool MANY>
 __global__ void __launch_bounds__(kSolverThreads, 1) k_gmres_mgs(KArgs a, GmresMgs C) {
     const int ep_base = a.epoch ? *a.epoch : 0;  // read before the counter can advance
     __shared__ double sh[kShDoubles];  // (grid_sync, norm)
@@ -291,11 +323,16 @@ __global__ void __launch_bounds__(kSolverThreads, 1) k_gmres_mgs(KArgs a, GmresM
                     for (int i = lane; i < k; i += 32) __stcg(&a.H[(size_t)m * (k - 1) + i], h[i]);
             } else {
                 const int skip = k > 0 ? 32 : 0;
-                for (int i = r0 + threadIdx.x - skip; i < r1; i += blockDim.x - skip) {
+                const int step = (int)blockDim.x - skip;
+                auto put = [&](int i, double sum) {
                     vk[i] = __ldcg(&raw[i]) / aux;
-                    const double v = row_dot(a.A, i, raw) * inv;
+                    const double v = sum * inv;
                     out[i] = jacobi ? v * a.invd[i] : v;
-                }
+                };
+                if constexpr (MANY)
+                    for (int i = r0 + threadIdx.x - skip; i < r1; i += 4 * step) gmres_rows<4>(a.A, raw, i, step, r1, put);
+                else
+                    for (int i = r0 + threadIdx.x - skip; i < r1; i += step) put(i, row_dot(a.A, i, raw));
             }
             __syncthreads();
             if (k > 0) res = fabs(beta[k]);
@@ -307,11 +344,11 @@ __global__ void __launch_bounds__(kSolverThreads, 1) k_gmres_mgs(KArgs a, GmresM
                 if (!precond_apply(a, a.q, w, r0, r1, apply++, ep_base)) return;
                 __syncthreads();
             }
-            // V^T w and V^T v_k: tasks of four vectors and a segment of the rows, eight of them at least
+            // V^T w and V^T v_k: tasks of four vectors and a segment of the rows, eight of them at least (many rows: 16)
             const unsigned s = ++seq;
             unsigned long long* const part = C.part + 2 * (size_t)(s & 1) * nval * G;
             unsigned long long* const total = tot + 2 * (size_t)(s & 1) * nval;
-            const int groups = (k + 4) / 4, segs = max(1, 8 / groups), len = (r1 - r0 + segs - 1) / segs;
+            const int groups = (k + 4) / 4, segs = max(1, (MANY ? 16 : 8) / groups), len = (r1 - r0 + segs - 1) / segs;
             // value of vector i: i (w) or k + 1 + i (v_k; none for i = k)
             auto send = [&](int i, int which, double v) {
                 if (which ? i < k : i <= k)
@@ -374,12 +411,32 @@ __global__ void __launch_bounds__(kSolverThreads, 1) k_gmres_mgs(KArgs a, GmresM
             __syncthreads();
             gmres_solve_lower(h, g, Ls, a.H, m, k);
             nn = 0.0;
-            for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
-                double v = w[j];
+            if constexpr (MANY) {  // two rows of a thread together
+                for (int j = r0 + threadIdx.x; j < r1; j += 2 * blockDim.x) {
+                    const bool two = j + (int)blockDim.x < r1;
+                    const int j2 = two ? j + (int)blockDim.x : j;
+                    double v = w[j], v2 = w[j2];
 #pragma unroll 4
-                for (int i = 0; i <= k; ++i) v -= h[i] * a.V[(size_t)i * n + j];
-                __stcg(&raw[j], v);
-                nn += v * v;
+                    for (int i = 0; i <= k; ++i) {
+                        const double* Vi = a.V + (size_t)i * n;
+                        v -= h[i] * Vi[j];
+                        v2 -= h[i] * Vi[j2];
+                    }
+                    __stcg(&raw[j], v);
+                    nn += v * v;
+                    if (two) {
+                        __stcg(&raw[j2], v2);
+                        nn += v2 * v2;
+                    }
+                }
+            } else {
+                for (int j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
+                    double v = w[j];
+#pragma unroll 4
+                    for (int i = 0; i <= k; ++i) v -= h[i] * a.V[(size_t)i * n + j];
+                    __stcg(&raw[j], v);
+                    nn += v * v;
+                }
             }
             if (!norm(nn, aux)) return;
             ++k;

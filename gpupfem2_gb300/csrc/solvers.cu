@@ -4290,7 +4290,7 @@ static int max_applies(const pf2_solver* S) {
 // standard iteration otherwise).
 static void* solve_kernel(const pf2_solver_options& o, bool csr) {
     if (o.kind == PF2_SOLVER_GMRES)
-        return o.orthogonalization == PF2_GS_MODIFIED ? (void*)k_gmres_mgs : (void*)k_gmres;
+        return o.orthogonalization == PF2_GS_MODIFIED ? (void*)k_gmres_mgs<false> : (void*)k_gmres;
     if (o.kind == PF2_SOLVER_BICGSTAB) return (void*)k_bicgstab;
     if (o.precision == PF2_PRECISION_MIXED) return (void*)k_pcg_mixed;
     const bool tri = o.precond == PF2_PRECOND_ILU || o.precond == PF2_PRECOND_IC;
@@ -4460,6 +4460,7 @@ static pf2_status launch_solver(pf2_solver* S, const pf2_csr* A, double* x, cons
     // iteration elsewhere
     if (!mixed && S->opt.kind == PF2_SOLVER_CG && S->opt.cg_variant == PF2_CG_PIPELINED && S->csr)
         fn = pipe_kernel();
+    if (fn == (void*)k_gmres_mgs<false> && S->n / S->blocks >= kGmresMany) fn = (void*)k_gmres_mgs<true>;
     GmresMgs gm{ S->packets.p };
     void* args_mgs[] = { &a, &gm };
     if (S->packets.p) PF2_CUDA(cudaMemsetAsync(S->packets.p, 0, S->packets.bytes(), st));  // exchanges count from 1
@@ -4594,8 +4595,9 @@ pf2_status pf2_solver_create(const pf2_csr* A, const pf2_solver_options* opt, pf
     // the banded triangular solve keeps a range of the solution in shared memory
     S->smem = S->band_P ? sizeof(double) * (size_t)S->band_R : 0;
     void* fn = solve_kernel(*opt, S->csr);
-    const bool mgs = fn == (void*)k_gmres_mgs;
+    const bool mgs = fn == (void*)k_gmres_mgs<false>;
     if (mgs) S->extra_smem = kGramBytes;
+    if (mgs && (s = allow_smem((void*)k_gmres_mgs<true>))) return fail(s);
     if (S->smem + S->extra_smem && (s = allow_smem(fn))) return fail(s);
     if (S->smem && (s = allow_smem((void*)k_precond_apply))) return fail(s);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kSolverThreads, S->smem + S->extra_smem) != cudaSuccess ||
