@@ -282,7 +282,10 @@ __device__ __forceinline__ HaloSm<V, RES> halo_sm(const PartHalo& C, int n, unsi
             for (unsigned o = 0; o < vb; o += 16384) halo_bulk_copy(halo_smem_u32(entries) + o, gv + o, min(16384u, vb - o), m);
             for (unsigned o = 0; o < cb; o += 16384) halo_bulk_copy(halo_smem_u32(cols) + o, gc + o, min(16384u, cb - o), m);
         }
-        if (!halo_mbar_wait(m, 0)) atomicExch(err, (int)DEV_TIMEOUT);
+        if (!halo_mbar_wait(m, 0)) {
+            atomicExch(err, (int)DEV_TIMEOUT);
+            halo_mbar_wait(m, 0);  // bounded: the copies may still be writing
+        }
         S.items.v0 = reinterpret_cast<const V*>(entries) + (size_t)(ew - e0) * 32 + lane;
         S.items.c0 = reinterpret_cast<const unsigned short*>(cols) + (size_t)(ew - e0) * 32 + lane;
     } else {
