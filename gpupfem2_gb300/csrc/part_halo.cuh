@@ -158,9 +158,10 @@ __device__ __forceinline__ unsigned halo_smem_u32(const void* p) {
 
 constexpr long long kHaloCopyPolls = 1ll << 22;
 
-// Bounded wait for phase `parity` of an mbarrier.
+// Bounded wait for phase `parity` of an mbarrier.  False where the limit ran out: it then has waited
+// as long again, as the copies may still have been writing.
 __device__ __forceinline__ bool halo_mbar_wait(unsigned mbar, unsigned parity) {
-    for (long long i = 0; i < kHaloCopyPolls; ++i) {
+    for (long long i = 0; i < 2 * kHaloCopyPolls; ++i) {
         unsigned done;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -168,7 +169,7 @@ __device__ __forceinline__ bool halo_mbar_wait(unsigned mbar, unsigned parity) {
             : "=r"(done)
             : "r"(mbar), "r"(parity)
             : "memory");
-        if (done) return true;
+        if (done) return i < kHaloCopyPolls;
     }
     return false;
 }
@@ -282,10 +283,7 @@ __device__ __forceinline__ HaloSm<V, RES> halo_sm(const PartHalo& C, int n, unsi
             for (unsigned o = 0; o < vb; o += 16384) halo_bulk_copy(halo_smem_u32(entries) + o, gv + o, min(16384u, vb - o), m);
             for (unsigned o = 0; o < cb; o += 16384) halo_bulk_copy(halo_smem_u32(cols) + o, gc + o, min(16384u, cb - o), m);
         }
-        if (!halo_mbar_wait(m, 0)) {
-            atomicExch(err, (int)DEV_TIMEOUT);
-            halo_mbar_wait(m, 0);  // bounded: the copies may still be writing
-        }
+        if (!halo_mbar_wait(m, 0)) atomicExch(err, (int)DEV_TIMEOUT);
         S.items.v0 = reinterpret_cast<const V*>(entries) + (size_t)(ew - e0) * 32 + lane;
         S.items.c0 = reinterpret_cast<const unsigned short*>(cols) + (size_t)(ew - e0) * 32 + lane;
     } else {
