@@ -3172,7 +3172,8 @@ constexpr int kHaloFactor = 1 << 30;  // flag of a factor value in the streams' 
 // columns, or the halo is over four times the part (many groups: a 3D graph), where every part
 // would compute most of its neighbours' sweeps.  Where it applies it measured faster at every
 // size (us per IC(0) iteration, waits in the sweeps against halo rows: 340 rows 23.6 / 12.8,
-// 16,705 rows 25.4 / 11.2, 125,364 rows 29.8 / 14.1, 499,288 rows 43.5 / 36.5).
+// 16,705 rows 25.4 / 11.2, 125,364 rows 29.8 / 14.1, 499,288 rows 43.5 / 36.5; tetrahedra 462 rows
+// 53.4 / 19.2, 9,471 rows 74.2 / 28.2, 211,191 rows 86.3 / 72.1).
 static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, const std::vector<int>& bcol,
                                   const std::vector<int>& bmap, const std::vector<int>& bdiag,
                                   const std::vector<int>& perm, const std::vector<int>& part,
