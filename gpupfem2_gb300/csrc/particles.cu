@@ -604,7 +604,7 @@ struct pf2_particles {
     DevBuf<int> cw[2];
     int cur = 0;
     DevBuf<int> rank, perm, count, mask, seg, segsz, scratch, cnt, err;
-    DevBuf<double> part, change;  // projection partial sums; k_node_change
+    DevBuf<double> part;  // projection partial sums; between a correction and the next sums, k_node_change's
     PinnedBuf<int> h_cnt;
     bool partials_valid = false;
     bool seeded = false;
@@ -698,10 +698,13 @@ pf2_status particles_correct(pf2_particles* H, const double* ux, const double* u
                              const double* uyo, cudaStream_t st) {
     const int nv = H->mesh->nv;
     if (uxo && (long long)H->mesh->nc * H->ppc >= kNodeChangeMin) {
-        k_node_change<<<blocks_for(nv), kThreads, 0, st>>>(nv, ux, uy, uxo, uyo, H->change.p, H->change.p + nv);
+        // (the correction makes the partial sums invalid: their place is free)
+        double* change = H->part.p;
+        H->partials_valid = false;
+        k_node_change<<<blocks_for(nv), kThreads, 0, st>>>(nv, ux, uy, uxo, uyo, change, change + nv);
         PF2_LAUNCH_CHECK();
-        ux = H->change.p;
-        uy = H->change.p + nv;
+        ux = change;
+        uy = change + nv;
         uxo = nullptr;
     }
     auto* correct = uxo ? k_correct<true> : k_correct<false>;
@@ -835,7 +838,7 @@ pf2_status pf2_particles_create(const pf2_mesh* m, int level, double capacity_fa
     if ((s = H->rank.alloc(H->cap)) || (s = H->perm.alloc(H->cap)) || (s = H->count.alloc(nc + 1)) ||
         (s = H->mask.alloc(nc + 1)) || (s = H->seg.alloc(nc + 1)) || (s = H->segsz.alloc(nc + 1)) ||
         (s = H->scratch.alloc(scan_scratch_ints(nc))) || (s = H->cnt.alloc(2)) || (s = H->err.alloc(1)) ||
-        (s = H->part.alloc(9 * (size_t)nc)) || (s = H->change.alloc(2 * (size_t)m->nv)) || (s = H->h_cnt.alloc(2)))
+        (s = H->part.alloc(std::max(9 * (size_t)nc, 2 * (size_t)m->nv))) || (s = H->h_cnt.alloc(2)))
         return fail(s);
     if (cudaMemset(H->count.p, 0, sizeof(int) * (nc + 1)) != cudaSuccess ||
         cudaMemset(H->mask.p, 0, sizeof(int) * (nc + 1)) != cudaSuccess ||

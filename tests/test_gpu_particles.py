@@ -153,3 +153,31 @@ def test_sub_cells_at_their_borders_bitwise(cuda, level):
     ph.advect(t, t, 0.1, 1)
     R, _, _ = O.advect(R, xy, tri, invJ, off, idx, still, still, 0.1, 1, level, cap=8 * level * level * nc)
     _assert_same(ph.download(), R)
+
+
+def test_large_sets_project_again_after_a_correction(cuda):
+    """From half a million particles on a correction forms the nodes' change in the place of the
+    projection's partial sums: the velocities are the oracle's bit for bit, and projections after it
+    are those of a handle that never corrected."""
+    xy, tri, m = _mesh(256, 64)
+    ph = g.ParticleHandler2D(m, 4)
+    ph.seed()
+    ux, uy = _field(xy)
+    tux, tuy = torch.tensor(ux, device="cuda"), torch.tensor(uy, device="cuda")
+    ph.init_velocity(tux, tuy)
+    px, py, qx, qy = (torch.empty_like(tux) for _ in range(4))
+    ph.project(px, py)
+    nx, ny = ux * 1.1, uy - 0.2
+    ph.correct(torch.tensor(nx, device="cuda"), torch.tensor(ny, device="cuda"), tux, tuy)
+    R = O.seed(xy, tri, 4)
+    R["u"], R["v"] = O.correct_velocity(R, tri, ux, uy)
+    R["u"], R["v"] = O.correct_velocity(R, tri, nx, ny, ux, uy)
+    P = ph.download()
+    assert P["cell"].size >= 1 << 19
+    _assert_same(P, R)
+    other = g.ParticleHandler2D(m, 4)
+    other.upload(P)
+    for _ in range(2):
+        ph.project(px, py)
+        other.project(qx, qy)
+        assert torch.equal(px, qx) and torch.equal(py, qy)
