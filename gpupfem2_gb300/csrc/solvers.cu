@@ -3175,8 +3175,9 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
                                   const std::vector<int>& bmap, const std::vector<int>& bdiag,
                                   const std::vector<int>& perm, const std::vector<int>& part,
                                   const std::vector<int>& grp, const std::vector<int>& qs, const std::vector<int>& bq,
-                                  const std::vector<int>& qb, const std::vector<int>& qa, int P, int ng, int R,
-                                  int optin, bool tri, bool mixed) {
+                                  const std::vector<int>& qb, const std::vector<int>& qa,
+                                  const std::vector<unsigned char>& bnd_a, int P, int ng, int R, int optin, bool tri,
+                                  bool mixed) {
     S->halo = false;
     const int n = S->n;
     if (const char* e = getenv("PF2_CG_PART"))
@@ -3217,6 +3218,7 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
                 cls[j] |= bits;
             };
             for (int q = p0; q < p0 + np; ++q) {
+                if (!bnd_a[qa[q]]) continue;
                 const int i = qb[q];
                 for (int e = brp[i]; e < brp[i + 1]; ++e) {
                     const int j = bcol[e];
@@ -3398,22 +3400,28 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
         add(all.r1off, w.r1off, all.r1off.back());
         add(all.ioff, w.ioff, all.ioff.back());
         add(all.went, w.went, (int)(all.col.size() / 32));
-        auto join = [](auto& to, auto& v) {
-            if (to.empty()) to = std::move(v);
-            else to.insert(to.end(), v.begin(), v.end());
+        auto join = [&](auto m) {
+            if (&w == &piece[0]) {
+                size_t size = 0;
+                for (const Piece& v : piece) size += (v.*m).size();
+                all.*m = std::move(w.*m);
+                (all.*m).reserve(size);
+            } else {
+                (all.*m).insert((all.*m).end(), (w.*m).begin(), (w.*m).end());
+            }
         };
-        join(all.hq, w.hq);
-        join(all.fg, w.fg);
-        join(all.zg, w.zg);
-        join(all.wit, w.wit);
-        join(all.gsl, w.gsl);
-        join(all.map, w.map);
-        join(all.dmap, w.dmap);
-        join(all.item, w.item);
-        join(all.fl, w.fl);
-        join(all.zl, w.zl);
-        join(all.r1, w.r1);
-        join(all.col, w.col);
+        join(&Piece::hq);
+        join(&Piece::fg);
+        join(&Piece::zg);
+        join(&Piece::wit);
+        join(&Piece::gsl);
+        join(&Piece::map);
+        join(&Piece::dmap);
+        join(&Piece::item);
+        join(&Piece::fl);
+        join(&Piece::zl);
+        join(&Piece::r1);
+        join(&Piece::col);
         all.TL = std::max(all.TL, w.TL);
     }
     auto& [hq, fg, zg, wit, went, gsl, map, dmap, hoff, foff, zoff, r1off, ioff, item, fl, zl, r1, col, TL] = all;
@@ -3439,6 +3447,9 @@ static pf2_status build_halo_plan(pf2_solver* S, const std::vector<int>& brp, co
     PF2_TRY(up(S->q_amap, map));
     // one allocation and one copy for the rest: a small system's plan is mostly their calls
     std::vector<unsigned char> plan;
+    plan.reserve(sizeof(short) * (col.size() + fl.size() + zl.size() + r1.size()) + item.size() + pub.size() +
+                 sizeof(int) * (dmap.size() + hoff.size() + hq.size() + foff.size() + fg.size() + zoff.size() + zg.size() +
+                                r1off.size() + ioff.size() + wit.size() + went.size() + gsl.size()) + 18 * 256);
     std::vector<std::function<void(unsigned char*)>> place;
     auto pack = [&](auto*& d, const auto& v) {
         const size_t at = (plan.size() + 255) / 256 * 256, bytes = sizeof(v[0]) * v.size();
@@ -3544,7 +3555,7 @@ static pf2_status build_part_plan(pf2_solver* S, const std::vector<int>& rp, con
         }
         R = 0;
         for (int p = 0; p < P; ++p) R = std::max(R, qs[(size_t)(p + 1) * ng] - qs[(size_t)p * ng]);
-        PF2_TRY(build_halo_plan(S, brp, bcol, bmap, bdiag, perm, part, grp, qs, bq, qb, qa, P, ng, R, optin, tri, mixed));
+        PF2_TRY(build_halo_plan(S, brp, bcol, bmap, bdiag, perm, part, grp, qs, bq, qb, qa, bnd_a, P, ng, R, optin, tri, mixed));
         if (S->halo) return PF2_OK;
     }
     const size_t smem = (part_smem_bytes(R, tri, mixed ? sizeof(float) : sizeof(double), mixed) + 15) / 16 * 16;
